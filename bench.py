@@ -266,8 +266,11 @@ def measured_peaks() -> tuple[float, str]:
 
 
 def kernel_bytes(name: str, na: int, nb: int, log_n: int, square: bool) -> int:
-    """Algorithmic global-memory bytes of one launch (minimal reads + writes)."""
+    """Algorithmic global-memory bytes of one launch (minimal reads + writes).
+    `log_n` counts 32-bit digits; the five-prime kernels (k_wide_*) take half
+    as many points of 64-bit digits."""
     n = 1 << log_n
+    s64 = 10 * n  # five primes x u32 on n / 2 points
     s32 = 12 * n  # one operand's residues: 3 primes x u32 per point
     ops = 1 if square else 2
     inp = (na + (0 if square else nb)) * 8
@@ -277,6 +280,10 @@ def kernel_bytes(name: str, na: int, nb: int, log_n: int, square: bool) -> int:
         "k_mid_rows": ops * s32 + s32,
         "k_inv_cols": s32 + chunk_bytes,
         "k_carry": chunk_bytes + (na + nb) * 8,
+        "k_wide_fwd": inp + ops * s64,
+        "k_wide_rows": ops * s64 + s64,
+        "k_wide_inv": 2 * s64,
+        "k_wide_carry": s64 + (na + nb) * 8,
     }[name]
 
 
@@ -316,7 +323,14 @@ def source_mul_counts(na: int, nb: int, log_n: int, log_n1: int, log_n2: int, sq
     r0 = _plan_rounds(log_n1)[0]
     mid = 3 * (n2 * (ops + 1) * _bfly_muls(log_n1) + 4 * n + 6 * n + 7 * n / (1 << r0))
     inv = 3 * n1 * _bfly_muls(log_n2) + 14 * n
-    return {"k_fwd_cols": fwd, "k_mid_rows": mid, "k_inv_cols": inv, "k_carry": 0.0}
+    # the five-prime kernels, on n / 2 points with the same column length: digit
+    # reduction 4, Shoup twiddles 6 a point, pointwise Montgomery product 3, CRT 20
+    m, m1 = n // 2, n1 // 2
+    wfwd = ops * 5 * (m1 * _bfly_muls(log_n2) + 4 * (m // 2 if half else m) + 6 * m)
+    wmid = 5 * (n2 * (ops + 1) * _bfly_muls(log_n1 - 1) + 9 * m)
+    winv = 5 * m1 * _bfly_muls(log_n2)
+    return {"k_fwd_cols": fwd, "k_mid_rows": mid, "k_inv_cols": inv, "k_carry": 0.0,
+            "k_wide_fwd": wfwd, "k_wide_rows": wmid, "k_wide_inv": winv, "k_wide_carry": 20.0 * m}
 
 
 def profiled_pipes() -> dict | None:
@@ -338,9 +352,9 @@ def compute_roofline(kernels_ms: dict, dom: str, prod_ms: float, sm_mhz: float |
     prof = profiled_pipes()
     res = {"bound": "int32 multiply pipe (fmaheavy)", "kernel": dom,
            "source_mul_ops_per_launch": counts.get(dom),
-           "source_mul_ops_per_product": sum(counts.values()),
+           "source_mul_ops_per_product": sum(v for k, v in counts.items() if k in kernels_ms),
            "source_note": "counted from the kernel source: 3 per Shoup butterfly or Montgomery product, "
-                          "2 per digit reduction, 14 per Garner CRT point"}
+                          "2 to 4 per digit reduction, 14 per Garner CRT point, 20 per five-prime CRT point"}
     if not prof or dom not in prof or not sm_mhz:
         res["profile"] = None
         return res
@@ -358,7 +372,7 @@ def compute_roofline(kernels_ms: dict, dom: str, prod_ms: float, sm_mhz: float |
         "ncu_busy_pct": k["fmaheavy_busy_pct"], "ncu_issue_active_pct": k["issue_active_pct"],
         "sm_mhz": sm_mhz,
     })
-    names = [x for x in ("k_fwd_cols", "k_mid_rows", "k_inv_cols", "k_carry") if x in prof]
+    names = [x for x in kernels_ms if x in prof]
     busy = sum(prof[x]["fmaheavy_busy_cycles_per_sm"] for x in names)
     insts = sum(prof[x]["warp_inst"] for x in names)
     prod_cycles = prod_ms * 1e-3 * clk

@@ -11,6 +11,13 @@
 //   469762049 (g 3), 1811939329 = 27*2^26+1 (g 13), 2013265921 = 15*2^27+1 (g 31)
 //   product ~2^90.47 > 2^89 >= (N/2)(2^32-1)^2 for N <= 2^26; residues are
 //   kept fully reduced in [0, p) (sums of two still fit in 32 bits).
+// Sets 2 and 3 have five primes and carry 64-bit digits (wide_kernels.cu):
+// Set 2 ("lazy", up to 2^22 points), all primes < 2^30 with 2^22 | p-1:
+//   998244353 (g 3), 985661441 (g 3), 943718401 (g 7), 935329793 (g 3), 918552577 (g 5)
+//   product ~2^149.16 > 2^149 >= (N/2)(2^64-1)^2 for N <= 2^22.
+// Set 3 ("strict", up to 2^25 points), all primes < 2^31 with 2^25 | p-1:
+//   1107296257 (g 10), 1711276033 (g 29), 1811939329 (g 13), 2013265921 (g 31), 2113929217 (g 5)
+//   product ~2^153.36 > 2^152 >= (N/2)(2^64-1)^2 for N <= 2^25.
 // 469762049 and 2013265921 are the reference's own P[0], P[1]
 // (include/bigint/ntt_base.h:15); its third prime 2281701377 > 2^31 would not
 // leave room for carry-free sums.
@@ -23,25 +30,34 @@
 
 namespace bgpu {
 
-constexpr int kNumPrimes = 3;
-constexpr int kNumSets = 2;
+constexpr int kNumPrimes = 3;   // of sets 0 and 1
+constexpr int kWidePrimes = 5;  // of sets 2 and 3
+constexpr int kMaxPrimes = 5;
+constexpr int kNumSets = 4;
 constexpr int kMaxLogN = 26;    // largest transform overall (set 1)
 constexpr int kLazyMaxLogN = 23;  // largest transform of set 0
 constexpr int kMaxLogRow = 15;  // stage tables cover pair distances h < 2^15
 
+constexpr int kWideLazyMaxLogN = 22;  // largest transform of set 2
+constexpr int kWideMaxLogN = 25;      // of set 3
+
 struct PrimeSetInfo {
-    uint32_t p[kNumPrimes];
-    uint32_t g[kNumPrimes];
+    int np;  // primes
+    uint32_t p[kMaxPrimes];
+    uint32_t g[kMaxPrimes];
     int log_max;  // 2^log_max | p-1 for every prime of the set
     int split;    // inter-pass twiddle exponent split: e = hi << split | lo
 };
 
 constexpr PrimeSetInfo kPrimeSets[kNumSets] = {
-    {{469762049u, 754974721u, 998244353u}, {3u, 11u, 3u}, kLazyMaxLogN, 12},
-    {{469762049u, 1811939329u, 2013265921u}, {3u, 13u, 31u}, kMaxLogN, 13},
+    {3, {469762049u, 754974721u, 998244353u}, {3u, 11u, 3u}, kLazyMaxLogN, 12},
+    {3, {469762049u, 1811939329u, 2013265921u}, {3u, 13u, 31u}, kMaxLogN, 13},
+    {5, {998244353u, 985661441u, 943718401u, 935329793u, 918552577u}, {3u, 3u, 7u, 3u, 5u}, kWideLazyMaxLogN, 11},
+    {5, {1107296257u, 1711276033u, 1811939329u, 2013265921u, 2113929217u}, {10u, 29u, 13u, 31u, 5u}, kWideMaxLogN, 13},
 };
 
 inline int prime_set_for(int log_n) { return log_n <= kLazyMaxLogN ? 0 : 1; }
+inline int wide_set_for(int log_n) { return log_n <= kWideLazyMaxLogN ? 2 : 3; }
 
 struct PrimeInfo {
     uint32_t p;

@@ -20,6 +20,7 @@
 #include "../../include/bigint_b200.h"
 #include "engine.h"
 #include "tables.h"
+#include "wide.h"
 
 namespace bgpu {
 namespace {
@@ -80,6 +81,7 @@ struct Engine {
     // optional per-kernel timing of NTT products: a ring of event sets, one
     // set per product, read back (and averaged) without per-product syncs
     bool kernel_timing = false;
+    bool timed_wide = false;  // the last product timed was a five-prime one
     std::vector<cudaEvent_t> kev;  // kTimingRing * (kNttLaunches + 1)
     uint64_t kev_count = 0;
     // operand block of products beyond the largest transform (a power of
@@ -144,7 +146,7 @@ int build_tables_locked() {
                        cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cuda_status(e);
         g.consts[ps] = make_consts(ps, kMaxLogRow, static_cast<const uint2*>(g.d_tables[ps]));
-        e = upload_consts(kSlotEngine + ps, g.consts[ps]);
+        e = ps < 2 ? upload_consts(kSlotEngine + ps, g.consts[ps]) : upload_wide_consts(ps, g.consts[ps]);
         if (e != cudaSuccess) return cuda_status(e);
     }
     std::vector<double2> fh(2 * fft_table_block());
@@ -232,6 +234,51 @@ int prepare_scratch(int log_n, bool square, ProductScratch* s) {
     return BGPU_OK;
 }
 
+// log2 of the five-prime transform of a product, in 64-bit digits, or 0 for
+// the three-prime one.
+int wide_log(const OperandDesc& a, const OperandDesc& b) {
+    const int ln = ceil_log2((uint64_t)wide_digits(a) + wide_digits(b) - 1);
+    return ln <= kWideMaxLogN && wide_shape(ln).log_n2 ? ln : 0;
+}
+
+// Product of two device operands on the five-prime transform.
+int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, int ln, void* out, int out_fmt,
+                  size_t out_cap, cudaStream_t st, bgpu_stats* stats) {
+    const size_t nn = (size_t)1 << ln;
+    const uint32_t bpp = wide_carry_blocks(out_cap, out_fmt);
+    const size_t y_bytes = align256((square ? 1 : 2) * (size_t)kWidePrimes * nn * 4);
+    int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + align256((size_t)bpp * 8));
+    if (rc != BGPU_OK) return rc;
+    ProductDesc one{};
+    one.op[0] = a;
+    one.op[1] = square ? a : b;
+    one.y = static_cast<uint32_t*>(g.d_scratch);
+    one.flags = reinterpret_cast<uint64_t*>(static_cast<char*>(g.d_scratch) + y_bytes);
+    one.out = out;
+    one.out_cap = out_cap;
+    CarryLaunch cl;
+    cl.ticket_base = g.ticket_base;
+    cl.epoch = ++g.epoch;
+    cl.ticket = g.d_ticket;
+    cl.err = g.d_err;
+    g.ticket_base += bpp;
+    g.ntt_log_n = -1;  // no forward pass overlaps this product's carry scan
+    cudaEvent_t* ev = nullptr;
+    if (g.kernel_timing) {
+        ev = g.kev.data() + (g.kev_count % kTimingRing) * (kNttLaunches + 1);
+        ++g.kev_count;
+        g.timed_wide = true;
+    }
+    const cudaError_t e = launch_wide_product(g.consts[wide_set_for(ln)], nullptr, one, 1, square, ln, out_fmt, bpp,
+                                              cl, st, ev);
+    g.last_launches = kNttLaunches;
+    if (stats) {
+        stats->method = BGPU_METHOD_NTT;
+        stats->log2_points = (uint32_t)std::max(5, ceil_log2((uint64_t)a.nd32 + b.nd32 - 1));
+    }
+    return cuda_status(e);
+}
+
 // Core: product of two device operands into a device output (async).
 // nd32 values are operand lengths in 32-bit digits.
 int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, void* out,
@@ -242,6 +289,7 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     const int log_n = ceil_log2(total32 - 1);
     if (log_n > kMaxLogN || !shape_supported(log_n < 5 ? 5 : log_n, square))
         return BGPU_ERR_CAPACITY;
+    if (const int wl = wide_log(a, b)) return multiply_wide(a, b, square, wl, out, out_fmt, out_cap, st, stats);
     const int ln = log_n < 5 ? 5 : log_n;
     ProductScratch s{};
     int rc = prepare_scratch(ln, square, &s);
@@ -264,6 +312,7 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     if (g.kernel_timing) {
         ev = g.kev.data() + (g.kev_count % kTimingRing) * (kNttLaunches + 1);
         ++g.kev_count;
+        g.timed_wide = false;
     }
     const int ps = prime_set_for(ln);
     cudaError_t e = launch_ntt_product(kSlotEngine + ps, g.consts[ps], a, b, square, ln, s, out,
@@ -2634,7 +2683,7 @@ int bgpu_kernel_times(const char** names, float* mean_ms, int cap, uint32_t* npr
             if (cudaEventElapsedTime(&t, ev[k], ev[k + 1]) != cudaSuccess) return BGPU_ERR_CUDA;
             sum += t;
         }
-        if (names) names[k] = kNttKernelNames[k];
+        if (names) names[k] = g.timed_wide ? kWideKernelNames[k] : kNttKernelNames[k];
         if (mean_ms) mean_ms[k] = (float)(sum / (double)n);
     }
     if (nproducts) *nproducts = (uint32_t)n;

@@ -18,13 +18,13 @@ enum DigitFormat : int {
 // Constants of one prime set, kept in __constant__ memory (one slot per owner
 // and prime set) so kernels can index them by the runtime prime number.
 struct NttConsts {
-    PrimeInfo pr[kNumPrimes];
-    uint32_t one_w[kNumPrimes], one_wp[kNumPrimes];  // Montgomery form of 1 (reduces any u32 mod p)
-    uint32_t red[kNumPrimes];  // floor(2^32 / p): Shoup form of 1, reduces any u32 into [0, 2p)
-    const uint2* stage[kNumPrimes][2];  // [prime][dir] Shoup pairs: entry h+m = omega_{2h}^{+-m}
-    const uint2* th[kNumPrimes][2];     // Montgomery pairs: omega_{2^log_max}^{+-(i << split)}
-    const uint2* tl[kNumPrimes][2];     // Montgomery pairs: omega_{2^log_max}^{+-i}
-    // Garner CRT for p0 < p1 < p2 (Montgomery constants with their w').
+    PrimeInfo pr[kMaxPrimes];
+    uint32_t one_w[kMaxPrimes], one_wp[kMaxPrimes];  // Montgomery form of 1 (reduces any u32 mod p)
+    uint32_t red[kMaxPrimes];  // floor(2^32 / p): Shoup form of 1, reduces any u32 into [0, 2p)
+    const uint2* stage[kMaxPrimes][2];  // [prime][dir] Shoup pairs: entry h+m = omega_{2h}^{+-m}
+    const uint2* th[kMaxPrimes][2];     // Montgomery pairs: omega_{2^log_max}^{+-(i << split)}
+    const uint2* tl[kMaxPrimes][2];     // Montgomery pairs: omega_{2^log_max}^{+-i}
+    // Garner CRT of the three-prime sets, p0 < p1 < p2 (Montgomery constants with their w').
     uint32_t k1, k1p;  // p0^-1 mod p1
     uint32_t k2, k2p;  // p0 mod p2
     uint32_t k3, k3p;  // (p0 p1)^-1 mod p2
@@ -173,6 +173,7 @@ cudaError_t launch_ntt_mixed(const MixedArgs& m, const MixedSizes& sizes, cudaSt
 TransformShape choose_shape(int log_n);        // the tuned split (bgpu_set_split), else the built-in one
 TransformShape choose_shape_batch(int log_n);  // batch classes (bgpu_set_batch_split), else built-in
 TransformShape builtin_shape(int log_n);       // the built-in split only
+int tuned_split(int log_n);                    // the split set by bgpu_set_split, or 0
 int set_split(int log_n, int log_n2);  // 0 on success; log_n2 == 0 restores the default
 int set_batch_split(int log_n, int log_n2);
 bool shape_supported(int log_n, bool square);

@@ -40,7 +40,7 @@ void build_tables(int ps, int stage_log, uint2* host) {
     const size_t stage_n = (size_t)1 << stage_log;
     const size_t th_n = (size_t)1 << (s.log_max - s.split), tl_n = (size_t)1 << s.split;
     const size_t blk = table_block_entries(ps, stage_log);
-    for (int q = 0; q < kNumPrimes; ++q) {
+    for (int q = 0; q < s.np; ++q) {
         const uint32_t p = s.p[q];
         for (int dir = 0; dir < 2; ++dir) {
             uint2* base = host + (size_t)(q * 2 + dir) * blk;
@@ -112,7 +112,7 @@ NttConsts make_consts(int ps, int stage_log, const uint2* dev_tables) {
     const size_t stage_n = (size_t)1 << stage_log;
     const size_t th_n = (size_t)1 << (s.log_max - s.split);
     const size_t blk = table_block_entries(ps, stage_log);
-    for (int q = 0; q < kNumPrimes; ++q) {
+    for (int q = 0; q < s.np; ++q) {
         const uint32_t p = s.p[q];
         c.pr[q].p = p;
         c.pr[q].pinv = inv32(p);
@@ -127,6 +127,9 @@ NttConsts make_consts(int ps, int stage_log, const uint2* dev_tables) {
             c.tl[q][dir] = base + stage_n + th_n;
         }
     }
+    c.log_max = s.log_max;
+    c.split = s.split;
+    if (s.np != 3) return c;
     const uint32_t p0 = s.p[0], p1 = s.p[1], p2 = s.p[2];
     const uint2 k1 = mont_pair(pow_mod(p0, p1 - 2, p1), p1);
     const uint2 k2 = mont_pair(p0 % p2, p2);
@@ -135,8 +138,6 @@ NttConsts make_consts(int ps, int stage_log, const uint2* dev_tables) {
     c.k2 = k2.x, c.k2p = k2.y;
     c.k3 = k3.x, c.k3p = k3.y;
     c.m01 = (uint64_t)p0 * p1;
-    c.log_max = s.log_max;
-    c.split = s.split;
     return c;
 }
 

@@ -21,7 +21,7 @@ constexpr size_t table_block_entries(int ps, int stage_log) {
 }
 
 constexpr size_t table_entries(int ps, int stage_log) {
-    return (size_t)kNumPrimes * 2 * table_block_entries(ps, stage_log);
+    return (size_t)kPrimeSets[ps].np * 2 * table_block_entries(ps, stage_log);
 }
 
 // Fill `host` (table_entries(ps, stage_log) pairs).

@@ -1,0 +1,782 @@
+// Five-prime NTT product pipeline (see wide.h): four launches,
+//   1. k_wide_fwd   per (8-column tile, prime, operand): 64-bit digits reduced mod p, length-N2 DIF over
+//                   n2, times omega_N^(n1 k2)
+//   2. k_wide_rows  per (row, prime): length-N1 DIF of A's and B's row, pointwise product, DIT back,
+//                   times omega_N^-(n1 k2) and the scale, in place
+//   3. k_wide_inv   per (8-column tile, prime): length-N2 DIT, in place, to natural order
+//   4. k_wide_carry CRT of the five residues, 256-bit chunk sums and the carry scan
+// The transforms are those of ntt_kernels.cu.  The CRT is not Garner's: the
+// scale of the row pass carries (M/p)^-1, so a coefficient is a sum of five
+// residue-by-constant products less a multiple q of M found in single
+// precision, 20 wide multiply-adds; it runs in the carry kernel, so no chunk
+// sums go through memory.
+#include <cstring>
+
+#include "carry_common.cuh"
+#include "ntt_bodies.cuh"
+#include "wide.h"
+
+namespace bgpu {
+
+constexpr int kWideCols = 8;
+constexpr int kWideThreads = 256;  // of the column passes
+
+__constant__ NttConsts c_wide[2];  // lazy, strict
+
+__device__ __forceinline__ ProductDesc wide_product(const WideArgs& a, uint32_t i) {
+    return a.descs ? a.descs[i] : a.one;
+}
+
+// (hi 2^32 + lo + k p) / 2^32 with the k that clears the low word: one wide
+// multiply-add with a 64-bit addend.
+__device__ __forceinline__ uint32_t redc(uint32_t lo, uint32_t hi, uint32_t p, uint32_t np) {
+    uint32_t r;
+    asm("{.reg .u32 z;\n\t"
+        "mad.lo.cc.u32 z, %1, %2, %3;\n\t"
+        "madc.hi.u32 %0, %1, %2, %4;}"
+        : "=r"(r)
+        : "r"(lo * np), "r"(p), "r"(lo), "r"(hi));
+    return r;
+}
+// a w 2^-32 mod p, below 2p for any 32-bit a and w < p (np = -p^-1 mod 2^32).
+__device__ __forceinline__ uint32_t mont(uint32_t a, uint32_t w, uint32_t p, uint32_t np) {
+    const uint64_t t = (uint64_t)a * w;
+    return redc((uint32_t)t, (uint32_t)(t >> 32), p, np);
+}
+// Shoup pair (w, floor(w 2^32 / p)) of w, given r = w 2^32 mod p: the quotient
+// is (w 2^32 - r) / p = -r / p mod 2^32.
+__device__ __forceinline__ uint2 shoup_of(uint32_t r, uint32_t p, uint32_t np) {
+    return make_uint2(csub(redc(r, 0, p, np), p), r * np);
+}
+// x s b for Shoup pairs: lazily below 2p, or below p for the strict set.
+template <bool LAZY>
+__device__ __forceinline__ uint32_t shoup2(uint32_t x, uint2 s, uint2 b, uint32_t p) {
+    const uint32_t y = shoup_lazy(shoup_lazy(x, s.x, s.y, p), b.x, b.y, p);
+    return LAZY ? y : csub(y, p);
+}
+
+// ---- 1: forward columns -----------------------------------------------------------
+
+// 64-bit digit n of an operand (0 beyond its length).
+template <bool LIMB>
+__device__ __forceinline__ uint64_t load_digit64(const OperandDesc& in, uint32_t nd, uint32_t n) {
+    if (n >= nd) return 0;
+    if constexpr (LIMB) {
+        return __ldg(static_cast<const unsigned long long*>(in.ptr) + n);
+    } else {
+        const uint32_t* d = static_cast<const uint32_t*>(in.ptr);
+        const uint64_t bit = (uint64_t)n * 64;
+        const uint32_t i = (uint32_t)(bit / 28), sh = (uint32_t)(bit - (uint64_t)i * 28);  // sh in {0, 4, ..., 24}
+        uint64_t v = __ldg(d + i) >> sh;
+        if (i + 1 < in.nsrc) v |= (uint64_t)__ldg(d + i + 1) << (28 - sh);
+        if (i + 2 < in.nsrc) v |= (uint64_t)__ldg(d + i + 2) << (56 - sh);
+        if (sh > 20 && i + 3 < in.nsrc) v |= (uint64_t)__ldg(d + i + 3) << (84 - sh);
+        return v;
+    }
+}
+
+// Round 0: rows n2 = base + (j << LO) read from the operand.  A digit
+// becomes digit 2^-32 mod p (the scale of the row pass undoes it), in [0, 2p)
+// or [0, p).  HALF: the rows of the upper half of the transform are zero; they
+// are not loaded and the first stage is one multiply per pair.
+template <bool LAZY, int L2, int T, bool LIMB, bool HALF>
+__device__ __forceinline__ void wide_round0(const WideArgs& a, const OperandDesc& in, uint32_t nd, const NttConsts& c,
+                                            int q, uint32_t c0, uint32_t* sm) {
+    using Gr = Group<L2, kWideCols, 0>;
+    constexpr int R = Gr::R;
+    constexpr int D = 1 << (R - 1);
+    constexpr int NL = HALF ? D : (1 << R);
+    const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv, red = c.red[q];
+    const uint2* tw = c.stage[q][0];
+    const uint32_t stride = 1u << (Gr::LO + a.log_n1);
+#pragma unroll 2
+    for (int g = threadIdx.x; g < Gr::G; g += T) {
+        const Gr gr(g);
+        uint32_t x[1 << R];
+        uint64_t any = 0;
+        uint32_t n = c0 + gr.col + (gr.base << a.log_n1);
+#pragma unroll
+        for (int j = 0; j < NL; ++j, n += stride) {
+            const uint64_t v = load_digit64<LIMB>(in, nd, n);
+            any |= v;
+            uint32_t hi = (uint32_t)(v >> 32);
+            hi -= __umulhi(hi, red) * p;  // [0, 2p)
+            if (!LAZY) hi = csub(hi, p);
+            const uint32_t r = redc((uint32_t)v, hi, p, np);  // one p more
+            x[j] = LAZY ? csub(r, 2 * p) : csub(r, p);
+        }
+        if (any) {
+            if constexpr (HALF) {
+                const uint2* twb = tw + gr.base_low;
+#pragma unroll
+                for (int j = 0; j < D; ++j) {
+                    const uint2 w = __ldg(twb + (1u << Gr::HI) + ((uint32_t)j << Gr::LO));
+                    const uint32_t t = shoup_lazy(x[j], w.x, w.y, p);
+                    x[j + D] = LAZY ? t : csub(t, p);
+                }
+                dif_regs<LAZY, R, Gr::HI, Gr::LO, 1>(x, gr.base_low, tw, p);
+            } else {
+                dif_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, tw, p);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) x[j] = 0;
+        }
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j) sm[gr.at(j)] = x[j];
+    }
+}
+
+#ifndef BGPU_WIDE_COL_BLOCKS
+#define BGPU_WIDE_COL_BLOCKS(l2) ((l2) == 9 ? 8 : ((l2) == 10 ? 4 : 1))
+#endif
+
+template <bool LAZY, int L2, int T>
+__global__ void __launch_bounds__(T, BGPU_WIDE_COL_BLOCKS(L2)) k_wide_fwd(const WideArgs a) {
+    using P2 = Plan<L2>;
+    constexpr int NR = P2::nr, RL = P2::r(NR - 1), SROW = (1 << RL) + 1;
+    static_assert(NR > 1, "column passes of several rounds");
+    extern __shared__ __align__(16) uint32_t sm[];  // [2^L2][8] and the column powers
+    const NttConsts& c = c_wide[LAZY ? 0 : 1];
+    const int q = blockIdx.y, op = (int)(blockIdx.z % (uint32_t)a.nops);
+    const ProductDesc pd = wide_product(a, blockIdx.z / (uint32_t)a.nops);
+    const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
+    const uint2* tw = c.stage[q][0];
+    const OperandDesc in = op == 0 ? pd.op[0] : pd.op[1];
+    const uint32_t c0 = blockIdx.x * kWideCols;
+    const size_t nn = (size_t)1 << a.log_n;
+    uint32_t* y = pd.y + ((size_t)op * kWidePrimes + q) * nn;
+
+    // The last round's groups hold slots base + j of one column n1, whose
+    // inter-pass twiddle is omega_N^(n1 bitrev(base)) S^bitrev(j): sS[col][m]
+    // holds S^m = omega_N^(n1 m 2^(L2-RL)), rows padded against bank conflicts.
+    uint2* sS = reinterpret_cast<uint2*>(sm + (kWideCols << L2));
+    for (int t = threadIdx.x; t < (kWideCols << RL); t += T) {
+        const uint32_t col = (uint32_t)t >> RL, m = (uint32_t)t & ((1u << RL) - 1u);
+        sS[col * SROW + m] = shoup_of(
+            inter_twiddle(c, q, 0, (((c0 + col) * m) << (L2 - RL)) & (uint32_t)(nn - 1), a.log_n, p), p, np);
+    }
+    pdl_wait();
+    const uint32_t nd = wide_digits(in);
+    if (in.fmt == kFmtLimb64) {
+        if (2 * (size_t)nd <= nn)
+            wide_round0<LAZY, L2, T, true, true>(a, in, nd, c, q, c0, sm);
+        else
+            wide_round0<LAZY, L2, T, true, false>(a, in, nd, c, q, c0, sm);
+    } else {
+        if (2 * (size_t)nd <= nn)
+            wide_round0<LAZY, L2, T, false, true>(a, in, nd, c, q, c0, sm);
+        else
+            wide_round0<LAZY, L2, T, false, false>(a, in, nd, c, q, c0, sm);
+    }
+    __syncthreads();
+    dif_rounds<LAZY, L2, kWideCols, T, 1, NR - 2>(sm, tw, p, threadIdx.x);
+    using Gr = Group<L2, kWideCols, NR - 1>;
+#pragma unroll 2
+    for (int g = threadIdx.x; g < Gr::G; g += T) {
+        const Gr gr(g);
+        uint32_t x[1 << RL];
+#pragma unroll
+        for (int j = 0; j < (1 << RL); ++j) x[j] = sm[gr.at(j)];
+        dif_regs<LAZY, RL, Gr::HI, Gr::LO>(x, gr.base_low, tw, p);
+        const uint32_t n1 = c0 + gr.col;
+        const uint2 bw = shoup_of(
+            inter_twiddle(c, q, 0, (n1 * bitrev(gr.base, L2)) & (uint32_t)(nn - 1), a.log_n, p), p, np);
+        const uint2* srow = sS + gr.col * SROW;
+#pragma unroll
+        for (int j = 0; j < (1 << RL); ++j)
+            y[((size_t)gr.idx(j) << a.log_n1) + n1] = shoup2<LAZY>(x[j], srow[brev_c(j, RL)], bw, p);
+    }
+    pdl_trigger();  // late: an early trigger parks row-pass CTAs on SMs this pass still fills
+}
+
+// ---- 2: rows -----------------------------------------------------------------------
+
+#ifndef BGPU_WIDE_ROW_BLOCKS
+#define BGPU_WIDE_ROW_BLOCKS(l1, t) ((t) < 64 ? 1 : ((l1) <= 12 ? 1024 / (t) : ((l1) == 13 ? 768 / (t) : 1)))
+#endif
+
+template <bool LAZY, int L1, int T, bool SQR>
+__global__ void __launch_bounds__(T, BGPU_WIDE_ROW_BLOCKS(L1, T)) k_wide_rows(const WideArgs a) {
+    using P1 = Plan<L1>;
+    constexpr int NR = P1::nr;
+    constexpr int R0 = P1::r(0), LO0 = P1::lo(0);
+    static_assert(NR > 1, "rows of several rounds");
+    extern __shared__ __align__(16) uint32_t sm[];  // A's row, B's, the powers
+    const NttConsts& c = c_wide[LAZY ? 0 : 1];
+    uint32_t* sa = sm;
+    uint32_t* sb = sm + (1u << L1);
+    uint2* sT = reinterpret_cast<uint2*>(sm + ((SQR ? 1u : 2u) << L1));
+    const int q = blockIdx.y, tid = threadIdx.x;
+    const ProductDesc pd = wide_product(a, blockIdx.z);
+    const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
+    const uint2* twf = c.stage[q][0];
+    const uint2* twi = c.stage[q][1];
+    const size_t nn = (size_t)1 << a.log_n;
+    uint32_t* row_a = pd.y + q * nn + ((size_t)blockIdx.x << L1);
+    const uint32_t* row_b = row_a + kWidePrimes * nn;
+    const uint32_t k2 = bitrev(blockIdx.x, a.log_n - L1);
+    const uint32_t scale = q == 0 ? a.scale[0] : q == 1 ? a.scale[1] : q == 2 ? a.scale[2] : q == 3 ? a.scale[3] : a.scale[4];
+
+    // The last DIT round's groups hold n1 = base + (j << LO0): twiddle
+    // omega_N^-(k2 base) sT[j], sT[j] = omega_N^-(k2 j << LO0).
+    for (int t = tid; t < (1 << R0); t += T)
+        sT[t] = shoup_of(inter_twiddle(c, q, 1, ((k2 * (uint32_t)t) << LO0) & (uint32_t)(nn - 1), a.log_n, p), p, np);
+    __syncthreads();
+    pdl_wait();
+
+    mid_dif_row<LAZY, L1, T, false>(row_a, sa, twf, p);
+    if constexpr (!SQR) {
+        smem_round<LAZY, L1, 1, T, NR - 1, false>(sa, twf, p, tid);  // A's last DIF round
+        mid_dif_row<LAZY, L1, T, false>(row_b, sb, twf, p);
+    }
+    {  // the last DIF round of B (or A), the pointwise product, the first DIT round
+        using Gr = Group<L1, 1, NR - 1>;
+        constexpr int R = Gr::R;
+        const uint32_t* src = SQR ? sa : sb;
+#pragma unroll 1
+        for (int g = tid; g < Gr::G; g += T) {
+            const Gr gr(g);
+            uint32_t x[1 << R];
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) x[j] = src[gr.at(j)];
+            dif_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twf, p);
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) {
+                // below p for factors below p; below 2p for factors below 2p, 4p < 2^32
+                const uint32_t z = mont(x[j], SQR ? x[j] : sa[gr.at(j)], p, np);
+                x[j] = LAZY ? z : csub(z, p);
+            }
+            dit_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) sa[gr.at(j)] = x[j];
+        }
+    }
+    __syncthreads();
+    dit_rounds<LAZY, L1, 1, T, NR - 2, 1>(sa, twi, p, tid);
+    using Gr = Group<L1, 1, 0>;
+#pragma unroll 2
+    for (int g = tid; g < Gr::G; g += T) {
+        const Gr gr(g);
+        uint32_t x[1 << R0];
+#pragma unroll
+        for (int j = 0; j < (1 << R0); ++j) x[j] = sa[gr.at(j)];
+        dit_regs<LAZY, R0, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
+        const uint2 bw = shoup_of(
+            csub(mont(inter_twiddle(c, q, 1, (k2 * gr.base) & (uint32_t)(nn - 1), a.log_n, p), scale, p, np), p), p, np);
+#pragma unroll
+        for (int j = 0; j < (1 << R0); ++j) row_a[gr.idx(j)] = shoup2<LAZY>(x[j], sT[j], bw, p);
+    }
+    pdl_trigger();
+}
+
+// ---- 3: inverse columns ---------------------------------------------------------------
+
+template <bool LAZY, int L2, int T>
+__global__ void __launch_bounds__(T, BGPU_WIDE_COL_BLOCKS(L2)) k_wide_inv(const WideArgs a) {
+    using P2 = Plan<L2>;
+    constexpr int NR = P2::nr;
+    extern __shared__ __align__(16) uint32_t sm[];  // [2^L2][8]
+    const NttConsts& c = c_wide[LAZY ? 0 : 1];
+    const int q = blockIdx.y;
+    const uint32_t p = c.pr[q].p;
+    const uint2* twi = c.stage[q][1];
+    uint32_t* y = wide_product(a, blockIdx.z).y + ((size_t)q << a.log_n) + blockIdx.x * kWideCols;
+    pdl_wait();
+    {
+        using Gr = Group<L2, kWideCols, NR - 1>;
+        constexpr int R = Gr::R;
+#pragma unroll 2
+        for (int g = threadIdx.x; g < Gr::G; g += T) {
+            const Gr gr(g);
+            uint32_t x[1 << R];
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) x[j] = y[((size_t)gr.idx(j) << a.log_n1) + gr.col];
+            dit_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) sm[gr.at(j)] = x[j];
+        }
+    }
+    __syncthreads();
+    dit_rounds<LAZY, L2, kWideCols, T, NR - 2, 1>(sm, twi, p, threadIdx.x);
+    using Gr = Group<L2, kWideCols, 0>;
+    constexpr int R = Gr::R;
+#pragma unroll 2
+    for (int g = threadIdx.x; g < Gr::G; g += T) {
+        const Gr gr(g);
+        uint32_t x[1 << R];
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j) x[j] = sm[gr.at(j)];
+        dit_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j)
+            y[((size_t)gr.idx(j) << a.log_n1) + gr.col] = Bfly<LAZY>::reduce(x[j], p);
+    }
+    pdl_trigger();
+}
+
+// ---- 4: CRT and carries --------------------------------------------------------------
+
+// C += a b, 64 bits, with the carry out counted in k.
+__device__ __forceinline__ void mac_count(uint32_t a, uint32_t b, uint32_t (&C)[2], uint32_t& k) {
+    asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32 %2, %2, 0;"
+        : "+r"(C[0]), "+r"(C[1]), "+r"(k)
+        : "r"(a), "r"(b));
+}
+__device__ __forceinline__ void mac(uint32_t a, uint32_t b, uint32_t (&C)[2]) {
+    asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
+        "madc.hi.u32 %1, %2, %3, %1;"
+        : "+r"(C[0]), "+r"(C[1])
+        : "r"(a), "r"(b));
+}
+
+// Adds the coefficient with residues y (each below its p) to the words W[0..4],
+// W[4] taking the carry: sum y_i M/p_i - q M.  The five products of a 32-bit
+// limb of the M/p_i sum to a 64-bit column and a carry count (LAZY: the first
+// four, p < 2^30, cannot overflow).  q = floor(sum y_i / p_i) in single
+// precision from the top bits of y_i, put below an exponent byte: the float is
+// 2^23 + floor(y_i / 256), and c.bias takes the 2^23 out again.  x / M is below
+// 0.9 and the bias keeps 0.05 on either side, well above the rounding.  -q M
+// comes from a table in shared memory (`nqm`, five words a q): lanes with
+// different q hit different banks there, a constant bank would serve them one
+// by one (measured the constant bank: 29.5 us for the whole pass at 2^21 points, with the table 26.8).
+template <bool LAZY>
+__device__ __forceinline__ void add_crt5(const WideCrt& c, const uint32_t* nqm, const uint32_t (&y)[kWidePrimes],
+                                         uint32_t* W) {
+    float f = c.bias;
+#pragma unroll
+    for (int i = 0; i < kWidePrimes; ++i) f = fmaf(__uint_as_float(__byte_perm(y[i], 0x4b000000u, 0x7321)), c.inv[i], f);
+    const uint32_t* s = nqm + 5 * min((int)f, kWideMaxQ - 1);
+    uint32_t C[4][2], k[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        const uint64_t t = (uint64_t)y[0] * c.m[0][l];
+        C[l][0] = (uint32_t)t, C[l][1] = (uint32_t)(t >> 32);
+#pragma unroll
+        for (int i = 1; i < kWidePrimes; ++i) {
+            if (LAZY && i < 4)
+                mac(y[i], c.m[i][l], C[l]);
+            else
+                mac_count(y[i], c.m[i][l], C[l], k[l]);
+        }
+    }
+    // words of the sum: C0.lo | C0.hi + C1.lo | C1.hi + C2.lo + k0 | C2.hi + C3.lo + k1 | C3.hi + k2
+    asm("add.cc.u32 %0, %0, %5;\n\t"
+        "addc.cc.u32 %1, %1, %6;\n\t"
+        "addc.cc.u32 %2, %2, %7;\n\t"
+        "addc.cc.u32 %3, %3, %8;\n\t"
+        "addc.u32 %4, %4, %9;\n\t"
+        "add.cc.u32 %1, %1, %10;\n\t"
+        "addc.cc.u32 %2, %2, %11;\n\t"
+        "addc.cc.u32 %3, %3, %12;\n\t"
+        "addc.u32 %4, %4, %13;\n\t"
+        "add.cc.u32 %2, %2, %14;\n\t"
+        "addc.cc.u32 %3, %3, %15;\n\t"
+        "addc.u32 %4, %4, 0;\n\t"
+        "add.cc.u32 %0, %0, %16;\n\t"
+        "addc.cc.u32 %1, %1, %17;\n\t"
+        "addc.cc.u32 %2, %2, %18;\n\t"
+        "addc.cc.u32 %3, %3, %19;\n\t"
+        "addc.u32 %4, %4, %20;"
+        : "+r"(W[0]), "+r"(W[1]), "+r"(W[2]), "+r"(W[3]), "+r"(W[4])
+        : "r"(C[0][0]), "r"(C[1][0]), "r"(C[2][0]), "r"(C[3][0]), "r"(k[2]), "r"(C[0][1]), "r"(C[1][1]), "r"(C[2][1]),
+          "r"(C[3][1]), "r"(k[0]), "r"(k[1]), "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]));
+}
+
+__device__ __forceinline__ uint64_t add_c(uint64_t a, uint64_t b, uint32_t& cy) {
+    const uint64_t t = a + b, r = t + cy;
+    cy = (uint32_t)(t < a) + (uint32_t)(r < t);
+    return r;
+}
+
+// Chunk c (coefficients 4c .. 4c+3): their exact sum as 256 bits D and a
+// spill of two limbs (below 2^90).
+template <bool LAZY>
+__device__ __forceinline__ void chunk5(const WideCrt& crt, const uint32_t* nqm, const uint32_t* y, size_t nn, size_t c, uint64_t (&D)[4],
+                                       uint64_t (&sp)[2]) {
+    uint32_t r[4][kWidePrimes];
+#pragma unroll
+    for (int i = 0; i < kWidePrimes; ++i) {
+        const uint4 v = *reinterpret_cast<const uint4*>(y + i * nn + 4 * c);
+        r[0][i] = v.x, r[1][i] = v.y, r[2][i] = v.z, r[3][i] = v.w;
+    }
+    uint32_t W[12] = {};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        // the coefficient is added from word 2k; the words from 2k + 4 on are
+        // still zero, and the sum so far stays below 2^(64 k + 160)
+        add_crt5<LAZY>(crt, nqm, r[k], W + 2 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) D[k] = W[2 * k] | ((uint64_t)W[2 * k + 1] << 32);
+    sp[0] = W[8] | ((uint64_t)W[9] << 32);
+    sp[1] = W[10] | ((uint64_t)W[11] << 32);
+}
+
+// The 28-bit digits that start in chunk c, whose final limbs are S; the last
+// one may reach into the final low limb `next` of the chunk above.
+__device__ __forceinline__ void store_digits28(uint32_t* o, size_t out_cap, uint64_t c, const uint64_t (&S)[4],
+                                               uint64_t next) {
+    const uint64_t mask = (1u << 28) - 1u;
+    const uint64_t bit0 = c * 256;
+    uint64_t k = (bit0 + 27) / 28;
+    const uint64_t kend = min((bit0 + 256 + 27) / 28, (uint64_t)out_cap);
+    const uint32_t off0 = (uint32_t)(k * 28 - bit0);  // < 28
+    uint64_t cur = S[0] >> off0;
+    int have = 64 - (int)off0;
+#pragma unroll
+    for (int w = 1; w <= 4; ++w) {
+        const uint64_t nxtw = w < 4 ? S[w & 3] : next;
+        while (have >= 28) {
+            if (k < kend) o[k] = (uint32_t)(cur & mask);
+            ++k;
+            cur >>= 28;
+            have -= 28;
+        }
+        if (k < kend) o[k] = (uint32_t)((cur | (nxtw << have)) & mask);
+        ++k;
+        cur = nxtw >> (28 - have);
+        have = 36 + have;
+    }
+}
+
+// One 256-bit chunk a thread, 256 chunks a block; a ninth warp recomputes the
+// 32 chunks below the block, whose carries almost always settle the block's
+// carry-in without waiting for another block (else the decoupled look-back on
+// the blocks' flags, in ticket order).  Chunk c's value is
+// (D_c + spill_{c-1} + carry_c) mod 2^256 with one-bit carries.
+constexpr int kWideCarryWarps = kWideCarryChunks / 32;
+template <bool LAZY>
+__global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __grid_constant__ WideCarryArgs a) {
+    __shared__ uint32_t s_bid, s_cin, s_win_g, s_win_p;
+    __shared__ uint32_t s_wg[kWideCarryWarps], s_wp[kWideCarryWarps];
+    __shared__ uint64_t s_sp[kWideCarryWarps + 1][2];
+    __shared__ uint64_t s_low[kWideCarryChunks];  // 28-bit output: each chunk's low limb before its spill and carry
+    __shared__ uint32_t s_nqm[kWideMaxQ * 5];
+    if (threadIdx.x == 0) s_bid = (uint32_t)(atomicAdd(a.ticket, 1ull) - a.ticket_base);
+    for (int i = threadIdx.x; i < kWideMaxQ * 5; i += kWideCarryChunks + 32) s_nqm[i] = a.crt.nqm[i / 5][i % 5];
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    if (s_bid >= gridDim.x) {  // the ticket counter and the launch disagree: report, touch nothing
+        if (threadIdx.x == 0) atomicOr(a.err, 2u);
+        return;
+    }
+    const uint32_t bid = s_bid % a.bpp;
+    const ProductDesc pd = a.descs ? a.descs[s_bid / a.bpp] : a.one;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool window = warp == kWideCarryWarps;
+    const size_t nn = (size_t)1 << a.log_n;
+    const uint32_t nch = (uint32_t)(nn / 4);
+    const int64_t c = (int64_t)bid * kWideCarryChunks + (window ? lane - 32 : (int)threadIdx.x);
+    uint64_t S[4] = {0, 0, 0, 0}, sp[2] = {0, 0};
+    if (c >= 0 && c < nch) chunk5<LAZY>(a.crt, s_nqm, pd.y, nn, (size_t)c, S, sp);
+    if (!window) s_low[threadIdx.x] = S[0];
+    if (lane == 31) {
+        s_sp[warp][0] = sp[0];
+        s_sp[warp][1] = sp[1];
+    }
+    uint64_t p0 = __shfl_up_sync(0xffffffffu, sp[0], 1), p1 = __shfl_up_sync(0xffffffffu, sp[1], 1);
+    __syncthreads();
+    if (lane == 0) {
+        p0 = window ? 0 : s_sp[warp ? warp - 1 : kWideCarryWarps][0];
+        p1 = window ? 0 : s_sp[warp ? warp - 1 : kWideCarryWarps][1];
+    }
+    uint32_t g = 0;
+    S[0] = add_c(S[0], p0, g);
+    S[1] = add_c(S[1], p1, g);
+    S[2] = add_c(S[2], 0, g);
+    S[3] = add_c(S[3], 0, g);
+    const uint32_t pbit = (S[0] & S[1] & S[2] & S[3]) == ~0ull;
+    // the window's lowest chunk lacks its predecessor's spill: it neither
+    // stops nor makes a carry there, except below chunk 0
+    const uint32_t gm = __ballot_sync(0xffffffffu, g);
+    uint32_t pm = __ballot_sync(0xffffffffu, pbit);
+    if (window && bid != 0) pm |= 1u;
+    const uint32_t bm = gm | pm;
+    if (lane == 0) {
+        if (window) {
+            s_win_g = gm;
+            s_win_p = pm;
+        } else {
+            s_wg[warp] = (uint32_t)((((uint64_t)gm + bm) >> 32) & 1u);
+            s_wp[warp] = pm == 0xffffffffu;
+        }
+    }
+    __syncthreads();
+    // The block's flag holds all that a later block reads, so its stores need
+    // no ordering; the inclusive one comes after the barrier that releases the
+    // block's own threads.
+    uint32_t bG = 0, bP = 1, cin = 0;
+    if (threadIdx.x == 0) {
+        for (int w = 0; w < kWideCarryWarps; ++w) {
+            bG = s_wg[w] | (s_wp[w] & bG);
+            bP = bP & s_wp[w];
+        }
+        const uint32_t stop = ~s_win_p;  // window chunks that do not propagate a carry
+        if (bid == 0) {
+            bP = 0;
+        } else if (stop) {
+            cin = (s_win_g >> (31 - __clz(stop))) & 1u;
+        } else {
+            uint64_t* flags = pd.flags;
+            cuda::atomic_ref<unsigned long long, cuda::thread_scope_device>(
+                *reinterpret_cast<unsigned long long*>(flags + bid))
+                .store(make_flag(a.epoch, 1, bG, bP), cuda::memory_order_relaxed);
+            for (int k = (int)bid - 1;; --k) {  // block 0 is inclusive
+                const uint64_t f = wait_flag(flags + k, a.epoch, kSpinLimit, a.err);
+                if (f == 0) break;  // gave up: error recorded, carry taken as 0
+                const uint32_t st = (uint32_t)(f >> 2) & 3u, fg = (uint32_t)(f >> 1) & 1u, fp = (uint32_t)f & 1u;
+                if (st == 2 || fg || !fp) {
+                    cin = fg;
+                    break;
+                }
+            }
+        }
+        s_cin = cin;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        cuda::atomic_ref<unsigned long long, cuda::thread_scope_device>(
+            *reinterpret_cast<unsigned long long*>(pd.flags + bid))
+            .store(make_flag(a.epoch, 2, bG | (bP & cin), 0), cuda::memory_order_relaxed);
+    if (window) return;
+    uint32_t cw = s_cin;
+    for (int w = 0; w < warp; ++w) cw = s_wg[w] | (s_wp[w] & cw);
+    const uint64_t sum = (uint64_t)gm + bm + cw;
+    const uint32_t carries = (uint32_t)sum ^ gm ^ bm;
+    uint32_t cy = (carries >> lane) & 1u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint64_t t = S[k] + cy;
+        cy = cy & (t == 0);
+        S[k] = t;
+    }
+    if (a.out_fmt == kFmtLimb64) {
+        uint64_t* o = static_cast<uint64_t*>(pd.out);
+        const size_t at = (size_t)c * 4;
+        if (at + 4 <= pd.out_cap && (reinterpret_cast<uintptr_t>(o) & 15u) == 0) {
+            ulonglong2* d = reinterpret_cast<ulonglong2*>(o + at);
+            d[0] = make_ulonglong2(S[0], S[1]);
+            d[1] = make_ulonglong2(S[2], S[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (at + k < pd.out_cap) o[at + k] = S[k];
+        }
+    } else {
+        uint64_t next = 0;  // low limb of the next chunk: its raw sum, this chunk's spill and carry out
+        if (threadIdx.x + 1 < kWideCarryChunks) {
+            next = s_low[threadIdx.x + 1];
+        } else if (c + 1 < nch) {
+            uint32_t r[kWidePrimes], w[5] = {};
+#pragma unroll
+            for (int i = 0; i < kWidePrimes; ++i) r[i] = pd.y[i * nn + 4 * (size_t)(c + 1)];
+            add_crt5<LAZY>(a.crt, s_nqm, r, w);
+            next = w[0] | ((uint64_t)w[1] << 32);
+        }
+        next += sp[0] + (lane == 31 ? (uint32_t)(sum >> 32) & 1u : (carries >> (lane + 1)) & 1u);
+        store_digits28(static_cast<uint32_t*>(pd.out), pd.out_cap, (uint64_t)c, S, next);
+    }
+}
+
+// ---- launches ------------------------------------------------------------------------
+
+namespace {
+
+constexpr int wide_row_threads(int l1) { return l1 >= 12 ? 256 : (l1 >= 9 ? (1 << (l1 - 4)) : 32); }
+
+template <bool LAZY, int L2>
+cudaError_t launch_cols(bool fwd, const WideArgs& a, uint32_t count, cudaStream_t st) {
+    constexpr int RL = Plan<L2>::r(Plan<L2>::nr - 1);
+    const size_t tile = (size_t)kWideCols * 4 << L2;
+    const uint32_t tiles = (1u << a.log_n1) / kWideCols;
+    if (fwd) {
+        auto k = k_wide_fwd<LAZY, L2, kWideThreads>;
+        const size_t sm = tile + kWideCols * ((1 << RL) + 1) * sizeof(uint2);
+        allow_smem(k, sm);
+        return launch_k(k, dim3(tiles, kWidePrimes, count * a.nops), dim3(kWideThreads), sm, st, a);
+    }
+    auto k = k_wide_inv<LAZY, L2, kWideThreads>;
+    allow_smem(k, tile);
+    return launch_k(k, dim3(tiles, kWidePrimes, count), dim3(kWideThreads), tile, st, a);
+}
+
+template <bool LAZY>
+cudaError_t dispatch_cols(int l2, bool fwd, const WideArgs& a, uint32_t count, cudaStream_t st) {
+    switch (l2) {
+        case 5: return launch_cols<LAZY, 5>(fwd, a, count, st);
+        case 6: return launch_cols<LAZY, 6>(fwd, a, count, st);
+        case 7: return launch_cols<LAZY, 7>(fwd, a, count, st);
+        case 8: return launch_cols<LAZY, 8>(fwd, a, count, st);
+        case 9: return launch_cols<LAZY, 9>(fwd, a, count, st);
+        case 10: return launch_cols<LAZY, 10>(fwd, a, count, st);
+        case 11: return launch_cols<LAZY, 11>(fwd, a, count, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+template <bool LAZY, int L1>
+cudaError_t launch_rows(const WideArgs& a, bool square, uint32_t count, cudaStream_t st) {
+    constexpr int T = wide_row_threads(L1);
+    const dim3 grid(1u << (a.log_n - L1), kWidePrimes, count);
+    const size_t sm = ((square ? 1 : 2) * ((size_t)4 << L1)) + 16 * sizeof(uint2);
+    if (square) {
+        auto k = k_wide_rows<LAZY, L1, T, true>;
+        allow_smem(k, sm);
+        return launch_k(k, grid, dim3(T), sm, st, a);
+    }
+    auto k = k_wide_rows<LAZY, L1, T, false>;
+    allow_smem(k, sm);
+    return launch_k(k, grid, dim3(T), sm, st, a);
+}
+
+template <bool LAZY>
+cudaError_t dispatch_rows(int l1, const WideArgs& a, bool square, uint32_t count, cudaStream_t st) {
+    switch (l1) {
+        case 5: return launch_rows<LAZY, 5>(a, square, count, st);
+        case 6: return launch_rows<LAZY, 6>(a, square, count, st);
+        case 7: return launch_rows<LAZY, 7>(a, square, count, st);
+        case 8: return launch_rows<LAZY, 8>(a, square, count, st);
+        case 9: return launch_rows<LAZY, 9>(a, square, count, st);
+        case 10: return launch_rows<LAZY, 10>(a, square, count, st);
+        case 11: return launch_rows<LAZY, 11>(a, square, count, st);
+        case 12: return launch_rows<LAZY, 12>(a, square, count, st);
+        case 13: return launch_rows<LAZY, 13>(a, square, count, st);
+        case 14: return launch_rows<LAZY, 14>(a, square, count, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+WideCrt make_crt(const NttConsts& h) {
+    WideCrt c{};
+    double off = 0;
+    uint32_t M[5] = {1, 0, 0, 0, 0};
+    auto times = [](uint32_t (&x)[5], uint32_t v) {
+        uint64_t cy = 0;
+        for (auto& w : x) {
+            cy += (uint64_t)w * v;
+            w = (uint32_t)cy;
+            cy >>= 32;
+        }
+    };
+    for (int i = 0; i < kWidePrimes; ++i) {
+        uint32_t x[5] = {1, 0, 0, 0, 0};
+        for (int j = 0; j < kWidePrimes; ++j)
+            if (j != i) times(x, h.pr[j].p);
+        std::memcpy(c.m[i], x, sizeof(c.m[i]));
+        times(M, h.pr[i].p);
+        c.inv[i] = (float)(256.0 / h.pr[i].p);
+        off += 8388608.0 * (double)c.inv[i];
+    }
+    c.bias = (float)(0.05 - off);
+    for (int q = 0; q < kWideMaxQ; ++q) {
+        uint32_t x[5];
+        std::memcpy(x, M, sizeof(x));
+        times(x, (uint32_t)q);
+        uint64_t cy = 1;  // its negative
+        for (int k = 0; k < 5; ++k) {
+            cy += (uint32_t)~x[k];
+            c.nqm[q][k] = (uint32_t)cy;
+            cy >>= 32;
+        }
+    }
+    return c;
+}
+
+uint32_t pow_m(uint64_t b, uint32_t e, uint32_t p) {
+    uint64_t r = 1;
+    for (b %= p; e; e >>= 1, b = b * b % p)
+        if (e & 1) r = r * b % p;
+    return (uint32_t)r;
+}
+
+// 2^96 / N / (M / p) mod p, times 2^32: the digits' two factors 2^-32 and the
+// pointwise product's, the inverse transform's 1/N, the CRT's (M/p)^-1.
+void set_scale(const NttConsts& h, int log_n, uint32_t* scale) {
+    for (int i = 0; i < kWidePrimes; ++i) {
+        const uint32_t p = h.pr[i].p;
+        uint64_t d = pow_m(2, (uint32_t)log_n, p);
+        for (int j = 0; j < kWidePrimes; ++j)
+            if (j != i) d = d * (h.pr[j].p % p) % p;
+        const uint64_t v = (uint64_t)pow_m(d, p - 2, p) * pow_m(2, 96, p) % p;
+        scale[i] = (uint32_t)((v << 32) % p);
+    }
+}
+
+// Launch constants of each set and length, made once at upload.
+WideCrt g_crt[2];
+uint32_t g_scale[kWideMaxLogN + 1][kWidePrimes];
+
+}  // namespace
+
+cudaError_t upload_wide_consts(int set, const NttConsts& c) {
+    g_crt[set - 2] = make_crt(c);
+    for (int ln = kWideMinLogN; ln <= kWideMaxLogN; ++ln)
+        if (wide_set_for(ln) == set) set_scale(c, ln, g_scale[ln]);
+    return cudaMemcpyToSymbol(c_wide, &c, sizeof(NttConsts), (set - 2) * sizeof(NttConsts));
+}
+
+// Built-in column lengths, the fastest measured on B200 (products of two
+// operands of half the points, 64-bit digits, us back to back against the next
+// length up or down): 2^17 points 23.8 (2^8) / 24.4 (2^7), 2^19 52.4 (2^9) /
+// 54.7 (2^8), 2^20 92.9 (2^9) / 94.5 (2^10), 2^21 178.7 (2^10) / 183.5 (2^9),
+// 2^23 798 (2^10) / 916 (2^11), 2^24 1890 (2^11) / 1963 (2^10).
+static constexpr int8_t kWideColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0,  0,  0,  5,  6,  7,
+                                                         7, 8, 7, 6, 8, 8, 9, 9, 10, 10, 10, 11, 11};
+
+TransformShape wide_shape(int log_n) {
+    TransformShape s{log_n, 0, 0};
+    if (log_n < kWideMinLogN || log_n > kWideMaxLogN) return s;
+    auto built = [&](int l2) { return l2 >= 5 && l2 <= 11 && log_n - l2 >= 5 && log_n - l2 <= 14; };
+    const int tuned = tuned_split(log_n + 1);
+    s.log_n2 = built(tuned) ? tuned : kWideColumn[log_n];
+    s.log_n1 = log_n - s.log_n2;
+    return s;
+}
+
+const char* const kWideKernelNames[kNttLaunches] = {"k_wide_fwd", "k_wide_rows", "k_wide_inv", "k_wide_carry"};
+
+cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs, const ProductDesc& one,
+                                uint32_t count, bool square, int log_n, int out_fmt, uint32_t bpp,
+                                const CarryLaunch& cl, cudaStream_t st, cudaEvent_t* ev) {
+    const int l2 = wide_shape(log_n).log_n2;
+    if (!l2 || log_n > host.log_max || count < 1) return cudaErrorInvalidValue;
+    const bool lazy = host.log_max == kPrimeSets[2].log_max;
+    WideArgs a{};
+    a.descs = descs;
+    a.one = one;
+    a.nops = square ? 1 : 2;
+    a.log_n = log_n;
+    a.log_n1 = log_n - l2;
+    std::memcpy(a.scale, g_scale[log_n], sizeof(a.scale));
+    if (ev) cudaEventRecord(ev[0], st);
+    cudaError_t e = lazy ? dispatch_cols<true>(l2, true, a, count, st) : dispatch_cols<false>(l2, true, a, count, st);
+    if (e != cudaSuccess) return e;
+    if (ev) cudaEventRecord(ev[1], st);
+    e = lazy ? dispatch_rows<true>(a.log_n1, a, square, count, st) : dispatch_rows<false>(a.log_n1, a, square, count, st);
+    if (e != cudaSuccess) return e;
+    if (ev) cudaEventRecord(ev[2], st);
+    e = lazy ? dispatch_cols<true>(l2, false, a, count, st) : dispatch_cols<false>(l2, false, a, count, st);
+    if (e != cudaSuccess) return e;
+    if (ev) cudaEventRecord(ev[3], st);
+    WideCarryArgs ca{};
+    ca.descs = descs;
+    ca.one = one;
+    ca.crt = g_crt[lazy ? 0 : 1];
+    ca.log_n = log_n;
+    ca.out_fmt = out_fmt;
+    ca.bpp = bpp;
+    ca.ticket = cl.ticket;
+    ca.ticket_base = cl.ticket_base;
+    ca.epoch = cl.epoch;
+    ca.err = cl.err;
+    e = launch_k(lazy ? k_wide_carry<true> : k_wide_carry<false>, dim3(bpp * count), dim3(kWideCarryChunks + 32), 0, st,
+                 ca);
+    if (ev) cudaEventRecord(ev[4], st);
+    return e;
+}
+
+}  // namespace bgpu

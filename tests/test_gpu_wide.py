@@ -1,0 +1,103 @@
+"""Five-prime products (64-bit digits) at the edges of their dispatch: lengths
+around powers of two, operands longer than half the transform, long runs of
+propagating carries, unaligned buffers, 28-bit Digits, both prime sets."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import SEED
+
+pytestmark = pytest.mark.gpu
+
+ONES = np.uint64(0xFFFFFFFFFFFFFFFF)
+M61 = (1 << 61) - 1
+
+
+def rand_limbs(rng, n):
+    a = rng.integers(0, 2**64, n, dtype=np.uint64)
+    a[-1] |= np.uint64(1 << 63)
+    return a
+
+
+def mod61(x):
+    return int.from_bytes(np.ascontiguousarray(x).tobytes(), "little") % M61
+
+
+@pytest.fixture(scope="module")
+def bb():
+    import bigint_b200
+
+    bigint_b200.init(0)
+    return bigint_b200
+
+
+# total limbs around 2^k + 1 (the longest product of a 2^k-point transform) and
+# around the shortest transform; the long operand of the second pair fills more
+# than half of the points
+@pytest.mark.parametrize("log_n", [9, 10, 11, 13, 14, 16, 18])
+@pytest.mark.parametrize("extra", [0, 1, 2])
+def test_length_edges(bb, port, log_n, extra):
+    rng = np.random.default_rng([SEED, log_n, extra])
+    total = (1 << log_n) + extra
+    for na in (total // 2, total - 5, total - total // 3):
+        a, b = rand_limbs(rng, na), rand_limbs(rng, total - na)
+        assert np.array_equal(bb.ntt_mul(a, b), port.mul(a, b)), (na, total - na)
+    a = rand_limbs(rng, total // 2)
+    assert np.array_equal(bb.ntt_mul(a), port.mul(a, a))
+
+
+@pytest.mark.parametrize("n", [1500, 70000])
+def test_propagating_carries(bb, port, n):
+    """Products whose chunks all propagate a carry or stop it only at the ends."""
+    ones = np.full(n, ONES)
+    one = np.array([1], dtype=np.uint64)
+    assert np.array_equal(bb.ntt_mul(ones, one), ones)
+    assert np.array_equal(bb.ntt_mul(ones), port.mul(ones, ones))
+    a = np.full(n, ONES)
+    a[0] = 1  # (B^n - B + 1)(B^(n/2) + 1): runs of ones met by a carry
+    b = np.zeros(n // 2 + 1, dtype=np.uint64)
+    b[0] = b[-1] = 1
+    assert np.array_equal(bb.ntt_mul(a, b), port.mul(a, b))
+
+
+def test_unaligned_device_buffers(bb, port):
+    import torch
+
+    rng = np.random.default_rng(SEED + 3)
+    a, b = rand_limbs(rng, 3001), rand_limbs(rng, 1777)
+    ta = torch.zeros(3002, dtype=torch.int64, device="cuda")
+    tb = torch.zeros(1778, dtype=torch.int64, device="cuda")
+    out = torch.full((3001 + 1777 + 2,), -1, dtype=torch.int64, device="cuda")
+    ta[1:] = torch.from_numpy(a.view(np.int64))
+    tb[1:] = torch.from_numpy(b.view(np.int64))
+    st = torch.cuda.current_stream().cuda_stream
+    bb.mul_device(ta.data_ptr() + 8, a.size, tb.data_ptr() + 8, b.size, out.data_ptr() + 8, st)
+    bb.device_status(st)
+    got = out.cpu().numpy().view(np.uint64)
+    want = port.mul(a, b)
+    assert np.array_equal(got[1 : 1 + want.size], want)
+    assert got[0] == ONES and got[-1] == ONES  # nothing written outside the product
+
+
+@pytest.mark.parametrize("na,nb", [(2500, 2300), (40000, 37450), (150000, 20000), (131073, 131071)])
+def test_digits28(bb, port, na, nb):
+    rng = np.random.default_rng([SEED, na])
+    a = rng.integers(0, 1 << 28, na).astype(np.uint32)
+    b = rng.integers(0, 1 << 28, nb).astype(np.uint32)
+    a[-1] |= 1 << 27
+    b[-1] |= 1
+    assert np.array_equal(bb.mul_digits(a, b), port.mul_digits(a, b))
+    full = np.full(na, (1 << 28) - 1, dtype=np.uint32)
+    assert np.array_equal(bb.mul_digits(full, b), port.mul_digits(full, b))
+
+
+@pytest.mark.parametrize("log_n", [22, 23, 24])
+def test_large_residue(bb, log_n):
+    """The longest lazy transform and the shorter strict ones, modulo 2^61 - 1."""
+    rng = np.random.default_rng([SEED, log_n, 61])
+    total = 1 << log_n
+    for na in (total // 2, total - total // 4 + 3):
+        a, b = rand_limbs(rng, na), np.full(total - na, ONES)
+        c = bb.ntt_mul(a, b)
+        assert mod61(c) == mod61(a) * mod61(b) % M61, (na, total - na)
