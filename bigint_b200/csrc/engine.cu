@@ -238,7 +238,7 @@ int prepare_scratch(int log_n, bool square, ProductScratch* s) {
 // the three-prime one.
 int wide_log(const OperandDesc& a, const OperandDesc& b) {
     const int ln = ceil_log2((uint64_t)wide_digits(a) + wide_digits(b) - 1);
-    return ln <= kWideMaxLogN && wide_shape(ln).log_n2 ? ln : 0;
+    return ln <= kWideMaxLogN && wide_shape(ln, false).log_n2 ? ln : 0;
 }
 
 // Product of two device operands on the five-prime transform.

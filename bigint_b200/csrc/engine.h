@@ -173,7 +173,7 @@ cudaError_t launch_ntt_mixed(const MixedArgs& m, const MixedSizes& sizes, cudaSt
 TransformShape choose_shape(int log_n);        // the tuned split (bgpu_set_split), else the built-in one
 TransformShape choose_shape_batch(int log_n);  // batch classes (bgpu_set_batch_split), else built-in
 TransformShape builtin_shape(int log_n);       // the built-in split only
-int tuned_split(int log_n);                    // the split set by bgpu_set_split, or 0
+int tuned_split(int log_n, bool batch);        // the split set by bgpu_set_split or bgpu_set_batch_split, or 0
 int set_split(int log_n, int log_n2);  // 0 on success; log_n2 == 0 restores the default
 int set_batch_split(int log_n, int log_n2);
 bool shape_supported(int log_n, bool square);

@@ -1044,7 +1044,9 @@ static int set_split_in(int* table, int log_n, int log_n2) {
 int set_split(int log_n, int log_n2) { return set_split_in(g_split, log_n, log_n2); }
 int set_batch_split(int log_n, int log_n2) { return set_split_in(g_batch_split, log_n, log_n2); }
 
-int tuned_split(int log_n) { return log_n >= 0 && log_n <= kMaxLogN ? g_split[log_n] : 0; }
+int tuned_split(int log_n, bool batch) {
+    return log_n >= 0 && log_n <= kMaxLogN ? (batch ? g_batch_split : g_split)[log_n] : 0;
+}
 
 TransformShape builtin_shape(int log_n) {
     TransformShape s;

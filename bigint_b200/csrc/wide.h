@@ -48,15 +48,15 @@ struct WideCarryArgs {
 
 constexpr uint32_t kWideCarryChunks = 256;  // 256-bit chunks per carry block
 // Carry blocks of a product with out_cap output elements.
-inline uint32_t wide_carry_blocks(size_t out_cap, int out_fmt) {
+__host__ __device__ inline uint32_t wide_carry_blocks(size_t out_cap, int out_fmt) {
     const uint64_t limbs = out_fmt == kFmtLimb64 ? out_cap : ((uint64_t)out_cap * 28 + 63) / 64;
     return (uint32_t)((limbs + 4 * kWideCarryChunks - 1) / (4 * kWideCarryChunks));
 }
 
 // Split of 2^log_n 64-bit digits: the tuned one of 2^(log_n + 1) 32-bit digits
-// (bgpu_set_split) where its kernels are built, else the built-in one.
-// log_n2 == 0: none is built.
-TransformShape wide_shape(int log_n);
+// (bgpu_set_split, bgpu_set_batch_split) where its kernels are built, else the
+// built-in one.  log_n2 == 0: no five-prime transform of this length.
+TransformShape wide_shape(int log_n, bool batch);
 cudaError_t upload_wide_consts(int set, const NttConsts& c);
 extern const char* const kWideKernelNames[kNttLaunches];
 
@@ -66,5 +66,10 @@ extern const char* const kWideKernelNames[kNttLaunches];
 cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs, const ProductDesc& one,
                                 uint32_t count, bool square, int log_n, int out_fmt, uint32_t bpp,
                                 const CarryLaunch& cl, cudaStream_t st, cudaEvent_t* ev);
+
+// The same for any number of products in the device array `descs`, in pieces
+// that fit a launch grid, all on one ticket sequence from cl.ticket_base.
+cudaError_t launch_wide_batch(const NttConsts& host, const ProductDesc* descs, uint32_t count, bool square, int log_n,
+                              int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st);
 
 }  // namespace bgpu

@@ -19,7 +19,25 @@
 namespace bgpu {
 
 constexpr int kWideCols = 8;
-constexpr int kWideThreads = 256;  // of the column passes
+// Threads of the column passes: the groups of a round (8 columns of 2^L2 / 8 or
+// 2^L2 / 16), so that short columns leave no thread idle: forward and inverse
+// pass per 2^19 points of a batch, columns of 2^6 rows 28.0 + 10.8 -> 14.2 + 5.5 us,
+// of 2^8 rows 16.8 + 9.1 -> 13.3 + 5.2 us against 256 threads throughout.
+__host__ __device__ constexpr int wide_col_threads(int l2) {
+    return l2 <= 5 ? 32 : l2 <= 7 ? 64 : l2 == 8 ? 128 : 256;
+}
+// Row pass: threads of a row and rows of a CTA.  Short rows have fewer groups
+// than a warp has lanes (16 at 2^8 points), so a CTA takes several side by
+// side: per 2^19 points of a batch, rows of 2^8 points 23.5 -> 12.7 us, of 2^7
+// points 34.8 -> 11.7 us, of 2^6 42.6 -> 11.3 us against one 32-thread CTA a row.
+__host__ __device__ constexpr int wide_row_threads(int l1) {
+    return l1 >= 12 ? 256 : l1 >= 9 ? (1 << (l1 - 4)) : l1 == 8 ? 16 : 8;
+}
+__host__ __device__ constexpr int wide_rows_per_cta(int l1) { return l1 >= 10 ? 1 : 128 / wide_row_threads(l1); }
+// Shared words of a row: its buffers and 16 Shoup pairs, a warp's rows in different banks.
+__host__ __device__ constexpr uint32_t wide_row_words(int l1, bool square) {
+    return ((square ? 1u : 2u) << l1) + 32u + (l1 >= 10 ? 0u : (uint32_t)wide_row_threads(l1) % 32u);
+}
 
 __constant__ NttConsts c_wide[2];  // lazy, strict
 
@@ -127,8 +145,11 @@ __device__ __forceinline__ void wide_round0(const WideArgs& a, const OperandDesc
     }
 }
 
+// CTAs per SM (register caps): 1024 threads' worth of 64 registers, except
+// columns of 2^9 rows at 1280 (2^19 points of a batch: 15.0 + 5.7 us; at 1024
+// 15.5 + 6.2, at 2048 15.1 + 5.9) and of 2^11 rows, whose tiles leave room for two.
 #ifndef BGPU_WIDE_COL_BLOCKS
-#define BGPU_WIDE_COL_BLOCKS(l2) ((l2) == 9 ? 8 : ((l2) == 10 ? 4 : 1))
+#define BGPU_WIDE_COL_BLOCKS(l2) ((l2) == 9 ? 5 : ((l2) == 11 ? 1 : 1024 / wide_col_threads(l2)))
 #endif
 
 template <bool LAZY, int L2, int T>
@@ -192,30 +213,38 @@ __global__ void __launch_bounds__(T, BGPU_WIDE_COL_BLOCKS(L2)) k_wide_fwd(const 
 
 // ---- 2: rows -----------------------------------------------------------------------
 
+// Rows of 2^8 points spill at 64 registers and run five CTAs of 128 threads
+// (14.1 -> 12.7 us per 2^19 points), 2^9 points six.
 #ifndef BGPU_WIDE_ROW_BLOCKS
-#define BGPU_WIDE_ROW_BLOCKS(l1, t) ((t) < 64 ? 1 : ((l1) <= 12 ? 1024 / (t) : ((l1) == 13 ? 768 / (t) : 1)))
+#define BGPU_WIDE_ROW_BLOCKS(l1, t) ((l1) == 8 ? 5 : (l1) == 9 ? 6 : ((l1) <= 12 ? 1024 / (t) : ((l1) == 13 ? 768 / (t) : 1)))
 #endif
 
-template <bool LAZY, int L1, int T, bool SQR>
-__global__ void __launch_bounds__(T, BGPU_WIDE_ROW_BLOCKS(L1, T)) k_wide_rows(const WideArgs a) {
+template <bool LAZY, int L1, bool SQR>
+__global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1),
+                                  BGPU_WIDE_ROW_BLOCKS(L1, wide_row_threads(L1) * wide_rows_per_cta(L1)))
+    k_wide_rows(const WideArgs a) {
+    constexpr int T = wide_row_threads(L1);
+    constexpr bool MULTI = wide_rows_per_cta(L1) > 1;
     using P1 = Plan<L1>;
     constexpr int NR = P1::nr;
     constexpr int R0 = P1::r(0), LO0 = P1::lo(0);
     static_assert(NR > 1, "rows of several rounds");
-    extern __shared__ __align__(16) uint32_t sm[];  // A's row, B's, the powers
+    extern __shared__ __align__(16) uint32_t sm[];  // per row: A's row, B's, the powers
     const NttConsts& c = c_wide[LAZY ? 0 : 1];
-    uint32_t* sa = sm;
-    uint32_t* sb = sm + (1u << L1);
-    uint2* sT = reinterpret_cast<uint2*>(sm + ((SQR ? 1u : 2u) << L1));
-    const int q = blockIdx.y, tid = threadIdx.x;
+    const uint32_t sub = MULTI ? threadIdx.x / T : 0u;
+    uint32_t* sa = sm + sub * wide_row_words(L1, SQR);
+    uint32_t* sb = sa + (1u << L1);
+    uint2* sT = reinterpret_cast<uint2*>(sa + ((SQR ? 1u : 2u) << L1));
+    const int q = blockIdx.y, tid = sub_tid<T, MULTI>();
+    const uint32_t slot = blockIdx.x * wide_rows_per_cta(L1) + sub;
     const ProductDesc pd = wide_product(a, blockIdx.z);
     const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
     const uint2* twf = c.stage[q][0];
     const uint2* twi = c.stage[q][1];
     const size_t nn = (size_t)1 << a.log_n;
-    uint32_t* row_a = pd.y + q * nn + ((size_t)blockIdx.x << L1);
+    uint32_t* row_a = pd.y + q * nn + ((size_t)slot << L1);
     const uint32_t* row_b = row_a + kWidePrimes * nn;
-    const uint32_t k2 = bitrev(blockIdx.x, a.log_n - L1);
+    const uint32_t k2 = bitrev(slot, a.log_n - L1);
     const uint32_t scale = q == 0 ? a.scale[0] : q == 1 ? a.scale[1] : q == 2 ? a.scale[2] : q == 3 ? a.scale[3] : a.scale[4];
 
     // The last DIT round's groups hold n1 = base + (j << LO0): twiddle
@@ -225,10 +254,10 @@ __global__ void __launch_bounds__(T, BGPU_WIDE_ROW_BLOCKS(L1, T)) k_wide_rows(co
     __syncthreads();
     pdl_wait();
 
-    mid_dif_row<LAZY, L1, T, false>(row_a, sa, twf, p);
+    mid_dif_row<LAZY, L1, T, MULTI>(row_a, sa, twf, p);
     if constexpr (!SQR) {
         smem_round<LAZY, L1, 1, T, NR - 1, false>(sa, twf, p, tid);  // A's last DIF round
-        mid_dif_row<LAZY, L1, T, false>(row_b, sb, twf, p);
+        mid_dif_row<LAZY, L1, T, MULTI>(row_b, sb, twf, p);
     }
     {  // the last DIF round of B (or A), the pointwise product, the first DIT round
         using Gr = Group<L1, 1, NR - 1>;
@@ -466,6 +495,8 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
     }
     const uint32_t bid = s_bid % a.bpp;
     const ProductDesc pd = a.descs ? a.descs[s_bid / a.bpp] : a.one;
+    // a product of a batch shorter than its class's longest: no later block waits on these
+    if (bid >= wide_carry_blocks(pd.out_cap, a.out_fmt)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool window = warp == kWideCarryWarps;
     const size_t nn = (size_t)1 << a.log_n;
@@ -586,22 +617,20 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
 
 namespace {
 
-constexpr int wide_row_threads(int l1) { return l1 >= 12 ? 256 : (l1 >= 9 ? (1 << (l1 - 4)) : 32); }
-
 template <bool LAZY, int L2>
 cudaError_t launch_cols(bool fwd, const WideArgs& a, uint32_t count, cudaStream_t st) {
     constexpr int RL = Plan<L2>::r(Plan<L2>::nr - 1);
     const size_t tile = (size_t)kWideCols * 4 << L2;
     const uint32_t tiles = (1u << a.log_n1) / kWideCols;
     if (fwd) {
-        auto k = k_wide_fwd<LAZY, L2, kWideThreads>;
+        auto k = k_wide_fwd<LAZY, L2, wide_col_threads(L2)>;
         const size_t sm = tile + kWideCols * ((1 << RL) + 1) * sizeof(uint2);
         allow_smem(k, sm);
-        return launch_k(k, dim3(tiles, kWidePrimes, count * a.nops), dim3(kWideThreads), sm, st, a);
+        return launch_k(k, dim3(tiles, kWidePrimes, count * a.nops), dim3(wide_col_threads(L2)), sm, st, a);
     }
-    auto k = k_wide_inv<LAZY, L2, kWideThreads>;
+    auto k = k_wide_inv<LAZY, L2, wide_col_threads(L2)>;
     allow_smem(k, tile);
-    return launch_k(k, dim3(tiles, kWidePrimes, count), dim3(kWideThreads), tile, st, a);
+    return launch_k(k, dim3(tiles, kWidePrimes, count), dim3(wide_col_threads(L2)), tile, st, a);
 }
 
 template <bool LAZY>
@@ -618,19 +647,17 @@ cudaError_t dispatch_cols(int l2, bool fwd, const WideArgs& a, uint32_t count, c
     }
 }
 
+template <bool LAZY, int L1, bool SQR>
+cudaError_t launch_rows_of(const WideArgs& a, uint32_t count, cudaStream_t st) {
+    constexpr int RP = wide_rows_per_cta(L1);
+    const size_t sm = (size_t)RP * wide_row_words(L1, SQR) * 4;
+    auto k = k_wide_rows<LAZY, L1, SQR>;
+    allow_smem(k, sm);
+    return launch_k(k, dim3((1u << (a.log_n - L1)) / RP, kWidePrimes, count), dim3(wide_row_threads(L1) * RP), sm, st, a);
+}
 template <bool LAZY, int L1>
 cudaError_t launch_rows(const WideArgs& a, bool square, uint32_t count, cudaStream_t st) {
-    constexpr int T = wide_row_threads(L1);
-    const dim3 grid(1u << (a.log_n - L1), kWidePrimes, count);
-    const size_t sm = ((square ? 1 : 2) * ((size_t)4 << L1)) + 16 * sizeof(uint2);
-    if (square) {
-        auto k = k_wide_rows<LAZY, L1, T, true>;
-        allow_smem(k, sm);
-        return launch_k(k, grid, dim3(T), sm, st, a);
-    }
-    auto k = k_wide_rows<LAZY, L1, T, false>;
-    allow_smem(k, sm);
-    return launch_k(k, grid, dim3(T), sm, st, a);
+    return square ? launch_rows_of<LAZY, L1, true>(a, count, st) : launch_rows_of<LAZY, L1, false>(a, count, st);
 }
 
 template <bool LAZY>
@@ -719,20 +746,25 @@ cudaError_t upload_wide_consts(int set, const NttConsts& c) {
     return cudaMemcpyToSymbol(c_wide, &c, sizeof(NttConsts), (set - 2) * sizeof(NttConsts));
 }
 
-// Built-in column lengths, the fastest measured on B200 (products of two
-// operands of half the points, 64-bit digits, us back to back against the next
-// length up or down): 2^17 points 23.8 (2^8) / 24.4 (2^7), 2^19 52.4 (2^9) /
-// 54.7 (2^8), 2^20 92.9 (2^9) / 94.5 (2^10), 2^21 178.7 (2^10) / 183.5 (2^9),
-// 2^23 798 (2^10) / 916 (2^11), 2^24 1890 (2^11) / 1963 (2^10).
-static constexpr int8_t kWideColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0,  0,  0,  5,  6,  7,
-                                                         7, 8, 7, 6, 8, 8, 9, 9, 10, 10, 10, 11, 11};
+// Built-in column lengths, the fastest measured on B200 for one product and
+// for a batch that fills the GPU (two operands of half the points).  us per
+// product back to back, the choice against the nearest other length: 2^12
+// points 9.8 (2^6) / 11.3 (2^7), 2^17 21.0 (2^6) / 22.2 (2^7), 2^18 28.9 (2^8) /
+// 29.8 (2^7), 2^19 47.7 (2^8) / 49.5 (2^9), 2^20 88.7 (2^8) / 90.4 (2^9), 2^21 175.7
+// (2^10) / 180.5 (2^9), 2^23 777 (2^10) / 900 (2^11), 2^24 1852 (2^11) / 1919 (2^10).
+// Batches, us per 2^19 points: 2^13 33.7 (2^7) / 35.7 (2^6), 2^15 34.5 (2^8) /
+// 35.4 (2^7), 2^17 37.8 (2^9) / 38.8 (2^8), 2^19 38.7 (2^8) / 40.4 (2^9).
+static constexpr int8_t kWideColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  5,  6,  6,
+                                                         7, 8, 8, 8, 6, 8, 8, 8, 10, 10, 10, 11, 11};
+static constexpr int8_t kWideBatchColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  5,  6,  6,
+                                                              7, 8, 8, 8, 9, 8, 8, 9, 10, 10, 10, 11, 11};
 
-TransformShape wide_shape(int log_n) {
+TransformShape wide_shape(int log_n, bool batch) {
     TransformShape s{log_n, 0, 0};
     if (log_n < kWideMinLogN || log_n > kWideMaxLogN) return s;
     auto built = [&](int l2) { return l2 >= 5 && l2 <= 11 && log_n - l2 >= 5 && log_n - l2 <= 14; };
-    const int tuned = tuned_split(log_n + 1);
-    s.log_n2 = built(tuned) ? tuned : kWideColumn[log_n];
+    const int tuned = tuned_split(log_n + 1, batch);
+    s.log_n2 = built(tuned) ? tuned : (batch ? kWideBatchColumn : kWideColumn)[log_n];
     s.log_n1 = log_n - s.log_n2;
     return s;
 }
@@ -742,7 +774,7 @@ const char* const kWideKernelNames[kNttLaunches] = {"k_wide_fwd", "k_wide_rows",
 cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs, const ProductDesc& one,
                                 uint32_t count, bool square, int log_n, int out_fmt, uint32_t bpp,
                                 const CarryLaunch& cl, cudaStream_t st, cudaEvent_t* ev) {
-    const int l2 = wide_shape(log_n).log_n2;
+    const int l2 = wide_shape(log_n, descs != nullptr).log_n2;
     if (!l2 || log_n > host.log_max || count < 1) return cudaErrorInvalidValue;
     const bool lazy = host.log_max == kPrimeSets[2].log_max;
     WideArgs a{};
@@ -777,6 +809,20 @@ cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs,
                  ca);
     if (ev) cudaEventRecord(ev[4], st);
     return e;
+}
+
+cudaError_t launch_wide_batch(const NttConsts& host, const ProductDesc* descs, uint32_t count, bool square, int log_n,
+                              int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st) {
+    constexpr uint32_t kPiece = 16384;  // grid z limit 65535, two operands a product
+    for (uint32_t done = 0; done < count; done += kPiece) {
+        CarryLaunch piece = cl;
+        piece.ticket_base = cl.ticket_base + (uint64_t)done * bpp;
+        const uint32_t n = count - done < kPiece ? count - done : kPiece;
+        const cudaError_t e = launch_wide_product(host, descs + done, ProductDesc{}, n, square, log_n, out_fmt, bpp,
+                                                  piece, st, nullptr);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace bgpu
