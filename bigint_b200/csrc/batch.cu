@@ -22,14 +22,25 @@
 
 #include "../../include/bigint_b200.h"
 #include "engine.h"
+#include "wide.h"
 
 namespace bgpu {
 
 // ---- plans -------------------------------------------------------------------
 
+// Classes of 2^14 32-bit digits and more (2^13 points of 64-bit digits) always
+// take the five-prime kernels: their launches fill the GPU on their own (4096
+// products of 2^10..2^22 bits: 10.60 ms with every class in the mixed-length
+// launches, 6.41 ms so, 6.49 with the long classes one after another instead of
+// on graph branches).  Shorter ones do when they cannot share the mixed-length
+// launches, which are one launch per pass for any number of lengths.
+constexpr int kBatchWideLog32 = 14;
+
 struct BatchClass {
-    int log_n = 0;
+    int log_n = 0;      // 32-bit digits
+    bool wide = false;  // five-prime kernels, 2^(log_n - 1) points
     bool square = false;
+    uint32_t bpp = 0;   // carry blocks per product
     std::vector<uint32_t> members;  // product indices
     size_t desc_off = 0;            // into the ProductDesc device array
     size_t flags_off = 0, flags_words = 0;
@@ -42,9 +53,10 @@ struct bgpu_batch_plan_s {
     int device = -1;
     size_t count = 0;
     std::vector<bgpu::BatchClass> classes;
-    // every NTT class (and the small products) run in the four mixed-length
-    // launches, one per pass
+    // the three-prime classes (classes[first_mixed ..)) and the small products
+    // run in the four mixed-length launches, one per pass
     bool mixed = false;
+    size_t first_mixed = 0;
     bgpu::MixedSizes mixed_sizes{};
     std::vector<std::array<uint32_t, 4>> mixed_begin;  // per class, per pass
     std::vector<bgpu::SchoolDesc> school;  // schoolbook products
@@ -67,8 +79,9 @@ int ceil_log2(uint64_t x) {
     return l;
 }
 
-size_t ntt_scratch_bytes(int log_n, bool square) {
+size_t ntt_scratch_bytes(int log_n, bool square, bool wide) {
     const size_t nn = (size_t)1 << log_n;
+    if (wide) return al256((square ? 1 : 2) * (size_t)kWidePrimes * (nn / 2) * 4);
     return al256((square ? 1 : 2) * (size_t)kNumPrimes * nn * 4) + al256(nn / 2 * 8) + al256(nn / 8 * 8);
 }
 
@@ -96,7 +109,8 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
         flag_words += c.flags_words;
     }
     const size_t mixed_off = al256(n_desc * sizeof(ProductDesc));
-    const size_t school_off = mixed_off + al256((p->mixed ? p->classes.size() : 0) * sizeof(MixedClass));
+    const size_t nmixed = p->mixed ? p->classes.size() - p->first_mixed : 0;
+    const size_t school_off = mixed_off + al256(nmixed * sizeof(MixedClass));
     const size_t kara_off = school_off + al256(p->school.size() * sizeof(SchoolDesc));
     const size_t tick_off = kara_off + al256(p->kara.size() * sizeof(SchoolDesc));
     unsigned long long* tickets = reinterpret_cast<unsigned long long*>(base + tick_off);
@@ -110,13 +124,13 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
     if (e != cudaSuccess) return BGPU_ERR_CUDA;
     uint32_t launches = 0;
     if (p->mixed) {
-        // every class and the small products: four launches on the recording stream
+        // the short classes and the small products: four launches on the recording stream
         MixedArgs m{};
         m.classes = reinterpret_cast<const MixedClass*>(base + mixed_off);
-        m.nclasses = (int)p->classes.size();
-        for (size_t i = 0; i < p->classes.size(); ++i)
+        m.nclasses = (int)nmixed;
+        for (size_t i = 0; i < nmixed; ++i)
             for (int pass = 0; pass < 4; ++pass) m.begin[pass][i] = p->mixed_begin[i][pass];
-        m.ticket = tickets;
+        m.ticket = tickets + p->first_mixed;
         m.ticket_base = 0;
         m.epoch = 1;
         m.err = hooks.err;
@@ -127,7 +141,8 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
         if (launch_ntt_mixed(m, p->mixed_sizes, st) != cudaSuccess) return BGPU_ERR_CUDA;
         launches += kNttLaunches;
     }
-    for (size_t ci = 0; !p->mixed && ci < p->classes.size(); ++ci) {
+    const size_t nbranched = p->mixed ? p->first_mixed : p->classes.size();
+    for (size_t ci = 0; ci < nbranched; ++ci) {
         const BatchClass& c = p->classes[ci];
         const int ps = prime_set_for(c.log_n);
         CarryLaunch cl;
@@ -135,12 +150,15 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
         cl.epoch = 1;
         cl.ticket = tickets + ci;
         cl.err = hooks.err;
-        e = launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], d_descs + c.desc_off,
-                             (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci]);
+        e = c.wide ? launch_wide_batch(hooks.consts[wide_set_for(c.log_n - 1)], d_descs + c.desc_off,
+                                       (uint32_t)c.members.size(), c.square, c.log_n - 1, kFmtLimb64, c.bpp, cl,
+                                       branches[ci])
+                   : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], d_descs + c.desc_off,
+                                      (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci]);
         if (e != cudaSuccess) return BGPU_ERR_CUDA;
         launches += kNttLaunches;
     }
-    size_t bi = p->mixed ? 0 : p->classes.size();
+    size_t bi = nbranched;
     if (!p->school.empty() && !p->mixed) {
         const SchoolDesc* d_school = reinterpret_cast<const SchoolDesc*>(base + school_off);
         if (launch_schoolbook_batch(d_school, (uint32_t)p->school.size(), branches[bi++]) != cudaSuccess)
@@ -208,19 +226,7 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
     // of each pass, start in the first wave and the short ones fill the tail.
     std::stable_sort(p->classes.begin(), p->classes.end(),
                      [](const BatchClass& x, const BatchClass& y) { return x.log_n > y.log_n; });
-    // Layout: [ProductDesc...][MixedClass...][SchoolDesc: schoolbook...]
-    //         [SchoolDesc: Karatsuba...][tickets][flags][scratch].
-    size_t n_desc = 0, flag_words = 0, scratch = 0;
-    for (auto& c : p->classes) {
-        c.desc_off = n_desc;
-        n_desc += c.members.size();
-        c.flags_off = flag_words;
-        c.flags_words = c.members.size() * carry_blocks((uint32_t)(((size_t)1 << c.log_n) / 8));
-        flag_words += c.flags_words;
-        c.scratch_off = scratch;
-        scratch += c.members.size() * ntt_scratch_bytes(c.log_n, c.square);
-    }
-    // The mixed-length launches take every class when each qualifies and
+    // The mixed-length launches take the short classes when each qualifies and
     // there are several lengths, unless the caller asks for per-class launch
     // sets (BGPU_BATCH_PER_CLASS); a single length runs its own per-length
     // kernels (tuned for it, without the mixed launches' register budget):
@@ -229,11 +235,33 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
 #ifndef BGPU_MIXED_BATCH
 #define BGPU_MIXED_BATCH 1
 #endif
-    p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && p->classes.size() >= 2 &&
-               p->classes.size() <= (size_t)kMaxMixedClasses;
-    for (auto& c : p->classes) p->mixed = p->mixed && mixed_class_ok(c.log_n, c.square);
+    while (p->first_mixed < p->classes.size() && p->classes[p->first_mixed].log_n >= kBatchWideLog32) ++p->first_mixed;
+    const size_t nshort = p->classes.size() - p->first_mixed;
+    p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && nshort >= 2 && nshort <= (size_t)kMaxMixedClasses;
+    for (size_t i = p->first_mixed; i < p->classes.size(); ++i)
+        p->mixed = p->mixed && mixed_class_ok(p->classes[i].log_n, p->classes[i].square);
+    // Layout: [ProductDesc...][MixedClass...][SchoolDesc: schoolbook...]
+    //         [SchoolDesc: Karatsuba...][tickets][flags][scratch].
+    size_t n_desc = 0, flag_words = 0, scratch = 0;
+    for (size_t i = 0; i < p->classes.size(); ++i) {
+        BatchClass& c = p->classes[i];
+        c.wide = (i < p->first_mixed || !p->mixed) && c.log_n > kWideMinLogN && c.log_n - 1 <= kWideMaxLogN;
+        if (c.wide) {
+            for (uint32_t m : c.members) c.bpp = std::max(c.bpp, wide_carry_blocks(prods[m].na + prods[m].nb, kFmtLimb64));
+        } else {
+            c.bpp = carry_blocks((uint32_t)(((size_t)1 << c.log_n) / 8));
+        }
+        c.desc_off = n_desc;
+        n_desc += c.members.size();
+        c.flags_off = flag_words;
+        c.flags_words = c.members.size() * c.bpp;
+        flag_words += c.flags_words;
+        c.scratch_off = scratch;
+        scratch += c.members.size() * ntt_scratch_bytes(c.log_n, c.square, c.wide);
+    }
+    const size_t nmixed = p->mixed ? nshort : 0;
     const size_t mixed_off = al256(n_desc * sizeof(ProductDesc));
-    const size_t school_off = mixed_off + al256((p->mixed ? p->classes.size() : 0) * sizeof(MixedClass));
+    const size_t school_off = mixed_off + al256(nmixed * sizeof(MixedClass));
     const size_t kara_off = school_off + al256(p->school.size() * sizeof(SchoolDesc));
     const size_t tick_off = kara_off + al256(p->kara.size() * sizeof(SchoolDesc));
     const size_t flags_base = tick_off + al256(std::max<size_t>(1, p->classes.size()) * 8);
@@ -248,7 +276,7 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
     std::vector<ProductDesc> descs(n_desc);
     for (auto& c : p->classes) {
         const size_t nn = (size_t)1 << c.log_n;
-        const size_t per = ntt_scratch_bytes(c.log_n, c.square);
+        const size_t per = ntt_scratch_bytes(c.log_n, c.square, c.wide);
         const size_t y_bytes = al256((c.square ? 1 : 2) * (size_t)kNumPrimes * nn * 4);
         for (size_t m = 0; m < c.members.size(); ++m) {
             const bgpu_product& q = prods[c.members[m]];
@@ -257,23 +285,22 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
             d.op[0] = OperandDesc{q.a, (uint32_t)q.na, (uint32_t)(2 * q.na), kFmtLimb64};
             d.op[1] = c.square ? d.op[0] : OperandDesc{q.b, (uint32_t)q.nb, (uint32_t)(2 * q.nb), kFmtLimb64};
             d.y = reinterpret_cast<uint32_t*>(sc);
-            d.chunks = reinterpret_cast<uint64_t*>(sc + y_bytes);
-            d.spill = reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
-            d.flags = reinterpret_cast<uint64_t*>(base + flags_base) + c.flags_off +
-                      m * carry_blocks((uint32_t)(nn / 8));
+            d.chunks = c.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes);
+            d.spill = c.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
+            d.flags = reinterpret_cast<uint64_t*>(base + flags_base) + c.flags_off + m * c.bpp;
             d.out = q.out;
             d.out_cap = q.na + q.nb;
         }
     }
     cudaError_t e = cudaMemcpy(base, descs.data(), n_desc * sizeof(ProductDesc), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && p->mixed) {
-        std::vector<MixedClassSpec> spec(p->classes.size());
-        for (size_t i = 0; i < p->classes.size(); ++i) {
-            const BatchClass& c = p->classes[i];
+        std::vector<MixedClassSpec> spec(nmixed);
+        for (size_t i = 0; i < nmixed; ++i) {
+            const BatchClass& c = p->classes[p->first_mixed + i];
             spec[i] = MixedClassSpec{reinterpret_cast<const ProductDesc*>(base) + c.desc_off,
                                      (uint32_t)c.members.size(), c.log_n, c.square};
         }
-        std::vector<MixedClass> mc(p->classes.size());
+        std::vector<MixedClass> mc(nmixed);
         if (mixed_fill(mc.data(), (int)mc.size(), spec.data(), kSlotEngine + 0, hooks.consts[0],
                        &p->mixed_sizes) != 0) {
             destroy_plan(p);
@@ -296,8 +323,8 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
         return BGPU_ERR_CUDA;
     }
     // Capture the whole batch into one graph (streams and events made first).
-    const size_t nbranch = p->mixed ? 0 : p->classes.size() + (p->school.empty() ? 0 : 1) +
-                                              (p->kara.empty() ? 0 : 1);
+    const size_t nbranch = p->mixed ? p->first_mixed
+                                    : p->classes.size() + (p->school.empty() ? 0 : 1) + (p->kara.empty() ? 0 : 1);
     std::vector<cudaStream_t> branches(nbranch, nullptr);
     std::vector<cudaEvent_t> joins(nbranch, nullptr);
     cudaStream_t cap = nullptr;
@@ -403,7 +430,9 @@ struct TreeLevel {
     uint32_t m, m2;
     size_t w;
     int kind;  // 0: thread per product (w <= 4), 1: schoolbook, 2: Karatsuba, 3: NTT
-    int log_n = 0;
+    int log_n = 0;        // kind 3: 32-bit digits
+    bool wide = false;    // kind 3: five-prime kernels, 2^(log_n - 1) points
+    uint32_t bpp = 0;     // kind 3: carry blocks per product
     size_t desc_off = 0;  // bytes into the descriptor region
 };
 
@@ -435,9 +464,11 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
             L.kind = 3;
             while (((uint64_t)1 << L.log_n) < 4 * (uint64_t)w - 1) ++L.log_n;
             if (!shape_supported_batch(L.log_n, false)) return BGPU_ERR_CAPACITY;
-            const size_t nn = (size_t)1 << L.log_n;
-            ntt_bytes = std::max(ntt_bytes, (size_t)L.m2 * ntt_scratch_bytes(L.log_n, false));
-            flag_words = std::max(flag_words, (size_t)L.m2 * carry_blocks((uint32_t)(nn / 8)));
+            L.wide = L.log_n > kWideMinLogN && L.log_n - 1 <= kWideMaxLogN;
+            L.bpp = L.wide ? wide_carry_blocks(2 * w, kFmtLimb64)
+                           : carry_blocks((uint32_t)(((size_t)1 << L.log_n) / 8));
+            ntt_bytes = std::max(ntt_bytes, (size_t)L.m2 * ntt_scratch_bytes(L.log_n, false, L.wide));
+            flag_words = std::max(flag_words, (size_t)L.m2 * L.bpp);
         }
         if (L.kind == 1 || L.kind == 2) {
             L.desc_off = desc_bytes;
@@ -488,8 +519,8 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
             } else if (L.kind == 3) {
                 ProductDesc* pd = reinterpret_cast<ProductDesc*>(hd.data() + L.desc_off);
                 const size_t nn = (size_t)1 << L.log_n;
-                const size_t per = ntt_scratch_bytes(L.log_n, false);
-                const uint32_t bpp = carry_blocks((uint32_t)(nn / 8));
+                const size_t per = ntt_scratch_bytes(L.log_n, false, L.wide);
+                const uint32_t bpp = L.bpp;
                 const size_t y_bytes = al256(2 * (size_t)kNumPrimes * nn * 4);
                 for (uint32_t i = 0; i < L.m2; ++i) {
                     char* sc = base + off_ntt + (size_t)i * per;
@@ -497,8 +528,8 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
                     d.op[0] = OperandDesc{in + (size_t)2 * i * w, (uint32_t)w, (uint32_t)(2 * w), kFmtLimb64};
                     d.op[1] = OperandDesc{in + (size_t)(2 * i + 1) * w, (uint32_t)w, (uint32_t)(2 * w), kFmtLimb64};
                     d.y = reinterpret_cast<uint32_t*>(sc);
-                    d.chunks = reinterpret_cast<uint64_t*>(sc + y_bytes);
-                    d.spill = reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
+                    d.chunks = L.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes);
+                    d.spill = L.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
                     d.flags = flags + (size_t)i * bpp;
                     d.out = out + (size_t)2 * i * w;
                     d.out_cap = 2 * w;
@@ -530,10 +561,8 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
             nl += 1;
         } else {
             // fresh carry-scan state for this level: ticket 0, flags 0, epoch 1
-            const size_t nn = (size_t)1 << L.log_n;
             e = cudaMemsetAsync(ticket, 0, 8, st);
-            if (e == cudaSuccess)
-                e = cudaMemsetAsync(flags, 0, (size_t)L.m2 * carry_blocks((uint32_t)(nn / 8)) * 8, st);
+            if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, (size_t)L.m2 * L.bpp * 8, st);
             if (e == cudaSuccess) {
                 CarryLaunch cl;
                 cl.ticket_base = 0;
@@ -541,9 +570,11 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
                 cl.ticket = ticket;
                 cl.err = hooks.err;
                 const int ps = prime_set_for(L.log_n);
-                e = launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps],
-                                     reinterpret_cast<const ProductDesc*>(base + off_desc + L.desc_off),
-                                     (int)L.m2, false, L.log_n, kFmtLimb64, cl, st);
+                const ProductDesc* pd = reinterpret_cast<const ProductDesc*>(base + off_desc + L.desc_off);
+                e = L.wide ? launch_wide_batch(hooks.consts[wide_set_for(L.log_n - 1)], pd, L.m2, false, L.log_n - 1,
+                                               kFmtLimb64, L.bpp, cl, st)
+                           : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], pd, (int)L.m2, false, L.log_n,
+                                              kFmtLimb64, cl, st);
             }
             nl += kNttLaunches;
         }

@@ -101,3 +101,40 @@ def test_large_residue(bb, log_n):
         a, b = rand_limbs(rng, na), np.full(total - na, ONES)
         c = bb.ntt_mul(a, b)
         assert mod61(c) == mod61(a) * mod61(b) % M61, (na, total - na)
+
+
+def _run_batch(bb, port, sizes, squares=(), flags=0):
+    import torch
+
+    rng = np.random.default_rng([SEED, len(sizes)])
+    host = [(rand_limbs(rng, na), rand_limbs(rng, nb)) for na, nb in sizes]
+    dev = [tuple(torch.from_numpy(x.view(np.int64)).cuda() for x in p) for p in host]
+    outs = [torch.full((2 * na if i in squares else na + nb,), -1, dtype=torch.int64, device="cuda")
+            for i, (na, nb) in enumerate(sizes)]
+    prods = []
+    for i, (a, b) in enumerate(dev):
+        b = a if i in squares else b
+        prods.append((a.data_ptr(), a.numel(), b.data_ptr(), b.numel(), outs[i].data_ptr()))
+    plan = bb.BatchPlan(prods, flags=flags)
+    for _ in range(2):
+        plan.run(0)
+        bb.device_status(0)
+    plan.close()
+    for i, (a, b) in enumerate(host):
+        want = port.mul(a, a if i in squares else b)
+        got = outs[i].cpu().numpy().view(np.uint64)
+        assert np.array_equal(got[: want.size], want) and not got[want.size:].any(), (i, sizes[i])
+
+
+# one length on its own; long classes beside the mixed-length launches, a class
+# holding products much shorter than its longest (their carry blocks end
+# early), operands over half the points, squares; every class on branches
+@pytest.mark.parametrize("sizes,squares", [
+    ([(700, 600), (1100, 90), (1023, 2)], ()),
+    ([(4097, 4097), (8000, 9), (5000, 7000), (300, 400), (1000, 900), (60, 70)], (2,)),
+    ([(16384, 16385), (16385, 16385), (40000, 30), (33000, 700)], (1,)),
+])
+@pytest.mark.parametrize("per_class", [False, True])
+def test_batch_classes(bb, port, sizes, squares, per_class):
+    _run_batch(bb, port, sizes * 3, [s + k * len(sizes) for s in squares for k in range(3)],
+               bb.BGPU_BATCH_PER_CLASS if per_class else 0)
