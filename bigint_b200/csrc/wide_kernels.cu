@@ -23,8 +23,12 @@ constexpr int kWideCols = 8;
 // 2^L2 / 16), so that short columns leave no thread idle: forward and inverse
 // pass per 2^19 points of a batch, columns of 2^6 rows 28.0 + 10.8 -> 14.2 + 5.5 us,
 // of 2^8 rows 16.8 + 9.1 -> 13.3 + 5.2 us against 256 threads throughout.
-__host__ __device__ constexpr int wide_col_threads(int l2) {
-    return l2 <= 5 ? 32 : l2 <= 7 ? 64 : l2 == 8 ? 128 : 256;
+// Columns of 2^11 rows (64 KB tiles, two or three a SM) run two CTAs of 512
+// threads forward and three of 256 inverse: 2^24 points 548 + 249 us against
+// 647 + 249 (256 x 3) and 548 + 265 (512 x 2), and 587 + 452 with the
+// compiler's registers at 256 threads.
+__host__ __device__ constexpr int wide_col_threads(int l2, bool fwd) {
+    return l2 <= 5 ? 32 : l2 <= 7 ? 64 : l2 == 8 ? 128 : l2 == 11 && fwd ? 512 : 256;
 }
 // Row pass: threads of a row and rows of a CTA.  Short rows have fewer groups
 // than a warp has lanes (16 at 2^8 points), so a CTA takes several side by
@@ -34,9 +38,16 @@ __host__ __device__ constexpr int wide_row_threads(int l1) {
     return l1 >= 12 ? 256 : l1 >= 9 ? (1 << (l1 - 4)) : l1 == 8 ? 16 : 8;
 }
 __host__ __device__ constexpr int wide_rows_per_cta(int l1) { return l1 >= 10 ? 1 : 128 / wide_row_threads(l1); }
+// Rows of 2^13 points and more of a product of two operands use one row buffer:
+// A's transform is parked in its own plane and read back by the pointwise
+// product, so that four and three CTAs share an SM instead of three and one.
+// Row pass, two buffers -> one: 2^23 points in rows of 2^13 358 -> 334 us, 2^25
+// points in rows of 2^14 1807 (512 threads) -> 1407 us; rows of 2^12 points are
+// faster with two (2^21 points 81 against 88 us).
+__host__ __device__ constexpr bool wide_one_buffer(int l1) { return l1 >= 13; }
 // Shared words of a row: its buffers and 16 Shoup pairs, a warp's rows in different banks.
 __host__ __device__ constexpr uint32_t wide_row_words(int l1, bool square) {
-    return ((square ? 1u : 2u) << l1) + 32u + (l1 >= 10 ? 0u : (uint32_t)wide_row_threads(l1) % 32u);
+    return ((square || wide_one_buffer(l1) ? 1u : 2u) << l1) + 32u + (l1 >= 10 ? 0u : (uint32_t)wide_row_threads(l1) % 32u);
 }
 
 __constant__ NttConsts c_wide[2];  // lazy, strict
@@ -147,13 +158,13 @@ __device__ __forceinline__ void wide_round0(const WideArgs& a, const OperandDesc
 
 // CTAs per SM (register caps): 1024 threads' worth of 64 registers, except
 // columns of 2^9 rows at 1280 (2^19 points of a batch: 15.0 + 5.7 us; at 1024
-// 15.5 + 6.2, at 2048 15.1 + 5.9) and of 2^11 rows, whose tiles leave room for two.
-#ifndef BGPU_WIDE_COL_BLOCKS
-#define BGPU_WIDE_COL_BLOCKS(l2) ((l2) == 9 ? 5 : ((l2) == 11 ? 1 : 1024 / wide_col_threads(l2)))
-#endif
+// 15.5 + 6.2, at 2048 15.1 + 5.9) and the inverse pass's tiles of 2^11 rows.
+__host__ __device__ constexpr int wide_col_blocks(int l2, bool fwd) {
+    return l2 == 9 ? 5 : l2 == 11 && !fwd ? 3 : 1024 / wide_col_threads(l2, fwd);
+}
 
 template <bool LAZY, int L2, int T>
-__global__ void __launch_bounds__(T, BGPU_WIDE_COL_BLOCKS(L2)) k_wide_fwd(const WideArgs a) {
+__global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const WideArgs a) {
     using P2 = Plan<L2>;
     constexpr int NR = P2::nr, RL = P2::r(NR - 1), SROW = (1 << RL) + 1;
     static_assert(NR > 1, "column passes of several rounds");
@@ -213,18 +224,20 @@ __global__ void __launch_bounds__(T, BGPU_WIDE_COL_BLOCKS(L2)) k_wide_fwd(const 
 
 // ---- 2: rows -----------------------------------------------------------------------
 
-// Rows of 2^8 points spill at 64 registers and run five CTAs of 128 threads
-// (14.1 -> 12.7 us per 2^19 points), 2^9 points six.
-#ifndef BGPU_WIDE_ROW_BLOCKS
-#define BGPU_WIDE_ROW_BLOCKS(l1, t) ((l1) == 8 ? 5 : (l1) == 9 ? 6 : ((l1) <= 12 ? 1024 / (t) : ((l1) == 13 ? 768 / (t) : 1)))
-#endif
+// CTAs per SM: 1024 threads' worth of 64 registers; rows of 2^8 points, which
+// spill there, five CTAs of 128 threads (14.1 -> 12.7 us per 2^19 points), of 2^9
+// points six, of 2^14 points three of 80 registers (1407 us at 2^25 points; two
+// of 512 threads 1488).
+__host__ __device__ constexpr int wide_row_blocks(int l1) {
+    return l1 == 8 ? 5 : l1 == 9 ? 6 : l1 == 13 ? 4 : l1 == 14 ? 3 : 1024 / (wide_row_threads(l1) * wide_rows_per_cta(l1));
+}
 
 template <bool LAZY, int L1, bool SQR>
-__global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1),
-                                  BGPU_WIDE_ROW_BLOCKS(L1, wide_row_threads(L1) * wide_rows_per_cta(L1)))
+__global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1), wide_row_blocks(L1))
     k_wide_rows(const WideArgs a) {
     constexpr int T = wide_row_threads(L1);
     constexpr bool MULTI = wide_rows_per_cta(L1) > 1;
+    constexpr bool ONE = !SQR && wide_one_buffer(L1);
     using P1 = Plan<L1>;
     constexpr int NR = P1::nr;
     constexpr int R0 = P1::r(0), LO0 = P1::lo(0);
@@ -233,8 +246,8 @@ __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1),
     const NttConsts& c = c_wide[LAZY ? 0 : 1];
     const uint32_t sub = MULTI ? threadIdx.x / T : 0u;
     uint32_t* sa = sm + sub * wide_row_words(L1, SQR);
-    uint32_t* sb = sa + (1u << L1);
-    uint2* sT = reinterpret_cast<uint2*>(sa + ((SQR ? 1u : 2u) << L1));
+    uint32_t* sb = ONE ? sa : sa + (1u << L1);
+    uint2* sT = reinterpret_cast<uint2*>(sa + ((SQR || ONE ? 1u : 2u) << L1));
     const int q = blockIdx.y, tid = sub_tid<T, MULTI>();
     const uint32_t slot = blockIdx.x * wide_rows_per_cta(L1) + sub;
     const ProductDesc pd = wide_product(a, blockIdx.z);
@@ -255,14 +268,30 @@ __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1),
     pdl_wait();
 
     mid_dif_row<LAZY, L1, T, MULTI>(row_a, sa, twf, p);
-    if constexpr (!SQR) {
+    if constexpr (ONE) {  // A's last DIF round, each group's outputs parked in its plane
+        using Gr = Group<L1, 1, NR - 1>;
+        static_assert(Gr::LO == 0 && Gr::R >= 2, "a group is a run of elements");
+#pragma unroll 1
+        for (int g = tid; g < Gr::G; g += T) {
+            const Gr gr(g);
+            uint32_t x[1 << Gr::R];
+#pragma unroll
+            for (int j = 0; j < (1 << Gr::R); ++j) x[j] = sa[gr.at(j)];
+            dif_regs<LAZY, Gr::R, Gr::HI, Gr::LO>(x, gr.base_low, twf, p);
+            uint4* o = reinterpret_cast<uint4*>(row_a + gr.base);
+#pragma unroll
+            for (int j = 0; j < (1 << Gr::R); j += 4) o[j / 4] = make_uint4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+        }
+        __syncthreads();  // the buffer takes B
+        mid_dif_row<LAZY, L1, T, MULTI>(row_b, sb, twf, p);
+    } else if constexpr (!SQR) {
         smem_round<LAZY, L1, 1, T, NR - 1, false>(sa, twf, p, tid);  // A's last DIF round
         mid_dif_row<LAZY, L1, T, MULTI>(row_b, sb, twf, p);
     }
     {  // the last DIF round of B (or A), the pointwise product, the first DIT round
         using Gr = Group<L1, 1, NR - 1>;
         constexpr int R = Gr::R;
-        const uint32_t* src = SQR ? sa : sb;
+        const uint32_t* src = SQR || ONE ? sa : sb;
 #pragma unroll 1
         for (int g = tid; g < Gr::G; g += T) {
             const Gr gr(g);
@@ -270,10 +299,18 @@ __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1),
 #pragma unroll
             for (int j = 0; j < (1 << R); ++j) x[j] = src[gr.at(j)];
             dif_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twf, p);
+            uint4 av{};
 #pragma unroll
             for (int j = 0; j < (1 << R); ++j) {
+                uint32_t o = x[j];
+                if constexpr (ONE) {  // parked by this thread
+                    if (j % 4 == 0) av = reinterpret_cast<const uint4*>(row_a + gr.base)[j / 4];
+                    o = j % 4 == 0 ? av.x : j % 4 == 1 ? av.y : j % 4 == 2 ? av.z : av.w;
+                } else if constexpr (!SQR) {
+                    o = sa[gr.at(j)];
+                }
                 // below p for factors below p; below 2p for factors below 2p, 4p < 2^32
-                const uint32_t z = mont(x[j], SQR ? x[j] : sa[gr.at(j)], p, np);
+                const uint32_t z = mont(x[j], o, p, np);
                 x[j] = LAZY ? z : csub(z, p);
             }
             dit_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
@@ -302,7 +339,7 @@ __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1),
 // ---- 3: inverse columns ---------------------------------------------------------------
 
 template <bool LAZY, int L2, int T>
-__global__ void __launch_bounds__(T, BGPU_WIDE_COL_BLOCKS(L2)) k_wide_inv(const WideArgs a) {
+__global__ void __launch_bounds__(T, wide_col_blocks(L2, false)) k_wide_inv(const WideArgs a) {
     using P2 = Plan<L2>;
     constexpr int NR = P2::nr;
     extern __shared__ __align__(16) uint32_t sm[];  // [2^L2][8]
@@ -623,14 +660,14 @@ cudaError_t launch_cols(bool fwd, const WideArgs& a, uint32_t count, cudaStream_
     const size_t tile = (size_t)kWideCols * 4 << L2;
     const uint32_t tiles = (1u << a.log_n1) / kWideCols;
     if (fwd) {
-        auto k = k_wide_fwd<LAZY, L2, wide_col_threads(L2)>;
+        auto k = k_wide_fwd<LAZY, L2, wide_col_threads(L2, true)>;
         const size_t sm = tile + kWideCols * ((1 << RL) + 1) * sizeof(uint2);
         allow_smem(k, sm);
-        return launch_k(k, dim3(tiles, kWidePrimes, count * a.nops), dim3(wide_col_threads(L2)), sm, st, a);
+        return launch_k(k, dim3(tiles, kWidePrimes, count * a.nops), dim3(wide_col_threads(L2, true)), sm, st, a);
     }
-    auto k = k_wide_inv<LAZY, L2, wide_col_threads(L2)>;
+    auto k = k_wide_inv<LAZY, L2, wide_col_threads(L2, false)>;
     allow_smem(k, tile);
-    return launch_k(k, dim3(tiles, kWidePrimes, count), dim3(wide_col_threads(L2)), tile, st, a);
+    return launch_k(k, dim3(tiles, kWidePrimes, count), dim3(wide_col_threads(L2, false)), tile, st, a);
 }
 
 template <bool LAZY>
@@ -751,13 +788,13 @@ cudaError_t upload_wide_consts(int set, const NttConsts& c) {
 // product back to back, the choice against the nearest other length: 2^12
 // points 9.8 (2^6) / 11.3 (2^7), 2^17 21.0 (2^6) / 22.2 (2^7), 2^18 28.9 (2^8) /
 // 29.8 (2^7), 2^19 47.7 (2^8) / 49.5 (2^9), 2^20 88.7 (2^8) / 90.4 (2^9), 2^21 175.7
-// (2^10) / 180.5 (2^9), 2^23 777 (2^10) / 900 (2^11), 2^24 1852 (2^11) / 1919 (2^10).
+// (2^10) / 180.5 (2^9), 2^23 753 (2^10) / 780 (2^11), 2^24 1543 (2^10) / 1572 (2^11).
 // Batches, us per 2^19 points: 2^13 33.7 (2^7) / 35.7 (2^6), 2^15 34.5 (2^8) /
 // 35.4 (2^7), 2^17 37.8 (2^9) / 38.8 (2^8), 2^19 38.7 (2^8) / 40.4 (2^9).
 static constexpr int8_t kWideColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  5,  6,  6,
-                                                         7, 8, 8, 8, 6, 8, 8, 8, 10, 10, 10, 11, 11};
+                                                         7, 8, 8, 8, 6, 8, 8, 8, 10, 10, 10, 10, 11};
 static constexpr int8_t kWideBatchColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  5,  6,  6,
-                                                              7, 8, 8, 8, 9, 8, 8, 9, 10, 10, 10, 11, 11};
+                                                              7, 8, 8, 8, 9, 8, 8, 9, 10, 10, 10, 10, 11};
 
 TransformShape wide_shape(int log_n, bool batch) {
     TransformShape s{log_n, 0, 0};
