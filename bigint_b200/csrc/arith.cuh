@@ -11,13 +11,19 @@
 //   469762049 (g 3), 1811939329 = 27*2^26+1 (g 13), 2013265921 = 15*2^27+1 (g 31)
 //   product ~2^90.47 > 2^89 >= (N/2)(2^32-1)^2 for N <= 2^26; residues are
 //   kept fully reduced in [0, p) (sums of two still fit in 32 bits).
-// Sets 2 and 3 have five primes and carry 64-bit digits (wide_kernels.cu):
+// Sets 2 to 7 have five, six and seven primes and carry 64-, 80- and 96-bit
+// digits (wide_kernels.cu): with D-bit digits every coefficient is at most
+// (N/2)(2^D-1)^2, below 0.9 of the product.
 // Set 2 ("lazy", up to 2^22 points), all primes < 2^30 with 2^22 | p-1:
 //   998244353 (g 3), 985661441 (g 3), 943718401 (g 7), 935329793 (g 3), 918552577 (g 5)
 //   product ~2^149.16 > 2^149 >= (N/2)(2^64-1)^2 for N <= 2^22.
 // Set 3 ("strict", up to 2^25 points), all primes < 2^31 with 2^25 | p-1:
 //   1107296257 (g 10), 1711276033 (g 29), 1811939329 (g 13), 2013265921 (g 31), 2113929217 (g 5)
 //   product ~2^153.36 > 2^152 >= (N/2)(2^64-1)^2 for N <= 2^25.
+// Set 4 (six, lazy, up to 2^20 points): product ~2^179.63 against 2^179.
+// Set 5 (six, strict, up to 2^24 points): product ~2^184.49 against 2^183.
+// Set 6 (seven, lazy, up to 2^18 points): product ~2^209.87 against 2^209.
+// Set 7 (seven, strict, up to 2^23 points): product ~2^215.73 against 2^214.
 // 469762049 and 2013265921 are the reference's own P[0], P[1]
 // (include/bigint/ntt_base.h:15); its third prime 2281701377 > 2^31 would not
 // leave room for carry-free sums.
@@ -32,8 +38,9 @@ namespace bgpu {
 
 constexpr int kNumPrimes = 3;   // of sets 0 and 1
 constexpr int kWidePrimes = 5;  // of sets 2 and 3
-constexpr int kMaxPrimes = 5;
-constexpr int kNumSets = 4;
+constexpr int kMaxPrimes = 7;
+constexpr int kNumSets = 8;
+constexpr int kFirstWideSet = 2;
 constexpr int kMaxLogN = 26;    // largest transform overall (set 1)
 constexpr int kLazyMaxLogN = 23;  // largest transform of set 0
 constexpr int kMaxLogRow = 15;  // stage tables cover pair distances h < 2^15
@@ -54,10 +61,21 @@ constexpr PrimeSetInfo kPrimeSets[kNumSets] = {
     {3, {469762049u, 1811939329u, 2013265921u}, {3u, 13u, 31u}, kMaxLogN, 13},
     {5, {998244353u, 985661441u, 943718401u, 935329793u, 918552577u}, {3u, 3u, 7u, 3u, 5u}, kWideLazyMaxLogN, 11},
     {5, {1107296257u, 1711276033u, 1811939329u, 2013265921u, 2113929217u}, {10u, 29u, 13u, 31u, 5u}, kWideMaxLogN, 13},
+    {6, {1053818881u, 1051721729u, 1045430273u, 1012924417u, 1007681537u, 1004535809u}, {7u, 6u, 3u, 5u, 3u, 3u}, 20, 10},
+    {6, {2130706433u, 2113929217u, 2013265921u, 1811939329u, 1711276033u, 1224736769u}, {3u, 5u, 31u, 13u, 29u, 3u}, 24, 12},
+    {7, {1073479681u, 1068236801u, 1062469633u, 1056440321u, 1056178177u, 1053818881u, 1052508161u},
+     {11u, 3u, 5u, 3u, 5u, 7u, 3u}, 18, 9},
+    {7, {2130706433u, 2113929217u, 2088763393u, 2013265921u, 1811939329u, 1711276033u, 1484783617u},
+     {3u, 5u, 5u, 31u, 13u, 29u, 5u}, 23, 12},
 };
 
 inline int prime_set_for(int log_n) { return log_n <= kLazyMaxLogN ? 0 : 1; }
-inline int wide_set_for(int log_n) { return log_n <= kWideLazyMaxLogN ? 2 : 3; }
+// Set of a transform of 2^log_n points over np primes: the lazy one up to its
+// largest length.
+inline int wide_set_for(int np, int log_n) {
+    const int lazy = kFirstWideSet + 2 * (np - kWidePrimes);
+    return log_n <= kPrimeSets[lazy].log_max ? lazy : lazy + 1;
+}
 
 struct PrimeInfo {
     uint32_t p;

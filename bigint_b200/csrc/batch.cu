@@ -150,9 +150,8 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
         cl.epoch = 1;
         cl.ticket = tickets + ci;
         cl.err = hooks.err;
-        e = c.wide ? launch_wide_batch(hooks.consts[wide_set_for(c.log_n - 1)], d_descs + c.desc_off,
-                                       (uint32_t)c.members.size(), c.square, c.log_n - 1, kFmtLimb64, c.bpp, cl,
-                                       branches[ci])
+        e = c.wide ? launch_wide_batch({kWidePrimes, c.log_n - 1}, d_descs + c.desc_off, (uint32_t)c.members.size(),
+                                       c.square, kFmtLimb64, c.bpp, cl, branches[ci])
                    : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], d_descs + c.desc_off,
                                       (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci]);
         if (e != cudaSuccess) return BGPU_ERR_CUDA;
@@ -247,7 +246,7 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
         BatchClass& c = p->classes[i];
         c.wide = (i < p->first_mixed || !p->mixed) && c.log_n > kWideMinLogN && c.log_n - 1 <= kWideMaxLogN;
         if (c.wide) {
-            for (uint32_t m : c.members) c.bpp = std::max(c.bpp, wide_carry_blocks(prods[m].na + prods[m].nb, kFmtLimb64));
+            for (uint32_t m : c.members) c.bpp = std::max(c.bpp, wide_carry_blocks(kWidePrimes, prods[m].na + prods[m].nb, kFmtLimb64));
         } else {
             c.bpp = carry_blocks((uint32_t)(((size_t)1 << c.log_n) / 8));
         }
@@ -465,7 +464,7 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
             while (((uint64_t)1 << L.log_n) < 4 * (uint64_t)w - 1) ++L.log_n;
             if (!shape_supported_batch(L.log_n, false)) return BGPU_ERR_CAPACITY;
             L.wide = L.log_n > kWideMinLogN && L.log_n - 1 <= kWideMaxLogN;
-            L.bpp = L.wide ? wide_carry_blocks(2 * w, kFmtLimb64)
+            L.bpp = L.wide ? wide_carry_blocks(kWidePrimes, 2 * w, kFmtLimb64)
                            : carry_blocks((uint32_t)(((size_t)1 << L.log_n) / 8));
             ntt_bytes = std::max(ntt_bytes, (size_t)L.m2 * ntt_scratch_bytes(L.log_n, false, L.wide));
             flag_words = std::max(flag_words, (size_t)L.m2 * L.bpp);
@@ -571,8 +570,7 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
                 cl.err = hooks.err;
                 const int ps = prime_set_for(L.log_n);
                 const ProductDesc* pd = reinterpret_cast<const ProductDesc*>(base + off_desc + L.desc_off);
-                e = L.wide ? launch_wide_batch(hooks.consts[wide_set_for(L.log_n - 1)], pd, L.m2, false, L.log_n - 1,
-                                               kFmtLimb64, L.bpp, cl, st)
+                e = L.wide ? launch_wide_batch({kWidePrimes, L.log_n - 1}, pd, L.m2, false, kFmtLimb64, L.bpp, cl, st)
                            : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], pd, (int)L.m2, false, L.log_n,
                                               kFmtLimb64, cl, st);
             }

@@ -234,19 +234,12 @@ int prepare_scratch(int log_n, bool square, ProductScratch* s) {
     return BGPU_OK;
 }
 
-// log2 of the five-prime transform of a product, in 64-bit digits, or 0 for
-// the three-prime one.
-int wide_log(const OperandDesc& a, const OperandDesc& b) {
-    const int ln = ceil_log2((uint64_t)wide_digits(a) + wide_digits(b) - 1);
-    return ln <= kWideMaxLogN && wide_shape(ln, false).log_n2 ? ln : 0;
-}
-
-// Product of two device operands on the five-prime transform.
-int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, int ln, void* out, int out_fmt,
+// Product of two device operands on the wide-digit transform.
+int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, WideForm f, void* out, int out_fmt,
                   size_t out_cap, cudaStream_t st, bgpu_stats* stats) {
-    const size_t nn = (size_t)1 << ln;
-    const uint32_t bpp = wide_carry_blocks(out_cap, out_fmt);
-    const size_t y_bytes = align256((square ? 1 : 2) * (size_t)kWidePrimes * nn * 4);
+    const size_t nn = (size_t)1 << f.log_n;
+    const uint32_t bpp = wide_carry_blocks(f.np, out_cap, out_fmt);
+    const size_t y_bytes = align256((square ? 1 : 2) * (size_t)f.np * nn * 4);
     int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + align256((size_t)bpp * 8));
     if (rc != BGPU_OK) return rc;
     ProductDesc one{};
@@ -269,8 +262,7 @@ int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, int l
         ++g.kev_count;
         g.timed_wide = true;
     }
-    const cudaError_t e = launch_wide_product(g.consts[wide_set_for(ln)], nullptr, one, 1, square, ln, out_fmt, bpp,
-                                              cl, st, ev);
+    const cudaError_t e = launch_wide_product(f, nullptr, one, 1, square, out_fmt, bpp, cl, st, ev);
     g.last_launches = kNttLaunches;
     if (stats) {
         stats->method = BGPU_METHOD_NTT;
@@ -289,7 +281,7 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     const int log_n = ceil_log2(total32 - 1);
     if (log_n > kMaxLogN || !shape_supported(log_n < 5 ? 5 : log_n, square))
         return BGPU_ERR_CAPACITY;
-    if (const int wl = wide_log(a, b)) return multiply_wide(a, b, square, wl, out, out_fmt, out_cap, st, stats);
+    if (const WideForm f = wide_form(a.nd32, b.nd32); f.np) return multiply_wide(a, b, square, f, out, out_fmt, out_cap, st, stats);
     const int ln = log_n < 5 ? 5 : log_n;
     ProductScratch s{};
     int rc = prepare_scratch(ln, square, &s);

@@ -1,7 +1,8 @@
-// The five-prime product pipeline: 64-bit digits over five primes
-// (wide_kernels.cu).  Against 32-bit digits over three primes a product takes
-// half the points with 5/3 of the residues each, 5/6 of the residues in all,
-// and one transform level less.
+// The wide-digit product pipeline (wide_kernels.cu): 64-bit digits over five
+// primes, 80-bit digits over six or 96-bit digits over seven.  Against 32-bit
+// digits over three primes a product in 64-bit digits takes half the points
+// with 5/3 of the residues each, 5/6 of the residues in all, and one transform
+// level less; the longer digits fill the steps between powers of two.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -12,27 +13,39 @@
 
 namespace bgpu {
 
-// 64-bit digits of an operand.
-__host__ __device__ inline uint32_t wide_digits(const OperandDesc& o) { return o.nd32 / 2 + o.nd32 % 2; }
+// Bits of a digit over np primes, and the digits of nd32 32-bit digits.
+__host__ __device__ constexpr uint32_t wide_bits(int np) { return 16u * (uint32_t)(np - 1); }
+__host__ __device__ constexpr uint32_t wide_digits(int np, uint32_t nd32) {
+    return (uint32_t)(((uint64_t)nd32 * 32 + wide_bits(np) - 1) / wide_bits(np));
+}
+
+constexpr int kWideMaxPrimes = 7;
+
+// Transform of a product: 2^log_n points over np primes (np == 0: none).
+struct WideForm {
+    int np = 0, log_n = 0;
+};
+// The form of least work for operands of nd32a and nd32b 32-bit digits.
+WideForm wide_form(uint32_t nd32a, uint32_t nd32b);
 
 // Shortest transform: below it (1024 limbs of product) the three-prime
 // kernels, whose few blocks are as fast.
 constexpr int kWideMinLogN = 10;
 
 struct WideArgs {
-    const ProductDesc* descs;  // y: (square ? 1 : 2) * 5 planes of N residues (the result replaces A's)
+    const ProductDesc* descs;  // y: (square ? 1 : 2) * np planes of N residues (the result replaces A's)
     ProductDesc one;
-    int nops, log_n, log_n1;
-    uint32_t scale[kWidePrimes];  // row pass: 2^96 / N / (M / p) mod p, Montgomery form
+    int nops, log_n, log_n1, np;
+    int set;                         // of the wide sets
+    uint32_t scale[kWideMaxPrimes];  // row pass, Montgomery form
 };
 
-// CRT of five residues y_i = x (M/p_i)^-1 mod p_i: x = sum y_i M/p_i - q M.
-constexpr int kWideMaxQ = 5;  // q is at most 4
+// CRT of residues y_i = x (M/p_i)^-1 mod p_i: x = sum y_i M/p_i - q M, q < np.
 struct WideCrt {
-    uint32_t m[kWidePrimes][4];  // M / p_i
-    uint32_t nqm[kWideMaxQ][5];  // -q M mod 2^160
-    float inv[kWidePrimes];      // 256 / p_i
-    float bias;                  // 0.05 - 2^23 sum inv
+    uint32_t m[kWideMaxPrimes][kWideMaxPrimes - 1];  // M / p_i, np - 1 words
+    uint32_t nqm[kWideMaxPrimes][kWideMaxPrimes];    // -q M mod 2^(32 np)
+    float inv[kWideMaxPrimes];                       // 256 / p_i
+    float bias;                                      // 0.05 - 2^23 sum inv
 };
 
 struct WideCarryArgs {
@@ -46,30 +59,31 @@ struct WideCarryArgs {
     uint32_t* err;
 };
 
-constexpr uint32_t kWideCarryChunks = 256;  // 256-bit chunks per carry block
+constexpr uint32_t kWideCarryChunks = 256;  // chunks of four digits (np - 1 limbs) per carry block
 // Carry blocks of a product with out_cap output elements.
-__host__ __device__ inline uint32_t wide_carry_blocks(size_t out_cap, int out_fmt) {
+__host__ __device__ inline uint32_t wide_carry_blocks(int np, size_t out_cap, int out_fmt) {
     const uint64_t limbs = out_fmt == kFmtLimb64 ? out_cap : ((uint64_t)out_cap * 28 + 63) / 64;
-    return (uint32_t)((limbs + 4 * kWideCarryChunks - 1) / (4 * kWideCarryChunks));
+    const uint32_t per = (uint32_t)(np - 1) * kWideCarryChunks;
+    return (uint32_t)((limbs + per - 1) / per);
 }
 
-// Split of 2^log_n 64-bit digits: the tuned one of 2^(log_n + 1) 32-bit digits
+// Split of 2^log_n points: the tuned one of 2^(log_n + 1) 32-bit digits
 // (bgpu_set_split, bgpu_set_batch_split) where its kernels are built, else the
-// built-in one.  log_n2 == 0: no five-prime transform of this length.
+// built-in one.  log_n2 == 0: no transform of this length.
 TransformShape wide_shape(int log_n, bool batch);
 cudaError_t upload_wide_consts(int set, const NttConsts& c);
 extern const char* const kWideKernelNames[kNttLaunches];
 
-// The four launches of `count` products of 2^log_n points (64-bit digits of
-// both operands together at most 2^log_n + 1); each product's carry scan has
-// `bpp` blocks (tickets).
-cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs, const ProductDesc& one,
-                                uint32_t count, bool square, int log_n, int out_fmt, uint32_t bpp,
+// The four launches of `count` products of one form (digits of both operands
+// together at most 2^log_n + 1); each product's carry scan has `bpp` blocks
+// (tickets).
+cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const ProductDesc& one,
+                                uint32_t count, bool square, int out_fmt, uint32_t bpp,
                                 const CarryLaunch& cl, cudaStream_t st, cudaEvent_t* ev);
 
 // The same for any number of products in the device array `descs`, in pieces
 // that fit a launch grid, all on one ticket sequence from cl.ticket_base.
-cudaError_t launch_wide_batch(const NttConsts& host, const ProductDesc* descs, uint32_t count, bool square, int log_n,
-                              int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st);
+cudaError_t launch_wide_batch(WideForm f, const ProductDesc* descs, uint32_t count, bool square, int out_fmt,
+                              uint32_t bpp, const CarryLaunch& cl, cudaStream_t st);
 
 }  // namespace bgpu

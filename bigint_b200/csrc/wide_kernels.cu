@@ -50,7 +50,9 @@ __host__ __device__ constexpr uint32_t wide_row_words(int l1, bool square) {
     return ((square || wide_one_buffer(l1) ? 1u : 2u) << l1) + 32u + (l1 >= 10 ? 0u : (uint32_t)wide_row_threads(l1) % 32u);
 }
 
-__constant__ NttConsts c_wide[2];  // lazy, strict
+__constant__ NttConsts c_wide[kNumSets - kFirstWideSet];  // lazy and strict of five, six and seven primes
+
+__host__ __device__ constexpr int wide_set_index(int np, bool lazy) { return 2 * (np - kWidePrimes) + (lazy ? 0 : 1); }
 
 __device__ __forceinline__ ProductDesc wide_product(const WideArgs& a, uint32_t i) {
     return a.descs ? a.descs[i] : a.one;
@@ -86,29 +88,51 @@ __device__ __forceinline__ uint32_t shoup2(uint32_t x, uint2 s, uint2 b, uint32_
 
 // ---- 1: forward columns -----------------------------------------------------------
 
-// 64-bit digit n of an operand (0 beyond its length).
-template <bool LIMB>
-__device__ __forceinline__ uint64_t load_digit64(const OperandDesc& in, uint32_t nd, uint32_t n) {
-    if (n >= nd) return 0;
-    if constexpr (LIMB) {
-        return __ldg(static_cast<const unsigned long long*>(in.ptr) + n);
+// 32-bit word w of an operand of 28-bit digits (0 beyond its length).
+__device__ __forceinline__ uint32_t load_word28(const OperandDesc& in, uint64_t w) {
+    const uint32_t* d = static_cast<const uint32_t*>(in.ptr);
+    const uint64_t bit = w * 32;
+    const uint32_t i = (uint32_t)(bit / 28), sh = (uint32_t)(bit - (uint64_t)i * 28);  // sh in {0, 4, ..., 24}
+    uint32_t v = i < in.nsrc ? __ldg(d + i) >> sh : 0u;
+    if (i + 1 < in.nsrc) v |= __ldg(d + i + 1) << (28 - sh);
+    return v;
+}
+
+// Digit n of an operand (0 beyond its nd digits): its words, the unused ones 0.
+template <int NP, bool LIMB>
+__device__ __forceinline__ void load_digit(const OperandDesc& in, uint32_t nd, uint32_t n, uint32_t (&d)[3]) {
+    d[0] = d[1] = d[2] = 0;
+    if (n >= nd) return;
+    if constexpr (NP == 5 && LIMB) {
+        const uint64_t v = __ldg(static_cast<const unsigned long long*>(in.ptr) + n);
+        d[0] = (uint32_t)v, d[1] = (uint32_t)(v >> 32);
     } else {
-        const uint32_t* d = static_cast<const uint32_t*>(in.ptr);
-        const uint64_t bit = (uint64_t)n * 64;
-        const uint32_t i = (uint32_t)(bit / 28), sh = (uint32_t)(bit - (uint64_t)i * 28);  // sh in {0, 4, ..., 24}
-        uint64_t v = __ldg(d + i) >> sh;
-        if (i + 1 < in.nsrc) v |= (uint64_t)__ldg(d + i + 1) << (28 - sh);
-        if (i + 2 < in.nsrc) v |= (uint64_t)__ldg(d + i + 2) << (56 - sh);
-        if (sh > 20 && i + 3 < in.nsrc) v |= (uint64_t)__ldg(d + i + 3) << (84 - sh);
-        return v;
+        const uint64_t w = ((uint64_t)n * wide_bits(NP)) >> 5;
+        constexpr int NW = NP == 5 ? 2 : 3;
+        if constexpr (LIMB) {
+            const uint32_t* x = static_cast<const uint32_t*>(in.ptr);
+            const uint64_t words = 2 * (uint64_t)in.nsrc;
+#pragma unroll
+            for (int k = 0; k < NW; ++k)
+                if (k == 0 || w + k < words) d[k] = __ldg(x + w + k);
+        } else {
+#pragma unroll
+            for (int k = 0; k < NW; ++k) d[k] = load_word28(in, w + k);
+        }
+        if constexpr (NP == 6) {  // 80 bits from an even or an odd half word
+            const uint32_t sh = (n & 1u) * 16u;
+            d[0] = __funnelshift_r(d[0], d[1], sh);
+            d[1] = __funnelshift_r(d[1], d[2], sh);
+            d[2] = (d[2] >> sh) & 0xffffu;
+        }
     }
 }
 
-// Round 0: rows n2 = base + (j << LO) read from the operand.  A digit
-// becomes digit 2^-32 mod p (the scale of the row pass undoes it), in [0, 2p)
-// or [0, p).  HALF: the rows of the upper half of the transform are zero; they
+// Round 0: rows n2 = base + (j << LO) read from the operand.  A digit of
+// two words becomes digit 2^-32 mod p, of three digit 2^-64 mod p (the scale of
+// the row pass undoes it), in [0, 2p) or [0, p).  HALF: the rows of the upper half of the transform are zero; they
 // are not loaded and the first stage is one multiply per pair.
-template <bool LAZY, int L2, int T, bool LIMB, bool HALF>
+template <bool LAZY, int L2, int T, int NP, bool LIMB, bool HALF>
 __device__ __forceinline__ void wide_round0(const WideArgs& a, const OperandDesc& in, uint32_t nd, const NttConsts& c,
                                             int q, uint32_t c0, uint32_t* sm) {
     using Gr = Group<L2, kWideCols, 0>;
@@ -122,16 +146,23 @@ __device__ __forceinline__ void wide_round0(const WideArgs& a, const OperandDesc
     for (int g = threadIdx.x; g < Gr::G; g += T) {
         const Gr gr(g);
         uint32_t x[1 << R];
-        uint64_t any = 0;
+        uint32_t any = 0;
         uint32_t n = c0 + gr.col + (gr.base << a.log_n1);
 #pragma unroll
         for (int j = 0; j < NL; ++j, n += stride) {
-            const uint64_t v = load_digit64<LIMB>(in, nd, n);
-            any |= v;
-            uint32_t hi = (uint32_t)(v >> 32);
-            hi -= __umulhi(hi, red) * p;  // [0, 2p)
-            if (!LAZY) hi = csub(hi, p);
-            const uint32_t r = redc((uint32_t)v, hi, p, np);  // one p more
+            uint32_t d[3];
+            load_digit<NP, LIMB>(in, nd, n, d);
+            any |= d[0] | d[1] | d[2];
+            d[1] -= __umulhi(d[1], red) * p;  // [0, 2p)
+            if (!LAZY) d[1] = csub(d[1], p);
+            uint32_t r = redc(d[0], d[1], p, np);  // one p more
+            if constexpr (NP > 5) {
+                if (NP == 7) {  // 80-bit digits have 16 bits here
+                    d[2] -= __umulhi(d[2], red) * p;
+                    if (!LAZY) d[2] = csub(d[2], p);
+                }
+                r = redc(r, d[2], p, np);  // below d[2] + p + 1
+            }
             x[j] = LAZY ? csub(r, 2 * p) : csub(r, p);
         }
         if (any) {
@@ -163,13 +194,13 @@ __host__ __device__ constexpr int wide_col_blocks(int l2, bool fwd) {
     return l2 == 9 ? 5 : l2 == 11 && !fwd ? 3 : 1024 / wide_col_threads(l2, fwd);
 }
 
-template <bool LAZY, int L2, int T>
+template <bool LAZY, int L2, int T, int NP>
 __global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const WideArgs a) {
     using P2 = Plan<L2>;
     constexpr int NR = P2::nr, RL = P2::r(NR - 1), SROW = (1 << RL) + 1;
     static_assert(NR > 1, "column passes of several rounds");
     extern __shared__ __align__(16) uint32_t sm[];  // [2^L2][8] and the column powers
-    const NttConsts& c = c_wide[LAZY ? 0 : 1];
+    const NttConsts& c = c_wide[wide_set_index(NP, LAZY)];
     const int q = blockIdx.y, op = (int)(blockIdx.z % (uint32_t)a.nops);
     const ProductDesc pd = wide_product(a, blockIdx.z / (uint32_t)a.nops);
     const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
@@ -177,7 +208,7 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const
     const OperandDesc in = op == 0 ? pd.op[0] : pd.op[1];
     const uint32_t c0 = blockIdx.x * kWideCols;
     const size_t nn = (size_t)1 << a.log_n;
-    uint32_t* y = pd.y + ((size_t)op * kWidePrimes + q) * nn;
+    uint32_t* y = pd.y + ((size_t)op * NP + q) * nn;
 
     // The last round's groups hold slots base + j of one column n1, whose
     // inter-pass twiddle is omega_N^(n1 bitrev(base)) S^bitrev(j): sS[col][m]
@@ -189,17 +220,17 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const
             inter_twiddle(c, q, 0, (((c0 + col) * m) << (L2 - RL)) & (uint32_t)(nn - 1), a.log_n, p), p, np);
     }
     pdl_wait();
-    const uint32_t nd = wide_digits(in);
+    const uint32_t nd = wide_digits(NP, in.nd32);
     if (in.fmt == kFmtLimb64) {
         if (2 * (size_t)nd <= nn)
-            wide_round0<LAZY, L2, T, true, true>(a, in, nd, c, q, c0, sm);
+            wide_round0<LAZY, L2, T, NP, true, true>(a, in, nd, c, q, c0, sm);
         else
-            wide_round0<LAZY, L2, T, true, false>(a, in, nd, c, q, c0, sm);
+            wide_round0<LAZY, L2, T, NP, true, false>(a, in, nd, c, q, c0, sm);
     } else {
         if (2 * (size_t)nd <= nn)
-            wide_round0<LAZY, L2, T, false, true>(a, in, nd, c, q, c0, sm);
+            wide_round0<LAZY, L2, T, NP, false, true>(a, in, nd, c, q, c0, sm);
         else
-            wide_round0<LAZY, L2, T, false, false>(a, in, nd, c, q, c0, sm);
+            wide_round0<LAZY, L2, T, NP, false, false>(a, in, nd, c, q, c0, sm);
     }
     __syncthreads();
     dif_rounds<LAZY, L2, kWideCols, T, 1, NR - 2>(sm, tw, p, threadIdx.x);
@@ -234,7 +265,7 @@ __host__ __device__ constexpr int wide_row_blocks(int l1) {
 
 template <bool LAZY, int L1, bool SQR>
 __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1), wide_row_blocks(L1))
-    k_wide_rows(const WideArgs a) {
+    k_wide_rows(const __grid_constant__ WideArgs a) {
     constexpr int T = wide_row_threads(L1);
     constexpr bool MULTI = wide_rows_per_cta(L1) > 1;
     constexpr bool ONE = !SQR && wide_one_buffer(L1);
@@ -243,7 +274,7 @@ __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1), 
     constexpr int R0 = P1::r(0), LO0 = P1::lo(0);
     static_assert(NR > 1, "rows of several rounds");
     extern __shared__ __align__(16) uint32_t sm[];  // per row: A's row, B's, the powers
-    const NttConsts& c = c_wide[LAZY ? 0 : 1];
+    const NttConsts& c = c_wide[a.set];
     const uint32_t sub = MULTI ? threadIdx.x / T : 0u;
     uint32_t* sa = sm + sub * wide_row_words(L1, SQR);
     uint32_t* sb = ONE ? sa : sa + (1u << L1);
@@ -256,9 +287,9 @@ __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1), 
     const uint2* twi = c.stage[q][1];
     const size_t nn = (size_t)1 << a.log_n;
     uint32_t* row_a = pd.y + q * nn + ((size_t)slot << L1);
-    const uint32_t* row_b = row_a + kWidePrimes * nn;
+    const uint32_t* row_b = row_a + a.np * nn;
     const uint32_t k2 = bitrev(slot, a.log_n - L1);
-    const uint32_t scale = q == 0 ? a.scale[0] : q == 1 ? a.scale[1] : q == 2 ? a.scale[2] : q == 3 ? a.scale[3] : a.scale[4];
+    const uint32_t scale = a.scale[q];
 
     // The last DIT round's groups hold n1 = base + (j << LO0): twiddle
     // omega_N^-(k2 base) sT[j], sT[j] = omega_N^-(k2 j << LO0).
@@ -343,7 +374,7 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, false)) k_wide_inv(cons
     using P2 = Plan<L2>;
     constexpr int NR = P2::nr;
     extern __shared__ __align__(16) uint32_t sm[];  // [2^L2][8]
-    const NttConsts& c = c_wide[LAZY ? 0 : 1];
+    const NttConsts& c = c_wide[a.set];
     const int q = blockIdx.y;
     const uint32_t p = c.pr[q].p;
     const uint2* twi = c.stage[q][1];
@@ -398,57 +429,83 @@ __device__ __forceinline__ void mac(uint32_t a, uint32_t b, uint32_t (&C)[2]) {
         : "r"(a), "r"(b));
 }
 
-// Adds the coefficient with residues y (each below its p) to the words W[0..4],
-// W[4] taking the carry: sum y_i M/p_i - q M.  The five products of a 32-bit
-// limb of the M/p_i sum to a 64-bit column and a carry count (LAZY: the first
-// four, p < 2^30, cannot overflow).  q = floor(sum y_i / p_i) in single
+// W += v on N words; the carry out is dropped.
+template <int N>
+__device__ __forceinline__ void add_words(uint32_t* W, const uint32_t* v) {
+    static_assert(N >= 3, "add_words");
+    if constexpr (N == 3)
+        asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+            : "+r"(W[0]), "+r"(W[1]), "+r"(W[2])
+            : "r"(v[0]), "r"(v[1]), "r"(v[2]));
+    else if constexpr (N == 4)
+        asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;"
+            : "+r"(W[0]), "+r"(W[1]), "+r"(W[2]), "+r"(W[3])
+            : "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
+    else if constexpr (N == 5)
+        asm("add.cc.u32 %0, %0, %5;\n\taddc.cc.u32 %1, %1, %6;\n\taddc.cc.u32 %2, %2, %7;\n\t"
+            "addc.cc.u32 %3, %3, %8;\n\taddc.u32 %4, %4, %9;"
+            : "+r"(W[0]), "+r"(W[1]), "+r"(W[2]), "+r"(W[3]), "+r"(W[4])
+            : "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]));
+    else if constexpr (N == 6)
+        asm("add.cc.u32 %0, %0, %6;\n\taddc.cc.u32 %1, %1, %7;\n\taddc.cc.u32 %2, %2, %8;\n\t"
+            "addc.cc.u32 %3, %3, %9;\n\taddc.cc.u32 %4, %4, %10;\n\taddc.u32 %5, %5, %11;"
+            : "+r"(W[0]), "+r"(W[1]), "+r"(W[2]), "+r"(W[3]), "+r"(W[4]), "+r"(W[5])
+            : "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]));
+    else if constexpr (N == 7)
+        asm("add.cc.u32 %0, %0, %7;\n\taddc.cc.u32 %1, %1, %8;\n\taddc.cc.u32 %2, %2, %9;\n\t"
+            "addc.cc.u32 %3, %3, %10;\n\taddc.cc.u32 %4, %4, %11;\n\taddc.cc.u32 %5, %5, %12;\n\taddc.u32 %6, %6, %13;"
+            : "+r"(W[0]), "+r"(W[1]), "+r"(W[2]), "+r"(W[3]), "+r"(W[4]), "+r"(W[5]), "+r"(W[6])
+            : "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]));
+    else {
+        uint32_t cy = 0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const uint64_t t = (uint64_t)W[k] + v[k] + cy;
+            W[k] = (uint32_t)t;
+            cy = (uint32_t)(t >> 32);
+        }
+    }
+}
+
+// Adds the coefficient with residues y (each below its p) to the words
+// W[0 .. NP-1], the last taking the carry: sum y_i M/p_i - q M.  The NP products of
+// a 32-bit limb of the M/p_i sum to a 64-bit column and a carry count (LAZY: the
+// first four, p < 2^30, cannot overflow).  q = floor(sum y_i / p_i) in single
 // precision from the top bits of y_i, put below an exponent byte: the float is
 // 2^23 + floor(y_i / 256), and c.bias takes the 2^23 out again.  x / M is below
 // 0.9 and the bias keeps 0.05 on either side, well above the rounding.  -q M
-// comes from a table in shared memory (`nqm`, five words a q): lanes with
+// comes from a table in shared memory (`nqm`, NP words a q): lanes with
 // different q hit different banks there, a constant bank would serve them one
 // by one (measured the constant bank: 29.5 us for the whole pass at 2^21 points, with the table 26.8).
-template <bool LAZY>
-__device__ __forceinline__ void add_crt5(const WideCrt& c, const uint32_t* nqm, const uint32_t (&y)[kWidePrimes],
-                                         uint32_t* W) {
+template <bool LAZY, int NP>
+__device__ __forceinline__ void add_crt(const WideCrt& c, const uint32_t* nqm, const uint32_t (&y)[NP], uint32_t* W) {
     float f = c.bias;
 #pragma unroll
-    for (int i = 0; i < kWidePrimes; ++i) f = fmaf(__uint_as_float(__byte_perm(y[i], 0x4b000000u, 0x7321)), c.inv[i], f);
-    const uint32_t* s = nqm + 5 * min((int)f, kWideMaxQ - 1);
-    uint32_t C[4][2], k[4] = {0, 0, 0, 0};
+    for (int i = 0; i < NP; ++i) f = fmaf(__uint_as_float(__byte_perm(y[i], 0x4b000000u, 0x7321)), c.inv[i], f);
+    const uint32_t* s = nqm + NP * min((int)f, NP - 1);
+    uint32_t lo[NP], hi[NP], k[NP] = {};  // columns and their carry counts
 #pragma unroll
-    for (int l = 0; l < 4; ++l) {
+    for (int l = 0; l < NP - 1; ++l) {
         const uint64_t t = (uint64_t)y[0] * c.m[0][l];
-        C[l][0] = (uint32_t)t, C[l][1] = (uint32_t)(t >> 32);
+        uint32_t C[2] = {(uint32_t)t, (uint32_t)(t >> 32)};
 #pragma unroll
-        for (int i = 1; i < kWidePrimes; ++i) {
+        for (int i = 1; i < NP; ++i) {
             if (LAZY && i < 4)
-                mac(y[i], c.m[i][l], C[l]);
+                mac(y[i], c.m[i][l], C);
             else
-                mac_count(y[i], c.m[i][l], C[l], k[l]);
+                mac_count(y[i], c.m[i][l], C, k[l]);
         }
+        lo[l] = C[0], hi[l] = C[1];
     }
-    // words of the sum: C0.lo | C0.hi + C1.lo | C1.hi + C2.lo + k0 | C2.hi + C3.lo + k1 | C3.hi + k2
-    asm("add.cc.u32 %0, %0, %5;\n\t"
-        "addc.cc.u32 %1, %1, %6;\n\t"
-        "addc.cc.u32 %2, %2, %7;\n\t"
-        "addc.cc.u32 %3, %3, %8;\n\t"
-        "addc.u32 %4, %4, %9;\n\t"
-        "add.cc.u32 %1, %1, %10;\n\t"
-        "addc.cc.u32 %2, %2, %11;\n\t"
-        "addc.cc.u32 %3, %3, %12;\n\t"
-        "addc.u32 %4, %4, %13;\n\t"
-        "add.cc.u32 %2, %2, %14;\n\t"
-        "addc.cc.u32 %3, %3, %15;\n\t"
-        "addc.u32 %4, %4, 0;\n\t"
-        "add.cc.u32 %0, %0, %16;\n\t"
-        "addc.cc.u32 %1, %1, %17;\n\t"
-        "addc.cc.u32 %2, %2, %18;\n\t"
-        "addc.cc.u32 %3, %3, %19;\n\t"
-        "addc.u32 %4, %4, %20;"
-        : "+r"(W[0]), "+r"(W[1]), "+r"(W[2]), "+r"(W[3]), "+r"(W[4])
-        : "r"(C[0][0]), "r"(C[1][0]), "r"(C[2][0]), "r"(C[3][0]), "r"(k[2]), "r"(C[0][1]), "r"(C[1][1]), "r"(C[2][1]),
-          "r"(C[3][1]), "r"(k[0]), "r"(k[1]), "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]));
+    lo[NP - 1] = k[NP - 3];  // word l + 2 takes column l's count; the sum is mod 2^(32 NP)
+    k[NP - 3] = 0;
+    add_words<NP>(W, lo);
+    add_words<NP - 1>(W + 1, hi);
+    add_words<NP - 2>(W + 2, k);
+    uint32_t m[NP];
+#pragma unroll
+    for (int l = 0; l < NP; ++l) m[l] = s[l];
+    add_words<NP>(W, m);
 }
 
 __device__ __forceinline__ uint64_t add_c(uint64_t a, uint64_t b, uint32_t& cy) {
@@ -457,44 +514,59 @@ __device__ __forceinline__ uint64_t add_c(uint64_t a, uint64_t b, uint32_t& cy) 
     return r;
 }
 
-// Chunk c (coefficients 4c .. 4c+3): their exact sum as 256 bits D and a
-// spill of two limbs (below 2^90).
-template <bool LAZY>
-__device__ __forceinline__ void chunk5(const WideCrt& crt, const uint32_t* nqm, const uint32_t* y, size_t nn, size_t c, uint64_t (&D)[4],
-                                       uint64_t (&sp)[2]) {
-    uint32_t r[4][kWidePrimes];
+// Chunk c (coefficients 4c .. 4c+3): their exact sum as the chunk's NP - 1 limbs D
+// and a spill of two limbs (below 2^122: a coefficient is below 2^(2 D + 22) for
+// digits of D <= 96 bits).
+template <bool LAZY, int NP>
+__device__ __forceinline__ void chunk_sum(const WideCrt& crt, const uint32_t* nqm, const uint32_t* y, size_t nn,
+                                          size_t c, uint64_t (&D)[NP - 1], uint64_t (&sp)[2]) {
+    uint32_t r[4][NP];
 #pragma unroll
-    for (int i = 0; i < kWidePrimes; ++i) {
+    for (int i = 0; i < NP; ++i) {
         const uint4 v = *reinterpret_cast<const uint4*>(y + i * nn + 4 * c);
         r[0][i] = v.x, r[1][i] = v.y, r[2][i] = v.z, r[3][i] = v.w;
     }
-    uint32_t W[12] = {};
+    // A coefficient is added where the words above the sum so far are still
+    // zero, and the sum so far leaves room in its NP words.
+    uint32_t W[2 * (NP + 1)] = {};
+    if constexpr (NP == 6) {  // 80-bit digits: the odd ones start in the middle of a word
+        uint32_t O[11] = {};
+        add_crt<LAZY, NP>(crt, nqm, r[0], W);
+        add_crt<LAZY, NP>(crt, nqm, r[2], W + 5);
+        add_crt<LAZY, NP>(crt, nqm, r[1], O);
+        add_crt<LAZY, NP>(crt, nqm, r[3], O + 5);
+        uint32_t V[12];
+        V[0] = O[0] << 16;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        // the coefficient is added from word 2k; the words from 2k + 4 on are
-        // still zero, and the sum so far stays below 2^(64 k + 160)
-        add_crt5<LAZY>(crt, nqm, r[k], W + 2 * k);
+        for (int k = 1; k < 11; ++k) V[k] = __funnelshift_l(O[k - 1], O[k], 16);
+        V[11] = O[10] >> 16;
+        add_words<12>(W + 2, V);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) add_crt<LAZY, NP>(crt, nqm, r[k], W + k * (int)(wide_bits(NP) / 32));
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) D[k] = W[2 * k] | ((uint64_t)W[2 * k + 1] << 32);
-    sp[0] = W[8] | ((uint64_t)W[9] << 32);
-    sp[1] = W[10] | ((uint64_t)W[11] << 32);
+    for (int k = 0; k < NP - 1; ++k) D[k] = W[2 * k] | ((uint64_t)W[2 * k + 1] << 32);
+    sp[0] = W[2 * NP - 2] | ((uint64_t)W[2 * NP - 1] << 32);
+    sp[1] = W[2 * NP] | ((uint64_t)W[2 * NP + 1] << 32);
 }
 
 // The 28-bit digits that start in chunk c, whose final limbs are S; the last
 // one may reach into the final low limb `next` of the chunk above.
-__device__ __forceinline__ void store_digits28(uint32_t* o, size_t out_cap, uint64_t c, const uint64_t (&S)[4],
+template <int NL>
+__device__ __forceinline__ void store_digits28(uint32_t* o, size_t out_cap, uint64_t c, const uint64_t (&S)[NL],
                                                uint64_t next) {
+    constexpr uint32_t kBits = 64 * NL;
     const uint64_t mask = (1u << 28) - 1u;
-    const uint64_t bit0 = c * 256;
+    const uint64_t bit0 = c * kBits;
     uint64_t k = (bit0 + 27) / 28;
-    const uint64_t kend = min((bit0 + 256 + 27) / 28, (uint64_t)out_cap);
+    const uint64_t kend = min((bit0 + kBits + 27) / 28, (uint64_t)out_cap);
     const uint32_t off0 = (uint32_t)(k * 28 - bit0);  // < 28
     uint64_t cur = S[0] >> off0;
     int have = 64 - (int)off0;
 #pragma unroll
-    for (int w = 1; w <= 4; ++w) {
-        const uint64_t nxtw = w < 4 ? S[w & 3] : next;
+    for (int w = 1; w <= NL; ++w) {
+        const uint64_t nxtw = w < NL ? S[w % NL] : next;
         while (have >= 28) {
             if (k < kend) o[k] = (uint32_t)(cur & mask);
             ++k;
@@ -508,21 +580,22 @@ __device__ __forceinline__ void store_digits28(uint32_t* o, size_t out_cap, uint
     }
 }
 
-// One 256-bit chunk a thread, 256 chunks a block; a ninth warp recomputes the
+// One chunk of NP - 1 limbs a thread, 256 chunks a block; a ninth warp recomputes the
 // 32 chunks below the block, whose carries almost always settle the block's
 // carry-in without waiting for another block (else the decoupled look-back on
 // the blocks' flags, in ticket order).  Chunk c's value is
-// (D_c + spill_{c-1} + carry_c) mod 2^256 with one-bit carries.
+// (D_c + spill_{c-1} + carry_c) mod 2^(64 (NP - 1)) with one-bit carries.
 constexpr int kWideCarryWarps = kWideCarryChunks / 32;
-template <bool LAZY>
+template <bool LAZY, int NP>
 __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __grid_constant__ WideCarryArgs a) {
+    constexpr int NL = NP - 1;
     __shared__ uint32_t s_bid, s_cin, s_win_g, s_win_p;
     __shared__ uint32_t s_wg[kWideCarryWarps], s_wp[kWideCarryWarps];
     __shared__ uint64_t s_sp[kWideCarryWarps + 1][2];
     __shared__ uint64_t s_low[kWideCarryChunks];  // 28-bit output: each chunk's low limb before its spill and carry
-    __shared__ uint32_t s_nqm[kWideMaxQ * 5];
+    __shared__ uint32_t s_nqm[NP * NP];
     if (threadIdx.x == 0) s_bid = (uint32_t)(atomicAdd(a.ticket, 1ull) - a.ticket_base);
-    for (int i = threadIdx.x; i < kWideMaxQ * 5; i += kWideCarryChunks + 32) s_nqm[i] = a.crt.nqm[i / 5][i % 5];
+    for (int i = threadIdx.x; i < NP * NP; i += kWideCarryChunks + 32) s_nqm[i] = a.crt.nqm[i / NP][i % NP];
     __syncthreads();
     pdl_wait();
     pdl_trigger();
@@ -533,14 +606,14 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
     const uint32_t bid = s_bid % a.bpp;
     const ProductDesc pd = a.descs ? a.descs[s_bid / a.bpp] : a.one;
     // a product of a batch shorter than its class's longest: no later block waits on these
-    if (bid >= wide_carry_blocks(pd.out_cap, a.out_fmt)) return;
+    if (bid >= wide_carry_blocks(NP, pd.out_cap, a.out_fmt)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool window = warp == kWideCarryWarps;
     const size_t nn = (size_t)1 << a.log_n;
     const uint32_t nch = (uint32_t)(nn / 4);
     const int64_t c = (int64_t)bid * kWideCarryChunks + (window ? lane - 32 : (int)threadIdx.x);
-    uint64_t S[4] = {0, 0, 0, 0}, sp[2] = {0, 0};
-    if (c >= 0 && c < nch) chunk5<LAZY>(a.crt, s_nqm, pd.y, nn, (size_t)c, S, sp);
+    uint64_t S[NL] = {}, sp[2] = {0, 0};
+    if (c >= 0 && c < nch) chunk_sum<LAZY, NP>(a.crt, s_nqm, pd.y, nn, (size_t)c, S, sp);
     if (!window) s_low[threadIdx.x] = S[0];
     if (lane == 31) {
         s_sp[warp][0] = sp[0];
@@ -555,9 +628,13 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
     uint32_t g = 0;
     S[0] = add_c(S[0], p0, g);
     S[1] = add_c(S[1], p1, g);
-    S[2] = add_c(S[2], 0, g);
-    S[3] = add_c(S[3], 0, g);
-    const uint32_t pbit = (S[0] & S[1] & S[2] & S[3]) == ~0ull;
+    uint64_t all = S[0] & S[1];
+#pragma unroll
+    for (int k = 2; k < NL; ++k) {
+        S[k] = add_c(S[k], 0, g);
+        all &= S[k];
+    }
+    const uint32_t pbit = all == ~0ull;
     // the window's lowest chunk lacks its predecessor's spill: it neither
     // stops nor makes a carry there, except below chunk 0
     const uint32_t gm = __ballot_sync(0xffffffffu, g);
@@ -617,21 +694,21 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
     const uint32_t carries = (uint32_t)sum ^ gm ^ bm;
     uint32_t cy = (carries >> lane) & 1u;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < NL; ++k) {
         const uint64_t t = S[k] + cy;
         cy = cy & (t == 0);
         S[k] = t;
     }
     if (a.out_fmt == kFmtLimb64) {
         uint64_t* o = static_cast<uint64_t*>(pd.out);
-        const size_t at = (size_t)c * 4;
-        if (at + 4 <= pd.out_cap && (reinterpret_cast<uintptr_t>(o) & 15u) == 0) {
+        const size_t at = (size_t)c * NL;
+        if (NL % 2 == 0 && at + NL <= pd.out_cap && (reinterpret_cast<uintptr_t>(o) & 15u) == 0) {
             ulonglong2* d = reinterpret_cast<ulonglong2*>(o + at);
-            d[0] = make_ulonglong2(S[0], S[1]);
-            d[1] = make_ulonglong2(S[2], S[3]);
+#pragma unroll
+            for (int k = 0; k + 1 < NL; k += 2) d[k / 2] = make_ulonglong2(S[k], S[k + 1]);
         } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < NL; ++k)
                 if (at + k < pd.out_cap) o[at + k] = S[k];
         }
     } else {
@@ -639,14 +716,14 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
         if (threadIdx.x + 1 < kWideCarryChunks) {
             next = s_low[threadIdx.x + 1];
         } else if (c + 1 < nch) {
-            uint32_t r[kWidePrimes], w[5] = {};
+            uint32_t r[NP], w[NP] = {};
 #pragma unroll
-            for (int i = 0; i < kWidePrimes; ++i) r[i] = pd.y[i * nn + 4 * (size_t)(c + 1)];
-            add_crt5<LAZY>(a.crt, s_nqm, r, w);
+            for (int i = 0; i < NP; ++i) r[i] = pd.y[i * nn + 4 * (size_t)(c + 1)];
+            add_crt<LAZY, NP>(a.crt, s_nqm, r, w);
             next = w[0] | ((uint64_t)w[1] << 32);
         }
         next += sp[0] + (lane == 31 ? (uint32_t)(sum >> 32) & 1u : (carries >> (lane + 1)) & 1u);
-        store_digits28(static_cast<uint32_t*>(pd.out), pd.out_cap, (uint64_t)c, S, next);
+        store_digits28<NL>(static_cast<uint32_t*>(pd.out), pd.out_cap, (uint64_t)c, S, next);
     }
 }
 
@@ -654,20 +731,25 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
 
 namespace {
 
+template <bool LAZY, int L2, int NP>
+cudaError_t launch_fwd(const WideArgs& a, uint32_t count, cudaStream_t st) {
+    constexpr int RL = Plan<L2>::r(Plan<L2>::nr - 1);
+    const size_t sm = ((size_t)kWideCols * 4 << L2) + kWideCols * ((1 << RL) + 1) * sizeof(uint2);
+    auto k = k_wide_fwd<LAZY, L2, wide_col_threads(L2, true), NP>;
+    allow_smem(k, sm);
+    return launch_k(k, dim3((1u << a.log_n1) / kWideCols, NP, count * a.nops), dim3(wide_col_threads(L2, true)), sm, st,
+                    a);
+}
 template <bool LAZY, int L2>
 cudaError_t launch_cols(bool fwd, const WideArgs& a, uint32_t count, cudaStream_t st) {
-    constexpr int RL = Plan<L2>::r(Plan<L2>::nr - 1);
+    if (fwd)
+        return a.np == 5   ? launch_fwd<LAZY, L2, 5>(a, count, st)
+               : a.np == 6 ? launch_fwd<LAZY, L2, 6>(a, count, st)
+                           : launch_fwd<LAZY, L2, 7>(a, count, st);
     const size_t tile = (size_t)kWideCols * 4 << L2;
-    const uint32_t tiles = (1u << a.log_n1) / kWideCols;
-    if (fwd) {
-        auto k = k_wide_fwd<LAZY, L2, wide_col_threads(L2, true)>;
-        const size_t sm = tile + kWideCols * ((1 << RL) + 1) * sizeof(uint2);
-        allow_smem(k, sm);
-        return launch_k(k, dim3(tiles, kWidePrimes, count * a.nops), dim3(wide_col_threads(L2, true)), sm, st, a);
-    }
     auto k = k_wide_inv<LAZY, L2, wide_col_threads(L2, false)>;
     allow_smem(k, tile);
-    return launch_k(k, dim3(tiles, kWidePrimes, count), dim3(wide_col_threads(L2, false)), tile, st, a);
+    return launch_k(k, dim3((1u << a.log_n1) / kWideCols, a.np, count), dim3(wide_col_threads(L2, false)), tile, st, a);
 }
 
 template <bool LAZY>
@@ -690,7 +772,7 @@ cudaError_t launch_rows_of(const WideArgs& a, uint32_t count, cudaStream_t st) {
     const size_t sm = (size_t)RP * wide_row_words(L1, SQR) * 4;
     auto k = k_wide_rows<LAZY, L1, SQR>;
     allow_smem(k, sm);
-    return launch_k(k, dim3((1u << (a.log_n - L1)) / RP, kWidePrimes, count), dim3(wide_row_threads(L1) * RP), sm, st, a);
+    return launch_k(k, dim3((1u << (a.log_n - L1)) / RP, a.np, count), dim3(wide_row_threads(L1) * RP), sm, st, a);
 }
 template <bool LAZY, int L1>
 cudaError_t launch_rows(const WideArgs& a, bool square, uint32_t count, cudaStream_t st) {
@@ -714,34 +796,36 @@ cudaError_t dispatch_rows(int l1, const WideArgs& a, bool square, uint32_t count
     }
 }
 
-WideCrt make_crt(const NttConsts& h) {
+WideCrt make_crt(const PrimeSetInfo& ps) {
     WideCrt c{};
+    const int np = ps.np;
     double off = 0;
-    uint32_t M[5] = {1, 0, 0, 0, 0};
-    auto times = [](uint32_t (&x)[5], uint32_t v) {
+    using Words = uint32_t[kWideMaxPrimes];
+    auto times = [np](Words& x, uint32_t v) {
         uint64_t cy = 0;
-        for (auto& w : x) {
-            cy += (uint64_t)w * v;
-            w = (uint32_t)cy;
+        for (int k = 0; k < np; ++k) {
+            cy += (uint64_t)x[k] * v;
+            x[k] = (uint32_t)cy;
             cy >>= 32;
         }
     };
-    for (int i = 0; i < kWidePrimes; ++i) {
-        uint32_t x[5] = {1, 0, 0, 0, 0};
-        for (int j = 0; j < kWidePrimes; ++j)
-            if (j != i) times(x, h.pr[j].p);
+    Words M = {1};
+    for (int i = 0; i < np; ++i) {
+        Words x = {1};
+        for (int j = 0; j < np; ++j)
+            if (j != i) times(x, ps.p[j]);
         std::memcpy(c.m[i], x, sizeof(c.m[i]));
-        times(M, h.pr[i].p);
-        c.inv[i] = (float)(256.0 / h.pr[i].p);
+        times(M, ps.p[i]);
+        c.inv[i] = (float)(256.0 / ps.p[i]);
         off += 8388608.0 * (double)c.inv[i];
     }
     c.bias = (float)(0.05 - off);
-    for (int q = 0; q < kWideMaxQ; ++q) {
-        uint32_t x[5];
+    for (int q = 0; q < np; ++q) {
+        Words x;
         std::memcpy(x, M, sizeof(x));
         times(x, (uint32_t)q);
         uint64_t cy = 1;  // its negative
-        for (int k = 0; k < 5; ++k) {
+        for (int k = 0; k < np; ++k) {
             cy += (uint32_t)~x[k];
             c.nqm[q][k] = (uint32_t)cy;
             cy >>= 32;
@@ -757,30 +841,32 @@ uint32_t pow_m(uint64_t b, uint32_t e, uint32_t p) {
     return (uint32_t)r;
 }
 
-// 2^96 / N / (M / p) mod p, times 2^32: the digits' two factors 2^-32 and the
-// pointwise product's, the inverse transform's 1/N, the CRT's (M/p)^-1.
-void set_scale(const NttConsts& h, int log_n, uint32_t* scale) {
-    for (int i = 0; i < kWidePrimes; ++i) {
-        const uint32_t p = h.pr[i].p;
+// 1 / N / (M / p) mod p times a power of two, Montgomery form: the inverse
+// transform's 1/N, the CRT's (M/p)^-1, and 2^32 for the pointwise product and
+// each reduction of the two digits (one each, two for three words).
+void set_scale(const PrimeSetInfo& ps, int log_n, uint32_t* scale) {
+    for (int i = 0; i < ps.np; ++i) {
+        const uint32_t p = ps.p[i];
         uint64_t d = pow_m(2, (uint32_t)log_n, p);
-        for (int j = 0; j < kWidePrimes; ++j)
-            if (j != i) d = d * (h.pr[j].p % p) % p;
-        const uint64_t v = (uint64_t)pow_m(d, p - 2, p) * pow_m(2, 96, p) % p;
+        for (int j = 0; j < ps.np; ++j)
+            if (j != i) d = d * (ps.p[j] % p) % p;
+        const uint64_t v = (uint64_t)pow_m(d, p - 2, p) * pow_m(2, ps.np == 5 ? 96 : 160, p) % p;
         scale[i] = (uint32_t)((v << 32) % p);
     }
 }
 
 // Launch constants of each set and length, made once at upload.
-WideCrt g_crt[2];
-uint32_t g_scale[kWideMaxLogN + 1][kWidePrimes];
+WideCrt g_crt[kNumSets - kFirstWideSet];
+uint32_t g_scale[kNumSets - kFirstWideSet][kWideMaxLogN + 1][kWideMaxPrimes];
 
 }  // namespace
 
 cudaError_t upload_wide_consts(int set, const NttConsts& c) {
-    g_crt[set - 2] = make_crt(c);
-    for (int ln = kWideMinLogN; ln <= kWideMaxLogN; ++ln)
-        if (wide_set_for(ln) == set) set_scale(c, ln, g_scale[ln]);
-    return cudaMemcpyToSymbol(c_wide, &c, sizeof(NttConsts), (set - 2) * sizeof(NttConsts));
+    const int w = set - kFirstWideSet;
+    const PrimeSetInfo& ps = kPrimeSets[set];
+    g_crt[w] = make_crt(ps);
+    for (int ln = kWideMinLogN; ln <= ps.log_max; ++ln) set_scale(ps, ln, g_scale[w][ln]);
+    return cudaMemcpyToSymbol(c_wide, &c, sizeof(NttConsts), w * sizeof(NttConsts));
 }
 
 // Built-in column lengths, the fastest measured on B200 for one product and
@@ -808,19 +894,51 @@ TransformShape wide_shape(int log_n, bool batch) {
 
 const char* const kWideKernelNames[kNttLaunches] = {"k_wide_fwd", "k_wide_rows", "k_wide_inv", "k_wide_carry"};
 
-cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs, const ProductDesc& one,
-                                uint32_t count, bool square, int log_n, int out_fmt, uint32_t bpp,
-                                const CarryLaunch& cl, cudaStream_t st, cudaEvent_t* ev) {
+// Longest transform over np primes.
+static int wide_max_log(int np) { return kPrimeSets[kFirstWideSet + 2 * (np - kWidePrimes) + 1].log_max; }
+
+// The shortest transform that holds the product, over the fewest primes that
+// reach it: at the same length six primes cost 1.25 times as much as five and
+// seven 1.4 (1.4 and 1.6 where only they need the strict set), twice the points
+// of five 1.8 to 2.  us per product at the longest operands of each form:
+// 2^18 points over six 36, over seven 40, 2^19 over five 48; 2^19 over six 60, over seven 71,
+// 2^20 over five 88; 2^22 over six 488, over seven 561, 2^23 over five 755.
+// Below 2^16 points the launches' latencies count and the three-word digits
+// load and reduce more slowly: 2^13 points over six 13.6, 2^14 over five 11.8; 2^15
+// over six 16.6, 2^16 over five 16.4; 2^16 over six 19.0, over seven 19.4, 2^17 over five 21.3.
+constexpr int kLongDigitMinLogN = 16;
+
+WideForm wide_form(uint32_t nd32a, uint32_t nd32b) {
+    WideForm best;
+    for (int np = kWidePrimes; np <= kWideMaxPrimes; ++np) {
+        const uint64_t points = (uint64_t)wide_digits(np, nd32a) + wide_digits(np, nd32b) - 1;
+        int ln = kWideMinLogN - 1;
+        while (ln <= kWideMaxLogN && ((uint64_t)1 << ln) < points) ++ln;
+        if (ln < (np == kWidePrimes ? kWideMinLogN : kLongDigitMinLogN) || ln > wide_max_log(np)) continue;
+        if (!best.np || ln < best.log_n) best = {np, ln};
+    }
+    return best;
+}
+
+cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const ProductDesc& one, uint32_t count,
+                                bool square, int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st,
+                                cudaEvent_t* ev) {
+    const int log_n = f.log_n;
+    if (f.np < kWidePrimes || f.np > kWideMaxPrimes || log_n > wide_max_log(f.np) || count < 1)
+        return cudaErrorInvalidValue;
     const int l2 = wide_shape(log_n, descs != nullptr).log_n2;
-    if (!l2 || log_n > host.log_max || count < 1) return cudaErrorInvalidValue;
-    const bool lazy = host.log_max == kPrimeSets[2].log_max;
+    if (!l2) return cudaErrorInvalidValue;
+    const int w = wide_set_for(f.np, log_n) - kFirstWideSet;
+    const bool lazy = w % 2 == 0;
     WideArgs a{};
     a.descs = descs;
     a.one = one;
     a.nops = square ? 1 : 2;
     a.log_n = log_n;
     a.log_n1 = log_n - l2;
-    std::memcpy(a.scale, g_scale[log_n], sizeof(a.scale));
+    a.np = f.np;
+    a.set = w;
+    std::memcpy(a.scale, g_scale[w][log_n], sizeof(a.scale));
     if (ev) cudaEventRecord(ev[0], st);
     cudaError_t e = lazy ? dispatch_cols<true>(l2, true, a, count, st) : dispatch_cols<false>(l2, true, a, count, st);
     if (e != cudaSuccess) return e;
@@ -834,7 +952,7 @@ cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs,
     WideCarryArgs ca{};
     ca.descs = descs;
     ca.one = one;
-    ca.crt = g_crt[lazy ? 0 : 1];
+    ca.crt = g_crt[w];
     ca.log_n = log_n;
     ca.out_fmt = out_fmt;
     ca.bpp = bpp;
@@ -842,21 +960,23 @@ cudaError_t launch_wide_product(const NttConsts& host, const ProductDesc* descs,
     ca.ticket_base = cl.ticket_base;
     ca.epoch = cl.epoch;
     ca.err = cl.err;
-    e = launch_k(lazy ? k_wide_carry<true> : k_wide_carry<false>, dim3(bpp * count), dim3(kWideCarryChunks + 32), 0, st,
-                 ca);
+    auto k = f.np == 5   ? (lazy ? k_wide_carry<true, 5> : k_wide_carry<false, 5>)
+             : f.np == 6 ? (lazy ? k_wide_carry<true, 6> : k_wide_carry<false, 6>)
+                         : (lazy ? k_wide_carry<true, 7> : k_wide_carry<false, 7>);
+    e = launch_k(k, dim3(bpp * count), dim3(kWideCarryChunks + 32), 0, st, ca);
     if (ev) cudaEventRecord(ev[4], st);
     return e;
 }
 
-cudaError_t launch_wide_batch(const NttConsts& host, const ProductDesc* descs, uint32_t count, bool square, int log_n,
-                              int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st) {
+cudaError_t launch_wide_batch(WideForm f, const ProductDesc* descs, uint32_t count, bool square, int out_fmt,
+                              uint32_t bpp, const CarryLaunch& cl, cudaStream_t st) {
     constexpr uint32_t kPiece = 16384;  // grid z limit 65535, two operands a product
     for (uint32_t done = 0; done < count; done += kPiece) {
         CarryLaunch piece = cl;
         piece.ticket_base = cl.ticket_base + (uint64_t)done * bpp;
         const uint32_t n = count - done < kPiece ? count - done : kPiece;
-        const cudaError_t e = launch_wide_product(host, descs + done, ProductDesc{}, n, square, log_n, out_fmt, bpp,
-                                                  piece, st, nullptr);
+        const cudaError_t e = launch_wide_product(f, descs + done, ProductDesc{}, n, square, out_fmt, bpp, piece, st,
+                                                  nullptr);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

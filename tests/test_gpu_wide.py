@@ -1,5 +1,5 @@
-"""Five-prime products (64-bit digits) at the edges of their dispatch: lengths
-around powers of two, operands longer than half the transform, long runs of
+"""Wide-digit products (64-, 80- and 96-bit digits) at the edges of their
+dispatch: lengths around the longest product of each transform, operands longer than half the transform, long runs of
 propagating carries, unaligned buffers, 28-bit Digits, both prime sets."""
 from __future__ import annotations
 
@@ -47,7 +47,22 @@ def test_length_edges(bb, port, log_n, extra):
     assert np.array_equal(bb.ntt_mul(a), port.mul(a, a))
 
 
-@pytest.mark.parametrize("n", [1500, 70000])
+# the same around the longest products of 2^k 80-bit digits (5/4 2^k limbs) and
+# 96-bit digits (6/4 2^k limbs), with the digits' odd half words and last partial digit
+@pytest.mark.parametrize("quarters", [5, 6])
+@pytest.mark.parametrize("log_n", [15, 16, 17, 18, 19])
+def test_digit_width_edges(bb, port, quarters, log_n):
+    rng = np.random.default_rng([SEED, quarters, log_n])
+    for extra in (-1, 0, 1):
+        total = (quarters << (log_n - 2)) + extra
+        for na in (total // 2, total - 5, total - total // 3):
+            a, b = rand_limbs(rng, na), rand_limbs(rng, total - na)
+            assert np.array_equal(bb.ntt_mul(a, b), port.mul(a, b)), (na, total - na)
+        a = rand_limbs(rng, total // 2)
+        assert np.array_equal(bb.ntt_mul(a), port.mul(a, a))
+
+
+@pytest.mark.parametrize("n", [600, 750, 1500, 70000, 80000])
 def test_propagating_carries(bb, port, n):
     """Products whose chunks all propagate a carry or stop it only at the ends."""
     ones = np.full(n, ONES)
@@ -80,7 +95,8 @@ def test_unaligned_device_buffers(bb, port):
     assert got[0] == ONES and got[-1] == ONES  # nothing written outside the product
 
 
-@pytest.mark.parametrize("na,nb", [(2500, 2300), (40000, 37450), (150000, 20000), (131073, 131071)])
+@pytest.mark.parametrize("na,nb", [(2500, 2300), (40000, 37450), (150000, 20000), (131073, 131071),
+                                   (2900, 2900), (3500, 3500), (330000, 310000), (400000, 380000)])
 def test_digits28(bb, port, na, nb):
     rng = np.random.default_rng([SEED, na])
     a = rng.integers(0, 1 << 28, na).astype(np.uint32)
@@ -97,6 +113,17 @@ def test_large_residue(bb, log_n):
     """The longest lazy transform and the shorter strict ones, modulo 2^61 - 1."""
     rng = np.random.default_rng([SEED, log_n, 61])
     total = 1 << log_n
+    for na in (total // 2, total - total // 4 + 3):
+        a, b = rand_limbs(rng, na), np.full(total - na, ONES)
+        c = bb.ntt_mul(a, b)
+        assert mod61(c) == mod61(a) * mod61(b) % M61, (na, total - na)
+
+
+@pytest.mark.parametrize("quarters,log_n", [(5, 20), (5, 21), (6, 19), (6, 22)])
+def test_large_width_residue(bb, quarters, log_n):
+    """80- and 96-bit digits on the longest lazy and on strict transforms."""
+    rng = np.random.default_rng([SEED, quarters, log_n])
+    total = quarters << (log_n - 2)
     for na in (total // 2, total - total // 4 + 3):
         a, b = rand_limbs(rng, na), np.full(total - na, ONES)
         c = bb.ntt_mul(a, b)
