@@ -35,10 +35,16 @@ namespace bgpu {
 // on graph branches).  Shorter ones do when they cannot share the mixed-length
 // launches, which are one launch per pass for any number of lengths.
 constexpr int kBatchWideLog32 = 14;
+// Products of a five-prime class that 80- or 96-bit digits hold in half the
+// points run there, on branches of their own, when they have this many points
+// together (4096 products of 2^10..2^22 bits 6.41 -> 5.46 ms, 64 of 2^14..2^22
+// bits 150 us; a line at 2^13 points 5.46 ms and 154 us, at 2^20 5.49 ms and
+// 166 us); fewer leave the GPU idle while their four launches pass.
+constexpr uint64_t kBatchSplitPoints = 1u << 16;
 
 struct BatchClass {
     int log_n = 0;      // 32-bit digits
-    bool wide = false;  // five-prime kernels, 2^(log_n - 1) points
+    WideForm form;      // wide-digit transform; np == 0: three primes
     bool square = false;
     uint32_t bpp = 0;   // carry blocks per product
     std::vector<uint32_t> members;  // product indices
@@ -79,10 +85,44 @@ int ceil_log2(uint64_t x) {
     return l;
 }
 
-size_t ntt_scratch_bytes(int log_n, bool square, bool wide) {
+size_t ntt_scratch_bytes(int log_n, bool square, WideForm f) {
+    if (f.np) return al256((square ? 1 : 2) * (size_t)f.np * ((size_t)4 << f.log_n));
     const size_t nn = (size_t)1 << log_n;
-    if (wide) return al256((square ? 1 : 2) * (size_t)kWidePrimes * (nn / 2) * 4);
     return al256((square ? 1 : 2) * (size_t)kNumPrimes * nn * 4) + al256(nn / 2 * 8) + al256(nn / 8 * 8);
+}
+
+// The wide-digit transforms of the classes outside the mixed-length launches.
+void split_wide_classes(bgpu_batch_plan_s* p, const bgpu_product* prods) {
+    std::vector<BatchClass> all;
+    size_t first_mixed = 0;
+    for (size_t i = 0; i < p->classes.size(); ++i) {
+        BatchClass& c = p->classes[i];
+        if (i == p->first_mixed) first_mixed = all.size();
+        if ((i < p->first_mixed || !p->mixed) && c.log_n > kWideMinLogN && c.log_n - 1 <= kWideMaxLogN) {
+            BatchClass part[kWideMaxPrimes + 1];
+            for (uint32_t m : c.members) {
+                const WideForm f = wide_form((uint32_t)(2 * prods[m].na), (uint32_t)(2 * prods[m].nb), kWideMinLogN);
+                part[f.log_n == c.log_n - 2 ? f.np : kWidePrimes].members.push_back(m);
+            }
+            auto& rest = part[kWidePrimes].members;
+            for (int np = kWideMaxPrimes; np >= kWidePrimes; --np) {
+                BatchClass& x = part[np];
+                x.log_n = c.log_n;
+                x.square = c.square;
+                x.form = {np, np == kWidePrimes ? c.log_n - 1 : c.log_n - 2};
+                if (np > kWidePrimes && ((uint64_t)x.members.size() << x.form.log_n) < kBatchSplitPoints) {
+                    rest.insert(rest.end(), x.members.begin(), x.members.end());
+                    x.members.clear();
+                }
+                if (!x.members.empty()) all.push_back(std::move(x));
+            }
+        } else {
+            all.push_back(std::move(c));
+        }
+    }
+    if (p->first_mixed >= p->classes.size()) first_mixed = all.size();
+    p->classes = std::move(all);
+    p->first_mixed = first_mixed;
 }
 
 void destroy_plan(bgpu_batch_plan_s* p) {
@@ -150,7 +190,7 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
         cl.epoch = 1;
         cl.ticket = tickets + ci;
         cl.err = hooks.err;
-        e = c.wide ? launch_wide_batch({kWidePrimes, c.log_n - 1}, d_descs + c.desc_off, (uint32_t)c.members.size(),
+        e = c.form.np ? launch_wide_batch(c.form, d_descs + c.desc_off, (uint32_t)c.members.size(),
                                        c.square, kFmtLimb64, c.bpp, cl, branches[ci])
                    : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], d_descs + c.desc_off,
                                       (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci]);
@@ -239,14 +279,15 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
     p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && nshort >= 2 && nshort <= (size_t)kMaxMixedClasses;
     for (size_t i = p->first_mixed; i < p->classes.size(); ++i)
         p->mixed = p->mixed && mixed_class_ok(p->classes[i].log_n, p->classes[i].square);
+    split_wide_classes(p, prods);
     // Layout: [ProductDesc...][MixedClass...][SchoolDesc: schoolbook...]
     //         [SchoolDesc: Karatsuba...][tickets][flags][scratch].
     size_t n_desc = 0, flag_words = 0, scratch = 0;
     for (size_t i = 0; i < p->classes.size(); ++i) {
         BatchClass& c = p->classes[i];
-        c.wide = (i < p->first_mixed || !p->mixed) && c.log_n > kWideMinLogN && c.log_n - 1 <= kWideMaxLogN;
-        if (c.wide) {
-            for (uint32_t m : c.members) c.bpp = std::max(c.bpp, wide_carry_blocks(kWidePrimes, prods[m].na + prods[m].nb, kFmtLimb64));
+        if (c.form.np) {
+            for (uint32_t m : c.members)
+                c.bpp = std::max(c.bpp, wide_carry_blocks(c.form.np, prods[m].na + prods[m].nb, kFmtLimb64));
         } else {
             c.bpp = carry_blocks((uint32_t)(((size_t)1 << c.log_n) / 8));
         }
@@ -256,7 +297,7 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
         c.flags_words = c.members.size() * c.bpp;
         flag_words += c.flags_words;
         c.scratch_off = scratch;
-        scratch += c.members.size() * ntt_scratch_bytes(c.log_n, c.square, c.wide);
+        scratch += c.members.size() * ntt_scratch_bytes(c.log_n, c.square, c.form);
     }
     const size_t nmixed = p->mixed ? nshort : 0;
     const size_t mixed_off = al256(n_desc * sizeof(ProductDesc));
@@ -275,7 +316,7 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
     std::vector<ProductDesc> descs(n_desc);
     for (auto& c : p->classes) {
         const size_t nn = (size_t)1 << c.log_n;
-        const size_t per = ntt_scratch_bytes(c.log_n, c.square, c.wide);
+        const size_t per = ntt_scratch_bytes(c.log_n, c.square, c.form);
         const size_t y_bytes = al256((c.square ? 1 : 2) * (size_t)kNumPrimes * nn * 4);
         for (size_t m = 0; m < c.members.size(); ++m) {
             const bgpu_product& q = prods[c.members[m]];
@@ -284,8 +325,8 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
             d.op[0] = OperandDesc{q.a, (uint32_t)q.na, (uint32_t)(2 * q.na), kFmtLimb64};
             d.op[1] = c.square ? d.op[0] : OperandDesc{q.b, (uint32_t)q.nb, (uint32_t)(2 * q.nb), kFmtLimb64};
             d.y = reinterpret_cast<uint32_t*>(sc);
-            d.chunks = c.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes);
-            d.spill = c.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
+            d.chunks = c.form.np ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes);
+            d.spill = c.form.np ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
             d.flags = reinterpret_cast<uint64_t*>(base + flags_base) + c.flags_off + m * c.bpp;
             d.out = q.out;
             d.out_cap = q.na + q.nb;
@@ -430,7 +471,7 @@ struct TreeLevel {
     size_t w;
     int kind;  // 0: thread per product (w <= 4), 1: schoolbook, 2: Karatsuba, 3: NTT
     int log_n = 0;        // kind 3: 32-bit digits
-    bool wide = false;    // kind 3: five-prime kernels, 2^(log_n - 1) points
+    WideForm form;        // kind 3: wide-digit transform; np == 0: three primes
     uint32_t bpp = 0;     // kind 3: carry blocks per product
     size_t desc_off = 0;  // bytes into the descriptor region
 };
@@ -463,10 +504,10 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
             L.kind = 3;
             while (((uint64_t)1 << L.log_n) < 4 * (uint64_t)w - 1) ++L.log_n;
             if (!shape_supported_batch(L.log_n, false)) return BGPU_ERR_CAPACITY;
-            L.wide = L.log_n > kWideMinLogN && L.log_n - 1 <= kWideMaxLogN;
-            L.bpp = L.wide ? wide_carry_blocks(kWidePrimes, 2 * w, kFmtLimb64)
+            if (L.log_n > kWideMinLogN && L.log_n - 1 <= kWideMaxLogN) L.form = {kWidePrimes, L.log_n - 1};
+            L.bpp = L.form.np ? wide_carry_blocks(kWidePrimes, 2 * w, kFmtLimb64)
                            : carry_blocks((uint32_t)(((size_t)1 << L.log_n) / 8));
-            ntt_bytes = std::max(ntt_bytes, (size_t)L.m2 * ntt_scratch_bytes(L.log_n, false, L.wide));
+            ntt_bytes = std::max(ntt_bytes, (size_t)L.m2 * ntt_scratch_bytes(L.log_n, false, L.form));
             flag_words = std::max(flag_words, (size_t)L.m2 * L.bpp);
         }
         if (L.kind == 1 || L.kind == 2) {
@@ -518,7 +559,7 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
             } else if (L.kind == 3) {
                 ProductDesc* pd = reinterpret_cast<ProductDesc*>(hd.data() + L.desc_off);
                 const size_t nn = (size_t)1 << L.log_n;
-                const size_t per = ntt_scratch_bytes(L.log_n, false, L.wide);
+                const size_t per = ntt_scratch_bytes(L.log_n, false, L.form);
                 const uint32_t bpp = L.bpp;
                 const size_t y_bytes = al256(2 * (size_t)kNumPrimes * nn * 4);
                 for (uint32_t i = 0; i < L.m2; ++i) {
@@ -527,8 +568,8 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
                     d.op[0] = OperandDesc{in + (size_t)2 * i * w, (uint32_t)w, (uint32_t)(2 * w), kFmtLimb64};
                     d.op[1] = OperandDesc{in + (size_t)(2 * i + 1) * w, (uint32_t)w, (uint32_t)(2 * w), kFmtLimb64};
                     d.y = reinterpret_cast<uint32_t*>(sc);
-                    d.chunks = L.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes);
-                    d.spill = L.wide ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
+                    d.chunks = L.form.np ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes);
+                    d.spill = L.form.np ? nullptr : reinterpret_cast<uint64_t*>(sc + y_bytes + al256(nn / 2 * 8));
                     d.flags = flags + (size_t)i * bpp;
                     d.out = out + (size_t)2 * i * w;
                     d.out_cap = 2 * w;
@@ -570,7 +611,7 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
                 cl.err = hooks.err;
                 const int ps = prime_set_for(L.log_n);
                 const ProductDesc* pd = reinterpret_cast<const ProductDesc*>(base + off_desc + L.desc_off);
-                e = L.wide ? launch_wide_batch({kWidePrimes, L.log_n - 1}, pd, L.m2, false, kFmtLimb64, L.bpp, cl, st)
+                e = L.form.np ? launch_wide_batch(L.form, pd, L.m2, false, kFmtLimb64, L.bpp, cl, st)
                            : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], pd, (int)L.m2, false, L.log_n,
                                               kFmtLimb64, cl, st);
             }

@@ -21,12 +21,19 @@ __host__ __device__ constexpr uint32_t wide_digits(int np, uint32_t nd32) {
 
 constexpr int kWideMaxPrimes = 7;
 
+// A single product takes more than five primes from here: below 2^16 points the
+// launches' latencies count and the three-word digits load and reduce more
+// slowly: us per product, 2^13 points over six primes 13.6, 2^14 over five 11.8;
+// 2^15 over six 16.6, 2^16 over five 16.4; 2^16 over six 19.0, over seven 19.4, 2^17 over five 21.3.
+constexpr int kLongDigitMinLogN = 16;
+
 // Transform of a product: 2^log_n points over np primes (np == 0: none).
 struct WideForm {
     int np = 0, log_n = 0;
 };
-// The form of least work for operands of nd32a and nd32b 32-bit digits.
-WideForm wide_form(uint32_t nd32a, uint32_t nd32b);
+// The form of least work for operands of nd32a and nd32b 32-bit digits; more
+// than five primes from 2^min_long points.
+WideForm wide_form(uint32_t nd32a, uint32_t nd32b, int min_long);
 
 // Shortest transform: below it (1024 limbs of product) the three-prime
 // kernels, whose few blocks are as fast.

@@ -903,18 +903,13 @@ static int wide_max_log(int np) { return kPrimeSets[kFirstWideSet + 2 * (np - kW
 // of five 1.8 to 2.  us per product at the longest operands of each form:
 // 2^18 points over six 36, over seven 40, 2^19 over five 48; 2^19 over six 60, over seven 71,
 // 2^20 over five 88; 2^22 over six 488, over seven 561, 2^23 over five 755.
-// Below 2^16 points the launches' latencies count and the three-word digits
-// load and reduce more slowly: 2^13 points over six 13.6, 2^14 over five 11.8; 2^15
-// over six 16.6, 2^16 over five 16.4; 2^16 over six 19.0, over seven 19.4, 2^17 over five 21.3.
-constexpr int kLongDigitMinLogN = 16;
-
-WideForm wide_form(uint32_t nd32a, uint32_t nd32b) {
+WideForm wide_form(uint32_t nd32a, uint32_t nd32b, int min_long) {
     WideForm best;
     for (int np = kWidePrimes; np <= kWideMaxPrimes; ++np) {
         const uint64_t points = (uint64_t)wide_digits(np, nd32a) + wide_digits(np, nd32b) - 1;
         int ln = kWideMinLogN - 1;
         while (ln <= kWideMaxLogN && ((uint64_t)1 << ln) < points) ++ln;
-        if (ln < (np == kWidePrimes ? kWideMinLogN : kLongDigitMinLogN) || ln > wide_max_log(np)) continue;
+        if (ln < (np == kWidePrimes ? kWideMinLogN : min_long) || ln > wide_max_log(np)) continue;
         if (!best.np || ln < best.log_n) best = {np, ln};
     }
     return best;

@@ -159,6 +159,7 @@ def _run_batch(bb, port, sizes, squares=(), flags=0):
 @pytest.mark.parametrize("sizes,squares", [
     ([(700, 600), (1100, 90), (1023, 2)], ()),
     ([(4097, 4097), (8000, 9), (5000, 7000), (300, 400), (1000, 900), (60, 70)], (2,)),
+    ([(5000, 5240), (6000, 6288), (6100, 6100), (4097, 4097)] * 4, (1, 6)),  # 80- and 96-bit digits, the longest ones
     ([(16384, 16385), (16385, 16385), (40000, 30), (33000, 700)], (1,)),
 ])
 @pytest.mark.parametrize("per_class", [False, True])
