@@ -262,13 +262,59 @@ int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, WideF
         ++g.kev_count;
         g.timed_wide = true;
     }
-    const cudaError_t e = launch_wide_product(f, nullptr, one, 1, square, out_fmt, bpp, cl, st, ev);
+    const cudaError_t e = launch_wide_product(f, nullptr, one, WideStep{}, 1, square, out_fmt, bpp, cl, st, ev);
     g.last_launches = kNttLaunches;
     if (stats) {
         stats->method = BGPU_METHOD_NTT;
         stats->log2_points = (uint32_t)std::max(5, ceil_log2((uint64_t)a.nd32 + b.nd32 - 1));
     }
     return cuda_status(e);
+}
+
+// Points of the equally spaced products one set of launches takes together:
+// the GPU is full well below, and the residues (40 to 56 bytes a point) stay
+// in the L2 cache.
+constexpr uint64_t kWideGroupPoints = 1u << 21;
+
+// `count` products of na x nb limbs, pr[i] being pr[0] moved by i equal steps,
+// as one set of four launches for each group.
+int multiply_wide_many(WideForm f, const bgpu_product* pr, size_t count, cudaStream_t st, uint32_t* launches) {
+    const size_t na = pr[0].na, nb = pr[0].nb;
+    const uint32_t bpp = wide_carry_blocks(f.np, na + nb, kFmtLimb64);
+    const size_t y_bytes = 2 * (size_t)f.np * ((size_t)4 << f.log_n), fl_bytes = (size_t)bpp * 8;
+    const size_t group = std::min<size_t>(
+        {count, kWidePiece, std::max<uint64_t>(1, kWideGroupPoints >> f.log_n)});
+    int rc = ensure(&g.d_scratch, &g.scratch_bytes, group * y_bytes + align256(group * fl_bytes));
+    if (rc != BGPU_OK) return rc;
+    auto apart = [&](const void* x, const void* y) { return static_cast<const char*>(x) - static_cast<const char*>(y); };
+    WideStep step;
+    if (count > 1) {
+        step.a = apart(pr[1].a, pr[0].a);
+        step.b = apart(pr[1].b, pr[0].b);
+        step.out = apart(pr[1].out, pr[0].out);
+    }
+    for (size_t done = 0; done < count; done += group) {
+        const uint32_t n = (uint32_t)std::min(group, count - done);
+        ProductDesc one{};
+        one.op[0] = OperandDesc{pr[done].a, (uint32_t)na, (uint32_t)(2 * na), kFmtLimb64};
+        one.op[1] = OperandDesc{pr[done].b, (uint32_t)nb, (uint32_t)(2 * nb), kFmtLimb64};
+        one.y = static_cast<uint32_t*>(g.d_scratch);
+        one.flags = reinterpret_cast<uint64_t*>(static_cast<char*>(g.d_scratch) + group * y_bytes);
+        one.out = pr[done].out;
+        one.out_cap = na + nb;
+        CarryLaunch cl;
+        cl.ticket_base = g.ticket_base;
+        cl.epoch = ++g.epoch;
+        cl.ticket = g.d_ticket;
+        cl.err = g.d_err;
+        g.ticket_base += (uint64_t)n * bpp;
+        g.ntt_log_n = -1;
+        const cudaError_t e =
+            launch_wide_product(f, nullptr, one, step, n, false, kFmtLimb64, bpp, cl, st, nullptr);
+        if (e != cudaSuccess) return cuda_status(e);
+        *launches += kNttLaunches;
+    }
+    return BGPU_OK;
 }
 
 // Core: product of two device operands into a device output (async).
@@ -1993,10 +2039,12 @@ static int ensure_powers(int J, bool with_v, cudaStream_t st, uint32_t* nl) {
     return rc;
 }
 
-// A batch of equal-size device products on `st` (the levels of the decimal
-// conversions): schoolbook or Karatsuba classes as one launch over a
-// descriptor array, up to 128 transform-size products as direct launches,
-// more through a batch plan.
+// A batch of equal-size, equally spaced device products on `st` (the levels of
+// the decimal conversions): schoolbook or Karatsuba classes as one launch over
+// a descriptor array, wide-digit transforms as one set of launches a group
+// (one product at a time a level of 64 products of 2^10 points took 10 us a product),
+// shorter transforms as direct launches up to 128 and through a batch plan
+// beyond.
 static int run_products(const bgpu_product* pr, size_t count, cudaStream_t st, uint32_t* launches) {
     if (count == 0) return BGPU_OK;
     const size_t na = pr[0].na, nb = pr[0].nb;
@@ -2015,6 +2063,10 @@ static int run_products(const bgpu_product* pr, size_t count, cudaStream_t st, u
             e = school ? launch_schoolbook_batch(dd, (uint32_t)count, st) : launch_karatsuba_batch(dd, (uint32_t)count, st);
         *launches += 1;
         return cuda_status(e);
+    }
+    if (count > 1) {
+        const WideForm f = wide_form((uint32_t)(2 * na), (uint32_t)(2 * nb), kWideMinLogN);
+        if (f.np) return multiply_wide_many(f, pr, count, st, launches);
     }
     if (count <= 128) {
         for (size_t i = 0; i < count; ++i) {

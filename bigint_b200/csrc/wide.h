@@ -39,12 +39,35 @@ WideForm wide_form(uint32_t nd32a, uint32_t nd32b, int min_long);
 // kernels, whose few blocks are as fast.
 constexpr int kWideMinLogN = 10;
 
-struct WideArgs {
-    const ProductDesc* descs;  // y: (square ? 1 : 2) * np planes of N residues (the result replaces A's)
-    ProductDesc one;
+// Products of one set of launches: descs, or one product moved by equal steps
+// (bytes; planes and flags follow one another).  Launch arguments are kept
+// short, the constants are in constant memory: the host's launches bound small
+// products (2^11 points 14.8 us a call, with the CRT's constants and a full
+// description of each product in the arguments 15.5).
+struct WideArgs {              // column and row passes
+    const ProductDesc* descs;  // y: nops * np planes of N residues (the result replaces A's)
+    uint32_t* y;
     int nops, log_n, log_n1, np;
-    int set;                         // of the wide sets
-    uint32_t scale[kWideMaxPrimes];  // row pass, Montgomery form
+    int set;  // of the wide sets
+};
+struct WideFwdArgs {
+    WideArgs w;
+    OperandDesc op[2];
+    int64_t step_a, step_b;
+};
+
+struct WideCarryArgs {
+    const ProductDesc* descs;  // y, flags, out, out_cap
+    uint32_t* y;
+    uint64_t* flags;
+    void* out;
+    size_t out_cap;
+    int64_t step_out;
+    unsigned long long* ticket;
+    uint64_t ticket_base, epoch;
+    uint32_t* err;
+    int nops, log_n, out_fmt;
+    uint32_t bpp;  // blocks per product
 };
 
 // CRT of residues y_i = x (M/p_i)^-1 mod p_i: x = sum y_i M/p_i - q M, q < np.
@@ -55,15 +78,8 @@ struct WideCrt {
     float bias;                                      // 0.05 - 2^23 sum inv
 };
 
-struct WideCarryArgs {
-    const ProductDesc* descs;  // y, flags, out, out_cap
-    ProductDesc one;
-    WideCrt crt;
-    int log_n, out_fmt;
-    uint32_t bpp;  // blocks per product
-    unsigned long long* ticket;
-    uint64_t ticket_base, epoch;
-    uint32_t* err;
+struct WideStep {
+    int64_t a = 0, b = 0, out = 0;
 };
 
 constexpr uint32_t kWideCarryChunks = 256;  // chunks of four digits (np - 1 limbs) per carry block
@@ -83,8 +99,9 @@ extern const char* const kWideKernelNames[kNttLaunches];
 
 // The four launches of `count` products of one form (digits of both operands
 // together at most 2^log_n + 1); each product's carry scan has `bpp` blocks
-// (tickets).
-cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const ProductDesc& one,
+// (tickets).  At most kWidePiece products.
+constexpr uint32_t kWidePiece = 16384;  // grid z limit 65535, two operands a product
+cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const ProductDesc& one, const WideStep& step,
                                 uint32_t count, bool square, int out_fmt, uint32_t bpp,
                                 const CarryLaunch& cl, cudaStream_t st, cudaEvent_t* ev);
 

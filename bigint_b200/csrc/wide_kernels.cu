@@ -50,12 +50,16 @@ __host__ __device__ constexpr uint32_t wide_row_words(int l1, bool square) {
     return ((square || wide_one_buffer(l1) ? 1u : 2u) << l1) + 32u + (l1 >= 10 ? 0u : (uint32_t)wide_row_threads(l1) % 32u);
 }
 
-__constant__ NttConsts c_wide[kNumSets - kFirstWideSet];  // lazy and strict of five, six and seven primes
-
+// lazy and strict sets of five, six and seven primes
+constexpr int kWideSets = kNumSets - kFirstWideSet;
+__constant__ NttConsts c_wide[kWideSets];
+__constant__ WideCrt c_crt[kWideSets];
+__constant__ uint32_t c_scale[kWideSets][kWideMaxLogN + 1][kWideMaxPrimes];  // row pass, Montgomery form
 __host__ __device__ constexpr int wide_set_index(int np, bool lazy) { return 2 * (np - kWidePrimes) + (lazy ? 0 : 1); }
 
-__device__ __forceinline__ ProductDesc wide_product(const WideArgs& a, uint32_t i) {
-    return a.descs ? a.descs[i] : a.one;
+// Planes of product i.
+__device__ __forceinline__ uint32_t* wide_planes(const WideArgs& a, uint32_t i) {
+    return a.descs ? a.descs[i].y : a.y + (((size_t)i * (uint32_t)(a.nops * a.np)) << a.log_n);
 }
 
 // (hi 2^32 + lo + k p) / 2^32 with the k that clears the low word: one wide
@@ -195,20 +199,27 @@ __host__ __device__ constexpr int wide_col_blocks(int l2, bool fwd) {
 }
 
 template <bool LAZY, int L2, int T, int NP>
-__global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const WideArgs a) {
+__global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const WideFwdArgs fa) {
+    const WideArgs& a = fa.w;
     using P2 = Plan<L2>;
     constexpr int NR = P2::nr, RL = P2::r(NR - 1), SROW = (1 << RL) + 1;
     static_assert(NR > 1, "column passes of several rounds");
     extern __shared__ __align__(16) uint32_t sm[];  // [2^L2][8] and the column powers
     const NttConsts& c = c_wide[wide_set_index(NP, LAZY)];
     const int q = blockIdx.y, op = (int)(blockIdx.z % (uint32_t)a.nops);
-    const ProductDesc pd = wide_product(a, blockIdx.z / (uint32_t)a.nops);
+    const uint32_t product = blockIdx.z / (uint32_t)a.nops;
     const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
     const uint2* tw = c.stage[q][0];
-    const OperandDesc in = op == 0 ? pd.op[0] : pd.op[1];
+    OperandDesc in;
+    if (a.descs) {
+        in = a.descs[product].op[op];
+    } else {
+        in = op == 0 ? fa.op[0] : fa.op[1];
+        in.ptr = static_cast<const char*>(in.ptr) + (int64_t)product * (op == 0 ? fa.step_a : fa.step_b);
+    }
     const uint32_t c0 = blockIdx.x * kWideCols;
     const size_t nn = (size_t)1 << a.log_n;
-    uint32_t* y = pd.y + ((size_t)op * NP + q) * nn;
+    uint32_t* y = wide_planes(a, product) + ((size_t)op * NP + q) * nn;
 
     // The last round's groups hold slots base + j of one column n1, whose
     // inter-pass twiddle is omega_N^(n1 bitrev(base)) S^bitrev(j): sS[col][m]
@@ -265,7 +276,7 @@ __host__ __device__ constexpr int wide_row_blocks(int l1) {
 
 template <bool LAZY, int L1, bool SQR>
 __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1), wide_row_blocks(L1))
-    k_wide_rows(const __grid_constant__ WideArgs a) {
+    k_wide_rows(const WideArgs a) {
     constexpr int T = wide_row_threads(L1);
     constexpr bool MULTI = wide_rows_per_cta(L1) > 1;
     constexpr bool ONE = !SQR && wide_one_buffer(L1);
@@ -281,15 +292,14 @@ __global__ void __launch_bounds__(wide_row_threads(L1) * wide_rows_per_cta(L1), 
     uint2* sT = reinterpret_cast<uint2*>(sa + ((SQR || ONE ? 1u : 2u) << L1));
     const int q = blockIdx.y, tid = sub_tid<T, MULTI>();
     const uint32_t slot = blockIdx.x * wide_rows_per_cta(L1) + sub;
-    const ProductDesc pd = wide_product(a, blockIdx.z);
     const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
     const uint2* twf = c.stage[q][0];
     const uint2* twi = c.stage[q][1];
     const size_t nn = (size_t)1 << a.log_n;
-    uint32_t* row_a = pd.y + q * nn + ((size_t)slot << L1);
+    uint32_t* row_a = wide_planes(a, blockIdx.z) + q * nn + ((size_t)slot << L1);
     const uint32_t* row_b = row_a + a.np * nn;
     const uint32_t k2 = bitrev(slot, a.log_n - L1);
-    const uint32_t scale = a.scale[q];
+    const uint32_t scale = c_scale[a.set][a.log_n][q];
 
     // The last DIT round's groups hold n1 = base + (j << LO0): twiddle
     // omega_N^-(k2 base) sT[j], sT[j] = omega_N^-(k2 j << LO0).
@@ -378,7 +388,7 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, false)) k_wide_inv(cons
     const int q = blockIdx.y;
     const uint32_t p = c.pr[q].p;
     const uint2* twi = c.stage[q][1];
-    uint32_t* y = wide_product(a, blockIdx.z).y + ((size_t)q << a.log_n) + blockIdx.x * kWideCols;
+    uint32_t* y = wide_planes(a, blockIdx.z) + ((size_t)q << a.log_n) + blockIdx.x * kWideCols;
     pdl_wait();
     {
         using Gr = Group<L2, kWideCols, NR - 1>;
@@ -589,13 +599,14 @@ constexpr int kWideCarryWarps = kWideCarryChunks / 32;
 template <bool LAZY, int NP>
 __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __grid_constant__ WideCarryArgs a) {
     constexpr int NL = NP - 1;
+    const WideCrt& crt = c_crt[wide_set_index(NP, LAZY)];
     __shared__ uint32_t s_bid, s_cin, s_win_g, s_win_p;
     __shared__ uint32_t s_wg[kWideCarryWarps], s_wp[kWideCarryWarps];
     __shared__ uint64_t s_sp[kWideCarryWarps + 1][2];
     __shared__ uint64_t s_low[kWideCarryChunks];  // 28-bit output: each chunk's low limb before its spill and carry
     __shared__ uint32_t s_nqm[NP * NP];
     if (threadIdx.x == 0) s_bid = (uint32_t)(atomicAdd(a.ticket, 1ull) - a.ticket_base);
-    for (int i = threadIdx.x; i < NP * NP; i += kWideCarryChunks + 32) s_nqm[i] = a.crt.nqm[i / NP][i % NP];
+    for (int i = threadIdx.x; i < NP * NP; i += kWideCarryChunks + 32) s_nqm[i] = crt.nqm[i / NP][i % NP];
     __syncthreads();
     pdl_wait();
     pdl_trigger();
@@ -604,7 +615,16 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
         return;
     }
     const uint32_t bid = s_bid % a.bpp;
-    const ProductDesc pd = a.descs ? a.descs[s_bid / a.bpp] : a.one;
+    const uint32_t product = s_bid / a.bpp;
+    ProductDesc pd;
+    if (a.descs) {
+        pd = a.descs[product];
+    } else {
+        pd.y = a.y + (((size_t)product * (uint32_t)(a.nops * NP)) << a.log_n);
+        pd.flags = a.flags + (size_t)product * a.bpp;
+        pd.out = static_cast<char*>(a.out) + (int64_t)product * a.step_out;
+        pd.out_cap = a.out_cap;
+    }
     // a product of a batch shorter than its class's longest: no later block waits on these
     if (bid >= wide_carry_blocks(NP, pd.out_cap, a.out_fmt)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -613,7 +633,7 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
     const uint32_t nch = (uint32_t)(nn / 4);
     const int64_t c = (int64_t)bid * kWideCarryChunks + (window ? lane - 32 : (int)threadIdx.x);
     uint64_t S[NL] = {}, sp[2] = {0, 0};
-    if (c >= 0 && c < nch) chunk_sum<LAZY, NP>(a.crt, s_nqm, pd.y, nn, (size_t)c, S, sp);
+    if (c >= 0 && c < nch) chunk_sum<LAZY, NP>(crt, s_nqm, pd.y, nn, (size_t)c, S, sp);
     if (!window) s_low[threadIdx.x] = S[0];
     if (lane == 31) {
         s_sp[warp][0] = sp[0];
@@ -719,7 +739,7 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
             uint32_t r[NP], w[NP] = {};
 #pragma unroll
             for (int i = 0; i < NP; ++i) r[i] = pd.y[i * nn + 4 * (size_t)(c + 1)];
-            add_crt<LAZY, NP>(a.crt, s_nqm, r, w);
+            add_crt<LAZY, NP>(crt, s_nqm, r, w);
             next = w[0] | ((uint64_t)w[1] << 32);
         }
         next += sp[0] + (lane == 31 ? (uint32_t)(sum >> 32) & 1u : (carries >> (lane + 1)) & 1u);
@@ -732,20 +752,21 @@ __global__ void __launch_bounds__(kWideCarryChunks + 32) k_wide_carry(const __gr
 namespace {
 
 template <bool LAZY, int L2, int NP>
-cudaError_t launch_fwd(const WideArgs& a, uint32_t count, cudaStream_t st) {
+cudaError_t launch_fwd(const WideFwdArgs& fa, uint32_t count, cudaStream_t st) {
     constexpr int RL = Plan<L2>::r(Plan<L2>::nr - 1);
     const size_t sm = ((size_t)kWideCols * 4 << L2) + kWideCols * ((1 << RL) + 1) * sizeof(uint2);
     auto k = k_wide_fwd<LAZY, L2, wide_col_threads(L2, true), NP>;
     allow_smem(k, sm);
-    return launch_k(k, dim3((1u << a.log_n1) / kWideCols, NP, count * a.nops), dim3(wide_col_threads(L2, true)), sm, st,
-                    a);
+    return launch_k(k, dim3((1u << fa.w.log_n1) / kWideCols, NP, count * fa.w.nops), dim3(wide_col_threads(L2, true)), sm,
+                    st, fa);
 }
 template <bool LAZY, int L2>
-cudaError_t launch_cols(bool fwd, const WideArgs& a, uint32_t count, cudaStream_t st) {
+cudaError_t launch_cols(bool fwd, const WideFwdArgs& fa, uint32_t count, cudaStream_t st) {
+    const WideArgs& a = fa.w;
     if (fwd)
-        return a.np == 5   ? launch_fwd<LAZY, L2, 5>(a, count, st)
-               : a.np == 6 ? launch_fwd<LAZY, L2, 6>(a, count, st)
-                           : launch_fwd<LAZY, L2, 7>(a, count, st);
+        return a.np == 5   ? launch_fwd<LAZY, L2, 5>(fa, count, st)
+               : a.np == 6 ? launch_fwd<LAZY, L2, 6>(fa, count, st)
+                           : launch_fwd<LAZY, L2, 7>(fa, count, st);
     const size_t tile = (size_t)kWideCols * 4 << L2;
     auto k = k_wide_inv<LAZY, L2, wide_col_threads(L2, false)>;
     allow_smem(k, tile);
@@ -753,7 +774,7 @@ cudaError_t launch_cols(bool fwd, const WideArgs& a, uint32_t count, cudaStream_
 }
 
 template <bool LAZY>
-cudaError_t dispatch_cols(int l2, bool fwd, const WideArgs& a, uint32_t count, cudaStream_t st) {
+cudaError_t dispatch_cols(int l2, bool fwd, const WideFwdArgs& a, uint32_t count, cudaStream_t st) {
     switch (l2) {
         case 5: return launch_cols<LAZY, 5>(fwd, a, count, st);
         case 6: return launch_cols<LAZY, 6>(fwd, a, count, st);
@@ -855,18 +876,18 @@ void set_scale(const PrimeSetInfo& ps, int log_n, uint32_t* scale) {
     }
 }
 
-// Launch constants of each set and length, made once at upload.
-WideCrt g_crt[kNumSets - kFirstWideSet];
-uint32_t g_scale[kNumSets - kFirstWideSet][kWideMaxLogN + 1][kWideMaxPrimes];
-
 }  // namespace
 
 cudaError_t upload_wide_consts(int set, const NttConsts& c) {
     const int w = set - kFirstWideSet;
     const PrimeSetInfo& ps = kPrimeSets[set];
-    g_crt[w] = make_crt(ps);
-    for (int ln = kWideMinLogN; ln <= ps.log_max; ++ln) set_scale(ps, ln, g_scale[w][ln]);
-    return cudaMemcpyToSymbol(c_wide, &c, sizeof(NttConsts), w * sizeof(NttConsts));
+    const WideCrt crt = make_crt(ps);
+    uint32_t scale[kWideMaxLogN + 1][kWideMaxPrimes] = {};
+    for (int ln = kWideMinLogN; ln <= ps.log_max; ++ln) set_scale(ps, ln, scale[ln]);
+    cudaError_t e = cudaMemcpyToSymbol(c_crt, &crt, sizeof(crt), w * sizeof(crt));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_scale, scale, sizeof(scale), w * sizeof(scale));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_wide, &c, sizeof(NttConsts), w * sizeof(NttConsts));
+    return e;
 }
 
 // Built-in column lengths, the fastest measured on B200 for one product and
@@ -915,39 +936,47 @@ WideForm wide_form(uint32_t nd32a, uint32_t nd32b, int min_long) {
     return best;
 }
 
-cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const ProductDesc& one, uint32_t count,
-                                bool square, int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st,
+cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const ProductDesc& one, const WideStep& step,
+                                uint32_t count, bool square, int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st,
                                 cudaEvent_t* ev) {
     const int log_n = f.log_n;
-    if (f.np < kWidePrimes || f.np > kWideMaxPrimes || log_n > wide_max_log(f.np) || count < 1)
+    if (f.np < kWidePrimes || f.np > kWideMaxPrimes || log_n > wide_max_log(f.np) || count < 1 || count > kWidePiece)
         return cudaErrorInvalidValue;
-    const int l2 = wide_shape(log_n, descs != nullptr).log_n2;
+    const int l2 = wide_shape(log_n, descs != nullptr || count > 1).log_n2;
     if (!l2) return cudaErrorInvalidValue;
     const int w = wide_set_for(f.np, log_n) - kFirstWideSet;
     const bool lazy = w % 2 == 0;
-    WideArgs a{};
+    WideFwdArgs fa{};
+    WideArgs& a = fa.w;
     a.descs = descs;
-    a.one = one;
+    a.y = one.y;
     a.nops = square ? 1 : 2;
     a.log_n = log_n;
     a.log_n1 = log_n - l2;
     a.np = f.np;
     a.set = w;
-    std::memcpy(a.scale, g_scale[w][log_n], sizeof(a.scale));
+    fa.op[0] = one.op[0];
+    fa.op[1] = one.op[1];
+    fa.step_a = step.a;
+    fa.step_b = step.b;
     if (ev) cudaEventRecord(ev[0], st);
-    cudaError_t e = lazy ? dispatch_cols<true>(l2, true, a, count, st) : dispatch_cols<false>(l2, true, a, count, st);
+    cudaError_t e = lazy ? dispatch_cols<true>(l2, true, fa, count, st) : dispatch_cols<false>(l2, true, fa, count, st);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[1], st);
     e = lazy ? dispatch_rows<true>(a.log_n1, a, square, count, st) : dispatch_rows<false>(a.log_n1, a, square, count, st);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[2], st);
-    e = lazy ? dispatch_cols<true>(l2, false, a, count, st) : dispatch_cols<false>(l2, false, a, count, st);
+    e = lazy ? dispatch_cols<true>(l2, false, fa, count, st) : dispatch_cols<false>(l2, false, fa, count, st);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[3], st);
     WideCarryArgs ca{};
     ca.descs = descs;
-    ca.one = one;
-    ca.crt = g_crt[w];
+    ca.y = one.y;
+    ca.flags = one.flags;
+    ca.out = one.out;
+    ca.out_cap = one.out_cap;
+    ca.step_out = step.out;
+    ca.nops = a.nops;
     ca.log_n = log_n;
     ca.out_fmt = out_fmt;
     ca.bpp = bpp;
@@ -965,13 +994,12 @@ cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const Prod
 
 cudaError_t launch_wide_batch(WideForm f, const ProductDesc* descs, uint32_t count, bool square, int out_fmt,
                               uint32_t bpp, const CarryLaunch& cl, cudaStream_t st) {
-    constexpr uint32_t kPiece = 16384;  // grid z limit 65535, two operands a product
-    for (uint32_t done = 0; done < count; done += kPiece) {
+    for (uint32_t done = 0; done < count; done += kWidePiece) {
         CarryLaunch piece = cl;
         piece.ticket_base = cl.ticket_base + (uint64_t)done * bpp;
-        const uint32_t n = count - done < kPiece ? count - done : kPiece;
-        const cudaError_t e = launch_wide_product(f, descs + done, ProductDesc{}, n, square, out_fmt, bpp, piece, st,
-                                                  nullptr);
+        const uint32_t n = count - done < kWidePiece ? count - done : kWidePiece;
+        const cudaError_t e = launch_wide_product(f, descs + done, ProductDesc{}, WideStep{}, n, square, out_fmt,
+                                                  bpp, piece, st, nullptr);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

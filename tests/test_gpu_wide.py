@@ -166,3 +166,24 @@ def _run_batch(bb, port, sizes, squares=(), flags=0):
 def test_batch_classes(bb, port, sizes, squares, per_class):
     _run_batch(bb, port, sizes * 3, [s + k * len(sizes) for s in squares for k in range(3)],
                bb.BGPU_BATCH_PER_CLASS if per_class else 0)
+
+
+# levels of equally spaced products: fewer than a group, more than 128, and (the
+# longest) several groups of launches a level
+@pytest.mark.parametrize("n", [1300, 20_000, 77_777, 2_500_000])
+def test_decimal_levels(bb, n):
+    rng = np.random.default_rng([SEED, n])
+    a = rng.integers(0, 1 << 28, n).astype(np.uint32)
+    a[-1] |= 1
+    text = bb.to_decimal(a)
+    back, neg = bb.from_decimal(text)
+    assert not neg and np.array_equal(back, a)
+    p = (1 << 61) - 1  # the text itself, modulo a prime
+    want = 0
+    for d in a[::-1].tolist():
+        want = ((want << 28) + d) % p
+    got = 0
+    for i in range(0, len(text), 18):
+        piece = text[i : i + 18]
+        got = (got * 10 ** len(piece) + int(piece)) % p
+    assert got == want
