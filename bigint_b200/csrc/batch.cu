@@ -195,7 +195,7 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
                    : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], d_descs + c.desc_off,
                                       (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci]);
         if (e != cudaSuccess) return BGPU_ERR_CUDA;
-        launches += kNttLaunches;
+        launches += c.form.np ? wide_launches(c.form) : kNttLaunches;
     }
     size_t bi = nbranched;
     if (!p->school.empty() && !p->mixed) {

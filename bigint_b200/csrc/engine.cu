@@ -81,7 +81,7 @@ struct Engine {
     // optional per-kernel timing of NTT products: a ring of event sets, one
     // set per product, read back (and averaged) without per-product syncs
     bool kernel_timing = false;
-    bool timed_wide = false;  // the last product timed was a five-prime one
+    int timed_wide = 0;  // the last product timed: 0 three primes, 1 and 2 the wide-digit kernels, short transforms' ones
     std::vector<cudaEvent_t> kev;  // kTimingRing * (kNttLaunches + 1)
     uint64_t kev_count = 0;
     // operand block of products beyond the largest transform (a power of
@@ -260,10 +260,10 @@ int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, WideF
     if (g.kernel_timing) {
         ev = g.kev.data() + (g.kev_count % kTimingRing) * (kNttLaunches + 1);
         ++g.kev_count;
-        g.timed_wide = true;
+        g.timed_wide = f.log_n <= kWideShortMaxLogN ? 2 : 1;
     }
     const cudaError_t e = launch_wide_product(f, nullptr, one, WideStep{}, 1, square, out_fmt, bpp, cl, st, ev);
-    g.last_launches = kNttLaunches;
+    g.last_launches = wide_launches(f);
     if (stats) {
         stats->method = BGPU_METHOD_NTT;
         stats->log2_points = (uint32_t)std::max(5, ceil_log2((uint64_t)a.nd32 + b.nd32 - 1));
@@ -277,7 +277,7 @@ int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, WideF
 constexpr uint64_t kWideGroupPoints = 1u << 21;
 
 // `count` products of na x nb limbs, pr[i] being pr[0] moved by i equal steps,
-// as one set of four launches for each group.
+// as one set of launches for each group.
 int multiply_wide_many(WideForm f, const bgpu_product* pr, size_t count, cudaStream_t st, uint32_t* launches) {
     const size_t na = pr[0].na, nb = pr[0].nb;
     const uint32_t bpp = wide_carry_blocks(f.np, na + nb, kFmtLimb64);
@@ -312,7 +312,7 @@ int multiply_wide_many(WideForm f, const bgpu_product* pr, size_t count, cudaStr
         const cudaError_t e =
             launch_wide_product(f, nullptr, one, step, n, false, kFmtLimb64, bpp, cl, st, nullptr);
         if (e != cudaSuccess) return cuda_status(e);
-        *launches += kNttLaunches;
+        *launches += wide_launches(f);
     }
     return BGPU_OK;
 }
@@ -350,7 +350,7 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     if (g.kernel_timing) {
         ev = g.kev.data() + (g.kev_count % kTimingRing) * (kNttLaunches + 1);
         ++g.kev_count;
-        g.timed_wide = false;
+        g.timed_wide = 0;
     }
     const int ps = prime_set_for(ln);
     cudaError_t e = launch_ntt_product(kSlotEngine + ps, g.consts[ps], a, b, square, ln, s, out,
@@ -2727,7 +2727,7 @@ int bgpu_kernel_times(const char** names, float* mean_ms, int cap, uint32_t* npr
             if (cudaEventElapsedTime(&t, ev[k], ev[k + 1]) != cudaSuccess) return BGPU_ERR_CUDA;
             sum += t;
         }
-        if (names) names[k] = g.timed_wide ? kWideKernelNames[k] : kNttKernelNames[k];
+        if (names) names[k] = g.timed_wide ? kWideKernelNames[g.timed_wide - 1][k] : kNttKernelNames[k];
         if (mean_ms) mean_ms[k] = (float)(sum / (double)n);
     }
     if (nproducts) *nproducts = (uint32_t)n;

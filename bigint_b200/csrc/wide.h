@@ -35,9 +35,9 @@ struct WideForm {
 // than five primes from 2^min_long points.
 WideForm wide_form(uint32_t nd32a, uint32_t nd32b, int min_long);
 
-// Shortest transform: below it (1024 limbs of product) the three-prime
-// kernels, whose few blocks are as fast.
-constexpr int kWideMinLogN = 10;
+// Shortest transform, and the longest that one block does whole.
+constexpr int kWideMinLogN = 8;
+constexpr int kWideShortMaxLogN = 12;
 
 // Products of one set of launches: descs, or one product moved by equal steps
 // (bytes; planes and flags follow one another).  Launch arguments are kept
@@ -95,7 +95,10 @@ __host__ __device__ inline uint32_t wide_carry_blocks(int np, size_t out_cap, in
 // built-in one.  log_n2 == 0: no transform of this length.
 TransformShape wide_shape(int log_n, bool batch);
 cudaError_t upload_wide_consts(int set, const NttConsts& c);
-extern const char* const kWideKernelNames[kNttLaunches];
+// Kernels of a form: four, or two where one block does a transform whole (the
+// middle entries of its timing are empty).
+inline uint32_t wide_launches(WideForm f) { return f.log_n <= kWideShortMaxLogN ? 2 : kNttLaunches; }
+extern const char* const kWideKernelNames[2][kNttLaunches];
 
 // The four launches of `count` products of one form (digits of both operands
 // together at most 2^log_n + 1); each product's carry scan has `bpp` blocks

@@ -136,22 +136,22 @@ __device__ __forceinline__ void load_digit(const OperandDesc& in, uint32_t nd, u
 // two words becomes digit 2^-32 mod p, of three digit 2^-64 mod p (the scale of
 // the row pass undoes it), in [0, 2p) or [0, p).  HALF: the rows of the upper half of the transform are zero; they
 // are not loaded and the first stage is one multiply per pair.
-template <bool LAZY, int L2, int T, int NP, bool LIMB, bool HALF>
-__device__ __forceinline__ void wide_round0(const WideArgs& a, const OperandDesc& in, uint32_t nd, const NttConsts& c,
-                                            int q, uint32_t c0, uint32_t* sm) {
-    using Gr = Group<L2, kWideCols, 0>;
+template <bool LAZY, int L2, int C, int T, int NP, bool LIMB, bool HALF>
+__device__ __forceinline__ void wide_round0(int log_n1, const OperandDesc& in, uint32_t nd, const NttConsts& c, int q,
+                                            uint32_t c0, uint32_t* sm, int tid) {
+    using Gr = Group<L2, C, 0>;
     constexpr int R = Gr::R;
     constexpr int D = 1 << (R - 1);
     constexpr int NL = HALF ? D : (1 << R);
     const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv, red = c.red[q];
     const uint2* tw = c.stage[q][0];
-    const uint32_t stride = 1u << (Gr::LO + a.log_n1);
+    const uint32_t stride = 1u << (Gr::LO + log_n1);
 #pragma unroll 2
-    for (int g = threadIdx.x; g < Gr::G; g += T) {
+    for (int g = tid; g < Gr::G; g += T) {
         const Gr gr(g);
         uint32_t x[1 << R];
         uint32_t any = 0;
-        uint32_t n = c0 + gr.col + (gr.base << a.log_n1);
+        uint32_t n = c0 + gr.col + (gr.base << log_n1);
 #pragma unroll
         for (int j = 0; j < NL; ++j, n += stride) {
             uint32_t d[3];
@@ -191,6 +191,31 @@ __device__ __forceinline__ void wide_round0(const WideArgs& a, const OperandDesc
     }
 }
 
+template <bool LAZY, int L2, int C, int T, int NP>
+__device__ __forceinline__ void wide_load(int log_n1, const OperandDesc& in, size_t nn, const NttConsts& c, int q,
+                                          uint32_t c0, uint32_t* sm, int tid) {
+    const uint32_t nd = wide_digits(NP, in.nd32);
+    const bool half = 2 * (size_t)nd <= nn;
+    if (in.fmt == kFmtLimb64) {
+        if (half)
+            wide_round0<LAZY, L2, C, T, NP, true, true>(log_n1, in, nd, c, q, c0, sm, tid);
+        else
+            wide_round0<LAZY, L2, C, T, NP, true, false>(log_n1, in, nd, c, q, c0, sm, tid);
+    } else {
+        if (half)
+            wide_round0<LAZY, L2, C, T, NP, false, true>(log_n1, in, nd, c, q, c0, sm, tid);
+        else
+            wide_round0<LAZY, L2, C, T, NP, false, false>(log_n1, in, nd, c, q, c0, sm, tid);
+    }
+}
+
+__device__ __forceinline__ OperandDesc wide_operand(const WideFwdArgs& fa, uint32_t product, int op) {
+    if (fa.w.descs) return fa.w.descs[product].op[op];
+    OperandDesc in = op == 0 ? fa.op[0] : fa.op[1];
+    in.ptr = static_cast<const char*>(in.ptr) + (int64_t)product * (op == 0 ? fa.step_a : fa.step_b);
+    return in;
+}
+
 // CTAs per SM (register caps): 1024 threads' worth of 64 registers, except
 // columns of 2^9 rows at 1280 (2^19 points of a batch: 15.0 + 5.7 us; at 1024
 // 15.5 + 6.2, at 2048 15.1 + 5.9) and the inverse pass's tiles of 2^11 rows.
@@ -210,13 +235,7 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const
     const uint32_t product = blockIdx.z / (uint32_t)a.nops;
     const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
     const uint2* tw = c.stage[q][0];
-    OperandDesc in;
-    if (a.descs) {
-        in = a.descs[product].op[op];
-    } else {
-        in = op == 0 ? fa.op[0] : fa.op[1];
-        in.ptr = static_cast<const char*>(in.ptr) + (int64_t)product * (op == 0 ? fa.step_a : fa.step_b);
-    }
+    const OperandDesc in = wide_operand(fa, product, op);
     const uint32_t c0 = blockIdx.x * kWideCols;
     const size_t nn = (size_t)1 << a.log_n;
     uint32_t* y = wide_planes(a, product) + ((size_t)op * NP + q) * nn;
@@ -231,18 +250,7 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const
             inter_twiddle(c, q, 0, (((c0 + col) * m) << (L2 - RL)) & (uint32_t)(nn - 1), a.log_n, p), p, np);
     }
     pdl_wait();
-    const uint32_t nd = wide_digits(NP, in.nd32);
-    if (in.fmt == kFmtLimb64) {
-        if (2 * (size_t)nd <= nn)
-            wide_round0<LAZY, L2, T, NP, true, true>(a, in, nd, c, q, c0, sm);
-        else
-            wide_round0<LAZY, L2, T, NP, true, false>(a, in, nd, c, q, c0, sm);
-    } else {
-        if (2 * (size_t)nd <= nn)
-            wide_round0<LAZY, L2, T, NP, false, true>(a, in, nd, c, q, c0, sm);
-        else
-            wide_round0<LAZY, L2, T, NP, false, false>(a, in, nd, c, q, c0, sm);
-    }
+    wide_load<LAZY, L2, kWideCols, T, NP>(a.log_n1, in, nn, c, q, c0, sm, threadIdx.x);
     __syncthreads();
     dif_rounds<LAZY, L2, kWideCols, T, 1, NR - 2>(sm, tw, p, threadIdx.x);
     using Gr = Group<L2, kWideCols, NR - 1>;
@@ -418,6 +426,79 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, false)) k_wide_inv(cons
 #pragma unroll
         for (int j = 0; j < (1 << R); ++j)
             y[((size_t)gr.idx(j) << a.log_n1) + gr.col] = Bfly<LAZY>::reduce(x[j], p);
+    }
+    pdl_trigger();
+}
+
+// ---- 1 to 3 of short transforms ------------------------------------------------------
+
+// Threads of an operand.
+__host__ __device__ constexpr int wide_short_threads(int l) { return l <= 9 ? 32 : 1 << (l - 4); }
+
+// Up to 2^12 points: the whole product of one prime in one CTA, both operands'
+// transforms at once in halves of the threads.  Loads, rounds and the
+// pointwise product are those of the passes above; nothing goes through memory
+// in between and there are no inter-pass twiddles.  us per product back to back,
+// four launches -> two: 2^10 points 11.5 -> 6.7, 2^11 9.5 -> 8.5, 2^12 9.7 -> 11.1,
+// but from the host, whose launches bound them, 14.2 -> 9.6 at 2^11 and no more at
+// 2^12; three primes at 2^10 32-bit digits 11.3, here at 2^9 points 6.7.
+// A batch: product tree of 2^20 leaves 2.28 -> 2.07 ms.
+template <int L, int NP, bool SQR>
+__global__ void __launch_bounds__(wide_short_threads(L) * (SQR ? 1 : 2)) k_wide_short(const WideFwdArgs fa) {
+    constexpr int T = wide_short_threads(L), TT = SQR ? T : 2 * T;
+    using P = Plan<L>;
+    constexpr int NR = P::nr;
+    static_assert(NR > 1, "several rounds");
+    extern __shared__ __align__(16) uint32_t sm[];  // A's row, B's
+    const NttConsts& c = c_wide[wide_set_index(NP, true)];
+    const int q = blockIdx.x, op = SQR ? 0 : (int)threadIdx.x / T, tid = (int)threadIdx.x - op * T;
+    const uint32_t product = blockIdx.z;
+    const uint32_t p = c.pr[q].p, np = 0u - c.pr[q].pinv;
+    const uint2* twf = c.stage[q][0];
+    const uint2* twi = c.stage[q][1];
+    const uint32_t scale = c_scale[wide_set_index(NP, true)][L][q];
+    uint32_t* s = sm + ((uint32_t)op << L);
+    pdl_wait();
+    const OperandDesc in = wide_operand(fa, product, op);
+    uint32_t* y = wide_planes(fa.w, product) + ((size_t)q << L);
+    wide_load<true, L, 1, T, NP>(0, in, (size_t)1 << L, c, q, 0, s, tid);
+    __syncthreads();
+    dif_rounds<true, L, 1, T, 1, NR - 2>(s, twf, p, tid);
+    if constexpr (!SQR) {
+        smem_round<true, L, 1, T, NR - 1, false>(s, twf, p, tid);
+        __syncthreads();
+    }
+    {  // the last DIF round of a square, the pointwise product, the first DIT round
+        using Gr = Group<L, 1, NR - 1>;
+        constexpr int R = Gr::R;
+#pragma unroll 1
+        for (int g = threadIdx.x; g < Gr::G; g += TT) {
+            const Gr gr(g);
+            uint32_t x[1 << R];
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) x[j] = sm[gr.at(j)];
+            if constexpr (SQR) dif_regs<true, R, Gr::HI, Gr::LO>(x, gr.base_low, twf, p);
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) x[j] = mont(x[j], SQR ? x[j] : sm[(1u << L) + gr.at(j)], p, np);
+            dit_regs<true, R, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) sm[gr.at(j)] = x[j];
+        }
+    }
+    __syncthreads();
+    dit_rounds<true, L, 1, TT, NR - 2, 1>(sm, twi, p, threadIdx.x);
+    using Gr = Group<L, 1, 0>;
+    constexpr int R = Gr::R;
+    const uint2 sc = shoup_of(scale, p, np);
+#pragma unroll 1
+    for (int g = threadIdx.x; g < Gr::G; g += TT) {
+        const Gr gr(g);
+        uint32_t x[1 << R];
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j) x[j] = sm[gr.at(j)];
+        dit_regs<true, R, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j) y[gr.idx(j)] = csub(shoup_lazy(x[j], sc.x, sc.y, p), p);
     }
     pdl_trigger();
 }
@@ -862,6 +943,30 @@ uint32_t pow_m(uint64_t b, uint32_t e, uint32_t p) {
     return (uint32_t)r;
 }
 
+template <int L, int NP>
+cudaError_t launch_short_of(const WideFwdArgs& fa, uint32_t count, cudaStream_t st) {
+    const size_t sm = (size_t)4 * fa.w.nops << L;
+    const dim3 grid(NP, 1, count);
+    return fa.w.nops == 1 ? launch_k(k_wide_short<L, NP, true>, grid, dim3(wide_short_threads(L)), sm, st, fa)
+                          : launch_k(k_wide_short<L, NP, false>, grid, dim3(2 * wide_short_threads(L)), sm, st, fa);
+}
+template <int L>
+cudaError_t launch_short(const WideFwdArgs& fa, uint32_t count, cudaStream_t st) {
+    return fa.w.np == 5   ? launch_short_of<L, 5>(fa, count, st)
+           : fa.w.np == 6 ? launch_short_of<L, 6>(fa, count, st)
+                          : launch_short_of<L, 7>(fa, count, st);
+}
+cudaError_t dispatch_short(const WideFwdArgs& fa, uint32_t count, cudaStream_t st) {
+    switch (fa.w.log_n) {
+        case 8: return launch_short<8>(fa, count, st);
+        case 9: return launch_short<9>(fa, count, st);
+        case 10: return launch_short<10>(fa, count, st);
+        case 11: return launch_short<11>(fa, count, st);
+        case 12: return launch_short<12>(fa, count, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 // 1 / N / (M / p) mod p times a power of two, Montgomery form: the inverse
 // transform's 1/N, the CRT's (M/p)^-1, and 2^32 for the pointwise product and
 // each reduction of the two digits (one each, two for three words).
@@ -913,7 +1018,8 @@ TransformShape wide_shape(int log_n, bool batch) {
     return s;
 }
 
-const char* const kWideKernelNames[kNttLaunches] = {"k_wide_fwd", "k_wide_rows", "k_wide_inv", "k_wide_carry"};
+const char* const kWideKernelNames[2][kNttLaunches] = {{"k_wide_fwd", "k_wide_rows", "k_wide_inv", "k_wide_carry"},
+                                                       {"k_wide_short", "none", "none", "k_wide_carry"}};
 
 // Longest transform over np primes.
 static int wide_max_log(int np) { return kPrimeSets[kFirstWideSet + 2 * (np - kWidePrimes) + 1].log_max; }
@@ -942,8 +1048,9 @@ cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const Prod
     const int log_n = f.log_n;
     if (f.np < kWidePrimes || f.np > kWideMaxPrimes || log_n > wide_max_log(f.np) || count < 1 || count > kWidePiece)
         return cudaErrorInvalidValue;
-    const int l2 = wide_shape(log_n, descs != nullptr || count > 1).log_n2;
-    if (!l2) return cudaErrorInvalidValue;
+    const bool whole = log_n <= kWideShortMaxLogN;
+    const int l2 = whole ? 0 : wide_shape(log_n, descs != nullptr || count > 1).log_n2;
+    if (log_n < kWideMinLogN || (!whole && !l2)) return cudaErrorInvalidValue;
     const int w = wide_set_for(f.np, log_n) - kFirstWideSet;
     const bool lazy = w % 2 == 0;
     WideFwdArgs fa{};
@@ -960,13 +1067,21 @@ cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const Prod
     fa.step_a = step.a;
     fa.step_b = step.b;
     if (ev) cudaEventRecord(ev[0], st);
-    cudaError_t e = lazy ? dispatch_cols<true>(l2, true, fa, count, st) : dispatch_cols<false>(l2, true, fa, count, st);
-    if (e != cudaSuccess) return e;
-    if (ev) cudaEventRecord(ev[1], st);
-    e = lazy ? dispatch_rows<true>(a.log_n1, a, square, count, st) : dispatch_rows<false>(a.log_n1, a, square, count, st);
-    if (e != cudaSuccess) return e;
-    if (ev) cudaEventRecord(ev[2], st);
-    e = lazy ? dispatch_cols<true>(l2, false, fa, count, st) : dispatch_cols<false>(l2, false, fa, count, st);
+    cudaError_t e = cudaSuccess;
+    if (whole) {
+        e = dispatch_short(fa, count, st);
+        if (ev) cudaEventRecord(ev[1], st);
+        if (ev) cudaEventRecord(ev[2], st);
+    } else {
+        e = lazy ? dispatch_cols<true>(l2, true, fa, count, st) : dispatch_cols<false>(l2, true, fa, count, st);
+        if (e != cudaSuccess) return e;
+        if (ev) cudaEventRecord(ev[1], st);
+        e = lazy ? dispatch_rows<true>(a.log_n1, a, square, count, st)
+                 : dispatch_rows<false>(a.log_n1, a, square, count, st);
+        if (e != cudaSuccess) return e;
+        if (ev) cudaEventRecord(ev[2], st);
+        e = lazy ? dispatch_cols<true>(l2, false, fa, count, st) : dispatch_cols<false>(l2, false, fa, count, st);
+    }
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[3], st);
     WideCarryArgs ca{};
