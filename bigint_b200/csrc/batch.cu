@@ -496,9 +496,9 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
         L.w = w;
         if (w <= 4) {
             L.kind = 0;
-        } else if (2 * w <= tu.batch_schoolbook_max_limbs) {
+        } else if (2 * w <= std::min<size_t>(tu.batch_schoolbook_max_limbs, kLevelSmallMaxLimbs)) {
             L.kind = 1;
-        } else if (2 * w <= tu.batch_karatsuba_max_limbs && karatsuba_fits(w, w)) {
+        } else if (2 * w <= std::min<size_t>(tu.batch_karatsuba_max_limbs, kLevelSmallMaxLimbs) && karatsuba_fits(w, w)) {
             L.kind = 2;
         } else {
             L.kind = 3;

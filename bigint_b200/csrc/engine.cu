@@ -2049,8 +2049,9 @@ static int run_products(const bgpu_product* pr, size_t count, cudaStream_t st, u
     if (count == 0) return BGPU_OK;
     const size_t na = pr[0].na, nb = pr[0].nb;
     const Tuning& tu = tuning();
-    const bool school = na + nb <= tu.batch_schoolbook_max_limbs;
-    if (school || (na + nb <= tu.batch_karatsuba_max_limbs && karatsuba_fits(na, nb))) {
+    const bool level = na + nb <= kLevelSmallMaxLimbs;
+    const bool school = level && na + nb <= tu.batch_schoolbook_max_limbs;
+    if (school || (level && na + nb <= tu.batch_karatsuba_max_limbs && karatsuba_fits(na, nb))) {
         std::vector<SchoolDesc> d(count);
         for (size_t i = 0; i < count; ++i)
             d[i] = SchoolDesc{pr[i].a, pr[i].b, pr[i].out, (uint32_t)pr[i].na, (uint32_t)pr[i].nb};

@@ -27,6 +27,12 @@ constexpr int kWideMaxPrimes = 7;
 // 2^15 over six 16.6, 2^16 over five 16.4; 2^16 over six 19.0, over seven 19.4, 2^17 over five 21.3.
 constexpr int kLongDigitMinLogN = 16;
 
+// Levels of equal products (product trees, decimal conversions) leave the
+// schoolbook and Karatsuba kernels here, whatever their crossovers: us per 1024
+// products, 192 limbs schoolbook 24.9, this 31.0; 256 limbs 37.0, Karatsuba
+// 45.5, this 31.0; 512 limbs Karatsuba 115, this 31.
+constexpr size_t kLevelSmallMaxLimbs = 192;
+
 // Transform of a product: 2^log_n points over np primes (np == 0: none).
 struct WideForm {
     int np = 0, log_n = 0;
