@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -2101,14 +2102,30 @@ static int from_decimal_locked(const char* s, size_t len, uint32_t* out, size_t 
         if (c >= '0' && c <= '9') break;
         if (c == '-') neg = true;
     }
-    std::vector<uint8_t> dig;
-    dig.reserve(len - i);
-    for (; i < len; ++i) {  // other characters are skipped; leading zeros dropped
-        const unsigned char c = (unsigned char)s[i];
-        if (c < '0' || c > '9' || (dig.empty() && c == '0')) continue;
-        dig.push_back((uint8_t)(c - '0'));
+    std::unique_ptr<uint8_t[]> dig(new (std::nothrow) uint8_t[len - i + 1]);
+    if (!dig) return BGPU_ERR_OOM;
+    uint64_t D = 0;
+    auto take = [&](size_t end) {  // other characters are skipped; leading zeros dropped
+        for (; i < end; ++i) {
+            const uint8_t d = (uint8_t)((uint8_t)s[i] - (uint8_t)'0');
+            if (d <= 9 && (D || d)) dig[D++] = d;
+        }
+    };
+    // Blocks of digits alone, which the compiler turns into vector code; a
+    // character at a time took most of the conversion (1.0 of 1.7 ms for a million).
+    constexpr size_t kBlock = 64;
+    while (len - i >= kBlock) {
+        uint8_t top = D ? 0 : 10;
+        for (size_t k = 0; k < kBlock; ++k) top = std::max(top, (uint8_t)((uint8_t)s[i + k] - (uint8_t)'0'));
+        if (top > 9) {
+            take(i + kBlock);
+            continue;
+        }
+        for (size_t k = 0; k < kBlock; ++k) dig[D + k] = (uint8_t)((uint8_t)s[i + k] - (uint8_t)'0');
+        D += kBlock;
+        i += kBlock;
     }
-    const uint64_t D = dig.size();
+    take(len);
     if (D == 0) {  // the reference's zero: one digit 0, not negative
         *out_len = 1;
         *out_neg = 0;
@@ -2135,7 +2152,7 @@ static int from_decimal_locked(const char* s, size_t len, uint32_t* out, size_t 
                         reinterpret_cast<uint64_t*>(base + lvl_off + align256(NL * 8))};
     uint32_t* dout = reinterpret_cast<uint32_t*>(base + o_off);
     cudaStream_t st = g.stream;
-    rc = host_to_device(ddig, dig.data(), D, st, nullptr);
+    rc = host_to_device(ddig, dig.get(), D, st, nullptr);
     if (rc != BGPU_OK) return rc;
     uint32_t nl = 0;
     rc = ensure_powers(J, false, st, &nl);  // 10^(19 * 2^j) at limb 2^j - 1, 2^j limbs

@@ -187,3 +187,18 @@ def test_decimal_levels(bb, n):
         piece = text[i : i + 18]
         got = (got * 10 ** len(piece) + int(piece)) % p
     assert got == want
+
+
+# text that is not digits alone, in and out of the blocks of 64 characters
+@pytest.mark.parametrize("text,value", [
+    ("0" * 200 + "7" * 300, int("7" * 300)),
+    ("-" + "0" * 63 + "9" * 64, -int("9" * 64)),
+    ("x" * 70 + "-" + "12,345." * 40 + "6", -int("12345" * 40 + "6")),
+    ("1" + "0" * 127 + "-" + "5" * 129, int("1" + "0" * 127 + "5" * 129)),
+    ("0" * 64, 0),
+    ("3" * 63 + ":" + "4" * 64 + "/", int("3" * 63 + "4" * 64)),
+])
+def test_decimal_text_blocks(bb, text, value):
+    digits, neg = bb.from_decimal(text)
+    got = sum(int(d) << (28 * k) for k, d in enumerate(digits))
+    assert (-got if neg else got) == value
