@@ -1277,8 +1277,8 @@ def run_gpu_arm(args) -> None:
     sptr = stream.cuda_stream
 
     def step(i, flags=bb.BGPU_INDEPENDENT):
-        # the products are independent: each one's transform may start under
-        # the previous product's carry scan (BGPU_INDEPENDENT)
+        # the products are independent (BGPU_INDEPENDENT; the wide-digit
+        # transforms make no use of it)
         k = i % npairs
         bb.mul_device(dA[k].data_ptr(), na, dB[k].data_ptr(), nb, dOut[k].data_ptr(), stream=sptr,
                       method=flags)
@@ -1482,8 +1482,9 @@ def run_gpu_arm(args) -> None:
                    "l2": f"inputs larger than L2: {npairs} distinct operand pairs "
                          f"({npairs * 2 * na * 8 >> 20} MiB) cycled, steps back to back",
                    "parallelism": f"replicas x{world}", "verified": verified,
-                   "pipelining": "independent products (BGPU_INDEPENDENT): each product's forward "
-                                 "transform starts under the previous product's carry scan",
+                   "pipelining": "independent products (BGPU_INDEPENDENT); launches chained with "
+                                 "programmatic dependent launch",
+                   "transform": "64-bit digits over five primes, half as many points as 32-bit digits",
                    "timing": f"median of {nwin} windows of exactly K={args.steps} products, each window "
                              "bracketed by barrier + synchronize, CUDA events on the launching stream; "
                              "max over ranks",

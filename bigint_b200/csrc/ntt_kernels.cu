@@ -267,13 +267,6 @@ __global__ void __launch_bounds__(T, fwd_min_blocks(L2, T)) k_fwd_cols(const Fwd
 // ---- kernel 2: middle row pass ----------------------------------------------
 
 
-// Rows too long for two row buffers in shared memory (2^15 points of a
-// non-square product): A's transformed row is parked in its own global plane
-// and read back there by the pointwise product, while B's row uses the one
-// shared buffer.
-template <int L1, bool SQR>
-constexpr bool kOneRowBuffer = !SQR && L1 >= 15;
-
 // Last DIF round of B (or A when squaring) fused with the pointwise product
 // and the first DIT round; with a single round also the inverse twiddle.
 template <bool LAZY, int L1, int T, bool SQR, bool SINGLE, bool MULTI>
@@ -281,7 +274,6 @@ __device__ __forceinline__ void mid_turn(const MidRowsArgs& a, const NttConsts& 
                                          uint32_t* sb, const uint32_t* row_a, const uint32_t* row_b,
                                          uint32_t* row_out, int q, uint32_t k2, const uint2* sT) {
     const int tid = sub_tid<T, MULTI>();
-    constexpr bool ONE = kOneRowBuffer<L1, SQR>;
     using P1 = Plan<L1>;
     constexpr int K = P1::nr - 1;
     using Gr = Group<L1, 1, K>;
@@ -291,7 +283,7 @@ __device__ __forceinline__ void mid_turn(const MidRowsArgs& a, const NttConsts& 
     const uint2* twi = c.stage[q][1];
     const uint32_t sw = q == 0 ? a.scale_w[0] : (q == 1 ? a.scale_w[1] : a.scale_w[2]);
     const uint32_t swp = q == 0 ? a.scale_wp[0] : (q == 1 ? a.scale_wp[1] : a.scale_wp[2]);
-    const uint32_t* src = (SQR || ONE) ? sa : sb;
+    const uint32_t* src = SQR ? sa : sb;
 #pragma unroll 1
     for (int g = tid; g < Gr::G; g += T) {
         const Gr gr(g);
@@ -306,7 +298,7 @@ __device__ __forceinline__ void mid_turn(const MidRowsArgs& a, const NttConsts& 
         dif_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twf, p);
 #pragma unroll
         for (int j = 0; j < (1 << R); ++j) {
-            const uint32_t other = SQR ? x[j] : (ONE ? row_a[gr.idx(j)] : sa[gr.at(j)]);
+            const uint32_t other = SQR ? x[j] : sa[gr.at(j)];
             x[j] = pointwise<LAZY>(x[j], other, p, pinv);
         }
         dit_regs<LAZY, R, Gr::HI, Gr::LO>(x, gr.base_low, twi, p);
@@ -369,11 +361,9 @@ template <int PS, int L1, int T, bool SQR, bool MULTI = false>
 __device__ __forceinline__ void mid_rows_body(const MidRowsArgs& a, uint32_t slot, uint32_t by,
                                               uint32_t* sm) {  // sm: sa[2^L1] (+ sb[2^L1]) + powers
     constexpr bool LAZY = PS == 0;
-    constexpr bool ONE = kOneRowBuffer<L1, SQR>;
     const int tid = sub_tid<T, MULTI>();
     using P1 = Plan<L1>;
     constexpr int NR = P1::nr;
-    static_assert(!ONE || NR > 1, "the one-buffer row pass needs several rounds");
     const NttConsts& c = c_consts[a.slot];
     uint32_t* sa = sm;
     uint32_t* sb = sm + (1u << L1);
@@ -397,7 +387,7 @@ __device__ __forceinline__ void mid_rows_body(const MidRowsArgs& a, uint32_t slo
     // register allocation, and the spills, of the mixed-length row launch
     // that inlines it.)
     constexpr int R0 = P1::r(0), LO0 = P1::lo(0);
-    uint2* sT = reinterpret_cast<uint2*>(sm + ((SQR || ONE ? 1u : 2u) << L1));
+    uint2* sT = reinterpret_cast<uint2*>(sm + ((SQR ? 1u : 2u) << L1));
     for (int t = tid; t < (1 << R0); t += T) {
         const uint32_t w = inter_twiddle(c, q, 1, ((k2 * (uint32_t)t) << LO0) & (uint32_t)(nn - 1),
                                          a.log_n, p);
@@ -425,15 +415,7 @@ __device__ __forceinline__ void mid_rows_body(const MidRowsArgs& a, uint32_t slo
         mid_turn<LAZY, L1, T, SQR, true, MULTI>(a, c, sa, sb, row_a, row_b, row_a, q, k2, sT);
     } else {
         mid_dif_row<LAZY, L1, T, MULTI>(row_a, sa, twf, p);
-        if constexpr (ONE) {
-            smem_round<LAZY, L1, 1, T, NR - 1, false>(sa, twf, p, tid);  // A's last DIF round
-            __syncthreads();
-            // park A's transform in its plane (element i at row_a[i]) ...
-            for (uint32_t i = tid; i < (1u << L1); i += T) row_a[i] = sa[sidx<1>(i, 0)];
-            __syncthreads();
-            // ... and transform B in the same buffer
-            mid_dif_row<LAZY, L1, T, MULTI>(row_b, sa, twf, p);
-        } else if constexpr (!SQR) {
+        if constexpr (!SQR) {
             smem_round<LAZY, L1, 1, T, NR - 1, false>(sa, twf, p, tid);  // A's last DIF round
             mid_dif_row<LAZY, L1, T, MULTI>(row_b, sb, twf, p);
         }
@@ -471,7 +453,7 @@ __global__ void __launch_bounds__(T, mid_min_blocks(L1, T)) k_mid_rows(const Mid
 //
 // k_rows_dif finishes an operand block's forward transform: the row DIF of
 // row blockIdx.x, prime blockIdx.y, stored back in place with element i at
-// row[i] (the order the one-buffer row pass parks A's transform in).
+// row[i].
 // k_rows_mac forms, per row, sum_t sa[t] (.) sb[t] over the launch's pairs of
 // such spectra (Montgomery products, so the sum carries 2^-32, which the scale
 // in the last round cancels) and runs the row DIT with the inverse
@@ -1076,7 +1058,7 @@ static bool shape_ok(const TransformShape& s, bool square) {
     if (s.log_n2 < 2 || s.log_n2 > 11) return false;
     if (s.log_n1 < 3 || s.log_n1 > 15) return false;
     // Rows of 2^15 points are built for the strict prime set only (transforms
-    // above 2^23 points); non-square products use the one-buffer row pass.
+    // above 2^23 points: spectral sums).
     if (s.log_n1 == 15 && prime_set_for(s.log_n) == 0) return false;
     (void)square;
     return true;
@@ -1149,25 +1131,23 @@ static cudaError_t launch_mid(const MidRowsArgs& m, bool square, uint32_t rows, 
     return launch_k(k, grid, dim3(T), sm, st, m);
 }
 
-template <int PS>
+// Lazy set only: transforms of the strict one are products of spectral sums,
+// every other product as long is a wide-digit one.
 static cudaError_t dispatch_mid(int l1, const MidRowsArgs& m, bool square, uint32_t rows, int count,
                                 cudaStream_t st) {
     switch (l1) {
-        case 3: return launch_mid<PS, 3>(m, square, rows, count, st);
-        case 4: return launch_mid<PS, 4>(m, square, rows, count, st);
-        case 5: return launch_mid<PS, 5>(m, square, rows, count, st);
-        case 6: return launch_mid<PS, 6>(m, square, rows, count, st);
-        case 7: return launch_mid<PS, 7>(m, square, rows, count, st);
-        case 8: return launch_mid<PS, 8>(m, square, rows, count, st);
-        case 9: return launch_mid<PS, 9>(m, square, rows, count, st);
-        case 10: return launch_mid<PS, 10>(m, square, rows, count, st);
-        case 11: return launch_mid<PS, 11>(m, square, rows, count, st);
-        case 12: return launch_mid<PS, 12>(m, square, rows, count, st);
-        case 13: return launch_mid<PS, 13>(m, square, rows, count, st);
-        case 14: return launch_mid<PS, 14>(m, square, rows, count, st);
-        case 15:
-            if constexpr (PS == 1) return launch_mid<PS, 15>(m, square, rows, count, st);
-            return cudaErrorInvalidValue;
+        case 3: return launch_mid<0, 3>(m, square, rows, count, st);
+        case 4: return launch_mid<0, 4>(m, square, rows, count, st);
+        case 5: return launch_mid<0, 5>(m, square, rows, count, st);
+        case 6: return launch_mid<0, 6>(m, square, rows, count, st);
+        case 7: return launch_mid<0, 7>(m, square, rows, count, st);
+        case 8: return launch_mid<0, 8>(m, square, rows, count, st);
+        case 9: return launch_mid<0, 9>(m, square, rows, count, st);
+        case 10: return launch_mid<0, 10>(m, square, rows, count, st);
+        case 11: return launch_mid<0, 11>(m, square, rows, count, st);
+        case 12: return launch_mid<0, 12>(m, square, rows, count, st);
+        case 13: return launch_mid<0, 13>(m, square, rows, count, st);
+        case 14: return launch_mid<0, 14>(m, square, rows, count, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -1274,8 +1254,8 @@ static cudaError_t launch_ntt_core(int slot, const NttConsts& c, const ProductDe
                                    const TransformShape& sh, int out_fmt, const CarryLaunch& cl,
                                    cudaStream_t st, cudaEvent_t* ev) {
     const int log_n = sh.log_n;
-    if (!shape_ok(sh, square) || log_n > c.log_max || count < 1) return cudaErrorInvalidValue;
-    const int ps = c.log_max == kPrimeSets[0].log_max ? 0 : 1;
+    if (!shape_ok(sh, square) || log_n > c.log_max || c.log_max != kPrimeSets[0].log_max || count < 1)
+        return cudaErrorInvalidValue;
     const uint32_t tiles = (1u << sh.log_n1) / kCols;
     if (ev) cudaEventRecord(ev[0], st);
 
@@ -1287,8 +1267,7 @@ static cudaError_t launch_ntt_core(int slot, const NttConsts& c, const ProductDe
     f.log_n1 = sh.log_n1;
     f.slot = slot;
     f.overlap = cl.overlap_prev && count == 1 ? 1 : 0;
-    cudaError_t e = ps == 0 ? dispatch_outer<0>(sh.log_n2, &f, nullptr, tiles, count, st)
-                            : dispatch_outer<1>(sh.log_n2, &f, nullptr, tiles, count, st);
+    cudaError_t e = dispatch_outer<0>(sh.log_n2, &f, nullptr, tiles, count, st);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[1], st);
 
@@ -1299,11 +1278,10 @@ static cudaError_t launch_ntt_core(int slot, const NttConsts& c, const ProductDe
     m.log_n2 = sh.log_n2;
     m.slot = slot;
     set_scale(c, log_n, m.scale_w, m.scale_wp);
-    e = ps == 0 ? dispatch_mid<0>(sh.log_n1, m, square, 1u << sh.log_n2, count, st)
-                : dispatch_mid<1>(sh.log_n1, m, square, 1u << sh.log_n2, count, st);
+    e = dispatch_mid(sh.log_n1, m, square, 1u << sh.log_n2, count, st);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[2], st);
-    return launch_inverse_carry(slot, ps, descs, one, count, sh, out_fmt, cl, st, ev);
+    return launch_inverse_carry(slot, 0, descs, one, count, sh, out_fmt, cl, st, ev);
 }
 
 // The inverse column pass (with CRT and chunk sums) and the carry scan of

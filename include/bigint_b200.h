@@ -38,7 +38,7 @@ extern "C" {
 
 /* Method selection (flags & BGPU_METHOD_MASK). */
 #define BGPU_METHOD_AUTO 0u
-#define BGPU_METHOD_NTT 1u        /* three-prime NTT (the plain method) */
+#define BGPU_METHOD_NTT 1u        /* multi-prime NTT (the plain method) */
 #define BGPU_METHOD_SCHOOLBOOK 2u /* O(n*m) kernel; na + nb <= BGPU_SCHOOLBOOK_MAX_LIMBS */
 #define BGPU_METHOD_FFT 3u        /* FP64 complex FFT (bgpu_mul_u64 only); products whose
                                      max |x - round(x)| exceeds 1/4 are redone on the NTT */
@@ -55,23 +55,25 @@ extern "C" {
  * or queued on the stream writes this product's operands (a stream of
  * independent products).  The transform of this product may then start while
  * the previous product's carry scan finishes; every later kernel still runs
- * after both.  Ignored when the operands overlap the previous call's output. */
+ * after both.  Ignored when the operands overlap the previous call's output,
+ * and by the wide-digit transforms (products of more than 129 limbs),
+ * whose launches already overlap as far as their buffers allow. */
 #define BGPU_INDEPENDENT 0x20u
 /* bgpu_batch_plan_create / bgpu_mul_batch_device: give every NTT class of the
- * batch its own four launches on parallel graph branches instead of one launch
- * per pass for all classes (see the batch plan section). */
+ * batch its own launches on parallel graph branches, the short lengths too
+ * (see the batch plan section). */
 #define BGPU_BATCH_PER_CLASS 0x40u
 
 #define BGPU_SCHOOLBOOK_MAX_LIMBS 256u
 #define BGPU_KARATSUBA_MAX_LIMBS 256u
-#define BGPU_MAX_LOG2_POINTS 26u  /* transform points are 32-bit digits */
+#define BGPU_MAX_LOG2_POINTS 26u  /* lengths are counted in 32-bit digits */
 /* Largest |point_pos| the BigFloat entry points take (BGPU_ERR_CAPACITY
  * above): 28 * point_pos then stays far inside int64_t. */
 #define BGPU_MAX_POINT_POS ((int64_t)1 << 40)
 
 typedef struct bgpu_stats {
     int32_t method;          /* BGPU_METHOD_* actually used */
-    uint32_t log2_points;    /* transform length (0 for schoolbook) */
+    uint32_t log2_points;    /* transform length in 32-bit digits (0 for schoolbook) */
     double max_round_err;    /* FFT form: max |x - round(x)| over all coefficients; 0 otherwise */
     int32_t fell_back;       /* FFT form: 1 if the product was recomputed on the NTT */
     float device_ms;         /* device time of the multiply kernels */
@@ -246,7 +248,8 @@ int bgpu_set_kernel_timing(int on);
 
 /* Mean device time of each kernel over the NTT products launched since
  * timing was switched on (the last 1024 of them): names[i], mean_ms[i] in
- * launch order, *nproducts = products averaged.  Returns the kernel count
+ * launch order, *nproducts = products averaged (products of short transforms
+ * have two kernels and name the two entries between them "none").  Returns the kernel count
  * (0 if none recorded).  Synchronizes on the last recorded event. */
 int bgpu_kernel_times(const char** names, float* mean_ms, int cap, uint32_t* nproducts);
 
@@ -256,13 +259,12 @@ int bgpu_kernel_times(const char** names, float* mean_ms, int cap, uint32_t* npr
  * step.  A plan groups a batch by size (schoolbook below
  * BGPU_SCHOOLBOOK_MAX_LIMBS, Karatsuba, then one NTT class per transform
  * length), allocates its scratch once and captures every launch of the batch
- * into one CUDA graph; running the plan is one graph launch.  A batch of
- * several transform lengths runs as one launch per NTT pass (four kernel
- * nodes holding every class's blocks, the small products riding in two of
- * them); with BGPU_BATCH_PER_CLASS every class gets its own four launches on
- * parallel graph branches, which overlap one another's pass boundaries (on a
- * B200 the 4096-product log-uniform batch ran 4.5 % faster that way, with 38
- * nodes instead of 4).  Pointers are device pointers; out receives na + nb
+ * into one CUDA graph; running the plan is one graph launch.  Classes from
+ * 2^14 32-bit digits get launches of their own on parallel graph branches; the
+ * shorter ones, when there are several lengths, share one launch per NTT pass
+ * (four kernel nodes holding every class's blocks, the small products riding
+ * in two of them).  With BGPU_BATCH_PER_CLASS every class gets its own
+ * launches.  Pointers are device pointers; out receives na + nb
  * limbs; a == b with na == nb squares.  A plan is bound to the pointers it
  * was made with (rebuild it for new buffers). */
 typedef struct bgpu_product {
@@ -307,7 +309,9 @@ int bgpu_product_tree_u64(const uint64_t* leaves, size_t n, uint64_t* out, size_
  * oracle at small sizes; 0 restores the default. */
 int bgpu_set_block_limbs(uint64_t limbs);
 
-/* Transform split used for 2^log2_points-point products: the column pass
+/* Transform split used for products of 2^log2_points 32-bit digits (a wide-digit
+ * transform of 2^(log2_points - 1) points takes it where its kernels are built; up
+ * to 2^12 points it has no split): the column pass
  * length 2^log2_column (the row pass gets the rest).  Set by the autotuner
  * (bigint_b200/autotune.py); log2_column = 0 restores the built-in choice.
  * No reference counterpart (the reference has one radix-2 schedule,
