@@ -218,9 +218,12 @@ __device__ __forceinline__ OperandDesc wide_operand(const WideFwdArgs& fa, uint3
 
 // CTAs per SM (register caps): 1024 threads' worth of 64 registers, except
 // columns of 2^9 rows at 1280 (2^19 points of a batch: 15.0 + 5.7 us; at 1024
-// 15.5 + 6.2, at 2048 15.1 + 5.9) and the inverse pass's tiles of 2^11 rows.
+// 15.5 + 6.2, at 2048 15.1 + 5.9), of 2^8 rows nine CTAs, which hold the 1280 CTAs
+// of a 2^19-point inverse pass in one wave (with the same for rows of 2^11 points
+// a product of 2^19 points 47.6 -> 46.2 us, at ten 47.2; 2^20 points 88.0 -> 87.8),
+// and the inverse pass's tiles of 2^11 rows.
 __host__ __device__ constexpr int wide_col_blocks(int l2, bool fwd) {
-    return l2 == 9 ? 5 : l2 == 11 && !fwd ? 3 : 1024 / wide_col_threads(l2, fwd);
+    return l2 == 8 ? 9 : l2 == 9 ? 5 : l2 == 11 && !fwd ? 3 : 1024 / wide_col_threads(l2, fwd);
 }
 
 template <bool LAZY, int L2, int T, int NP>
@@ -276,10 +279,10 @@ __global__ void __launch_bounds__(T, wide_col_blocks(L2, true)) k_wide_fwd(const
 
 // CTAs per SM: 1024 threads' worth of 64 registers; rows of 2^8 points, which
 // spill there, five CTAs of 128 threads (14.1 -> 12.7 us per 2^19 points), of 2^9
-// points six, of 2^14 points three of 80 registers (1407 us at 2^25 points; two
+// points six, of 2^11 points nine (as the columns above), of 2^14 points three of 80 registers (1407 us at 2^25 points; two
 // of 512 threads 1488).
 __host__ __device__ constexpr int wide_row_blocks(int l1) {
-    return l1 == 8 ? 5 : l1 == 9 ? 6 : l1 == 13 ? 4 : l1 == 14 ? 3 : 1024 / (wide_row_threads(l1) * wide_rows_per_cta(l1));
+    return l1 == 8 ? 5 : l1 == 9 ? 6 : l1 == 11 ? 9 : l1 == 13 ? 4 : l1 == 14 ? 3 : 1024 / (wide_row_threads(l1) * wide_rows_per_cta(l1));
 }
 
 template <bool LAZY, int L1, bool SQR>
