@@ -32,8 +32,10 @@ namespace bgpu {
 // take the five-prime kernels: their launches fill the GPU on their own (4096
 // products of 2^10..2^22 bits: 10.60 ms with every class in the mixed-length
 // launches, 6.41 ms so, 6.49 with the long classes one after another instead of
-// on graph branches).  Shorter ones do when they cannot share the mixed-length
-// launches, which are one launch per pass for any number of lengths.
+// on graph branches).  Shorter ones do beside them (4096 products as above 5.35
+// -> 4.83 ms, 64 of 2^10..2^18 bits 73.9 -> 42.0 us, 512 of 2^10..2^22 bits 718 ->
+// 634 us) and alone; several short lengths without a long one share the
+// mixed-length launches, one per pass.
 constexpr int kBatchWideLog32 = 14;
 // Products of a five-prime class that 80- or 96-bit digits hold in half the
 // points run there, on branches of their own, when they have this many points
@@ -276,7 +278,8 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
 #endif
     while (p->first_mixed < p->classes.size() && p->classes[p->first_mixed].log_n >= kBatchWideLog32) ++p->first_mixed;
     const size_t nshort = p->classes.size() - p->first_mixed;
-    p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && nshort >= 2 && nshort <= (size_t)kMaxMixedClasses;
+    p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && p->first_mixed == 0 && nshort >= 2 &&
+               nshort <= (size_t)kMaxMixedClasses;
     for (size_t i = p->first_mixed; i < p->classes.size(); ++i)
         p->mixed = p->mixed && mixed_class_ok(p->classes[i].log_n, p->classes[i].square);
     split_wide_classes(p, prods);

@@ -82,7 +82,7 @@ struct Engine {
     // optional per-kernel timing of NTT products: a ring of event sets, one
     // set per product, read back (and averaged) without per-product syncs
     bool kernel_timing = false;
-    int timed_wide = 0;  // the last product timed: 0 three primes, 1 and 2 the wide-digit kernels, short transforms' ones
+    int timed_wide = 0;  // the last product timed: 0 three primes, 1 wide digits, 2 a short transform of them
     std::vector<cudaEvent_t> kev;  // kTimingRing * (kNttLaunches + 1)
     uint64_t kev_count = 0;
     // operand block of products beyond the largest transform (a power of

@@ -259,12 +259,12 @@ int bgpu_kernel_times(const char** names, float* mean_ms, int cap, uint32_t* npr
  * step.  A plan groups a batch by size (schoolbook below
  * BGPU_SCHOOLBOOK_MAX_LIMBS, Karatsuba, then one NTT class per transform
  * length), allocates its scratch once and captures every launch of the batch
- * into one CUDA graph; running the plan is one graph launch.  Classes from
- * 2^14 32-bit digits get launches of their own on parallel graph branches; the
- * shorter ones, when there are several lengths, share one launch per NTT pass
+ * into one CUDA graph; running the plan is one graph launch.  Every class gets
+ * launches of its own on parallel graph branches, except that several classes
+ * below 2^14 32-bit digits with none above share one launch per NTT pass
  * (four kernel nodes holding every class's blocks, the small products riding
- * in two of them).  With BGPU_BATCH_PER_CLASS every class gets its own
- * launches.  Pointers are device pointers; out receives na + nb
+ * in two of them).  With BGPU_BATCH_PER_CLASS these get their own launches
+ * too.  Pointers are device pointers; out receives na + nb
  * limbs; a == b with na == nb squares.  A plan is bound to the pointers it
  * was made with (rebuild it for new buffers). */
 typedef struct bgpu_product {
