@@ -45,6 +45,7 @@ struct Engine {
     uint32_t* d_err = nullptr;
     unsigned long long* d_ticket = nullptr;
     uint64_t ticket_base = 0, epoch = 0;
+    uint64_t* d_flags = nullptr;  // kFlagWords block flags of the carry scans
     // device I/O buffers of the host API
     void* d_io = nullptr;
     size_t io_bytes = 0;
@@ -92,6 +93,13 @@ struct Engine {
 
 constexpr uint64_t kTimingRing = 1024;  // products whose kernel times are kept
 
+// Block flags of the engine's carry scans: one for every 1024 limbs of the
+// longest product (2^25 limbs, a little more as Digits), or one a product of a
+// group of equal ones.  They have memory of their own, cleared once: a flag
+// is valid by its epoch, and in memory that products use for anything else
+// a residue or a coefficient could hold the value of one.
+constexpr size_t kFlagWords = (size_t)1 << 16;
+
 Engine g;
 std::mutex g_mu;
 Tuning g_tuning;
@@ -119,6 +127,7 @@ void release_locked() {
     cudaFree(g.d_pv);
     cudaFree(g.d_err);
     cudaFree(g.d_ticket);
+    cudaFree(g.d_flags);
     cudaFree(g.d_io);
     cudaFree(g.tree.ptr);
     for (auto p : g.rs) cudaFree(p);
@@ -180,6 +189,9 @@ int init_locked(int device) {
     if (rc == BGPU_OK) rc = cuda_status(cudaMemset(g.d_err, 0, sizeof(uint32_t)));
     if (rc == BGPU_OK) rc = cuda_status(cudaMalloc(&g.d_ticket, sizeof(unsigned long long)));
     if (rc == BGPU_OK) rc = cuda_status(cudaMemset(g.d_ticket, 0, sizeof(unsigned long long)));
+    if (rc == BGPU_OK) rc = cuda_status(cudaMalloc(&g.d_flags, kFlagWords * 8));
+    if (rc == BGPU_OK) rc = cuda_status(cudaMemset(g.d_flags, 0, kFlagWords * 8));
+    if (rc == BGPU_OK) rc = cuda_status(cudaStreamSynchronize(nullptr));  // the clearing above, before any other stream
     if (rc == BGPU_OK) rc = cuda_status(cudaEventCreate(&g.ev0));
     if (rc == BGPU_OK) rc = cuda_status(cudaEventCreate(&g.ev1));
     if (rc != BGPU_OK) {
@@ -222,14 +234,14 @@ int prepare_scratch(int log_n, bool square, ProductScratch* s) {
     const size_t y_bytes = align256((square ? 1 : 2) * (size_t)kNumPrimes * nn * 4);
     const size_t ch_bytes = align256(nn / 2 * 8);
     const size_t sp_bytes = align256(nn / 8 * 8);
-    const size_t fl_bytes = align256((size_t)carry_blocks_narrow((uint32_t)(nn / 8)) * 8);  // either shape
-    int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + ch_bytes + sp_bytes + fl_bytes);
+    if (carry_blocks_narrow((uint32_t)(nn / 8)) > kFlagWords) return BGPU_ERR_CAPACITY;  // either shape
+    int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + ch_bytes + sp_bytes);
     if (rc != BGPU_OK) return rc;
     char* b = static_cast<char*>(g.d_scratch);
     s->y = reinterpret_cast<uint32_t*>(b);
     s->chunks = reinterpret_cast<uint64_t*>(b + y_bytes);
     s->spill = reinterpret_cast<uint64_t*>(b + y_bytes + ch_bytes);
-    s->flags = reinterpret_cast<uint64_t*>(b + y_bytes + ch_bytes + sp_bytes);
+    s->flags = g.d_flags;
     s->ticket = g.d_ticket;
     s->err = g.d_err;
     return BGPU_OK;
@@ -240,14 +252,14 @@ int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, WideF
                   size_t out_cap, cudaStream_t st, bgpu_stats* stats) {
     const size_t nn = (size_t)1 << f.log_n;
     const uint32_t bpp = wide_carry_blocks(f.np, out_cap, out_fmt);
-    const size_t y_bytes = align256((square ? 1 : 2) * (size_t)f.np * nn * 4);
-    int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + align256((size_t)bpp * 8));
+    if (bpp > kFlagWords) return BGPU_ERR_CAPACITY;
+    int rc = ensure(&g.d_scratch, &g.scratch_bytes, align256((square ? 1 : 2) * (size_t)f.np * nn * 4));
     if (rc != BGPU_OK) return rc;
     ProductDesc one{};
     one.op[0] = a;
     one.op[1] = square ? a : b;
     one.y = static_cast<uint32_t*>(g.d_scratch);
-    one.flags = reinterpret_cast<uint64_t*>(static_cast<char*>(g.d_scratch) + y_bytes);
+    one.flags = g.d_flags;
     one.out = out;
     one.out_cap = out_cap;
     CarryLaunch cl;
@@ -282,10 +294,11 @@ constexpr uint64_t kWideGroupPoints = 1u << 21;
 int multiply_wide_many(WideForm f, const bgpu_product* pr, size_t count, cudaStream_t st, uint32_t* launches) {
     const size_t na = pr[0].na, nb = pr[0].nb;
     const uint32_t bpp = wide_carry_blocks(f.np, na + nb, kFmtLimb64);
-    const size_t y_bytes = 2 * (size_t)f.np * ((size_t)4 << f.log_n), fl_bytes = (size_t)bpp * 8;
+    const size_t y_bytes = 2 * (size_t)f.np * ((size_t)4 << f.log_n);
+    if (bpp > kFlagWords) return BGPU_ERR_CAPACITY;
     const size_t group = std::min<size_t>(
-        {count, kWidePiece, std::max<uint64_t>(1, kWideGroupPoints >> f.log_n)});
-    int rc = ensure(&g.d_scratch, &g.scratch_bytes, group * y_bytes + align256(group * fl_bytes));
+        {count, kWidePiece, std::max<uint64_t>(1, kWideGroupPoints >> f.log_n), kFlagWords / bpp});
+    int rc = ensure(&g.d_scratch, &g.scratch_bytes, group * y_bytes);
     if (rc != BGPU_OK) return rc;
     auto apart = [&](const void* x, const void* y) { return static_cast<const char*>(x) - static_cast<const char*>(y); };
     WideStep step;
@@ -300,7 +313,7 @@ int multiply_wide_many(WideForm f, const bgpu_product* pr, size_t count, cudaStr
         one.op[0] = OperandDesc{pr[done].a, (uint32_t)na, (uint32_t)(2 * na), kFmtLimb64};
         one.op[1] = OperandDesc{pr[done].b, (uint32_t)nb, (uint32_t)(2 * nb), kFmtLimb64};
         one.y = static_cast<uint32_t*>(g.d_scratch);
-        one.flags = reinterpret_cast<uint64_t*>(static_cast<char*>(g.d_scratch) + group * y_bytes);
+        one.flags = g.d_flags;
         one.out = pr[done].out;
         one.out_cap = na + nb;
         CarryLaunch cl;
@@ -336,8 +349,8 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     CarryLaunch cl;
     cl.ticket_base = g.ticket_base;
     cl.epoch = ++g.epoch;
-    // The scratch layout (residue planes first, then the chunk sums, spills
-    // and flags the carry scan reads) depends on the length and on squaring:
+    // The scratch layout (residue planes first, then the chunk sums and spills
+    // the carry scan reads) depends on the length and on squaring:
     // only an identical layout keeps this forward pass's planes clear of the
     // previous product's carry data while that scan still runs.
     cl.overlap_prev = overlap_prev && st == g.ntt_stream && ln == g.ntt_log_n && square == g.ntt_square;
@@ -633,8 +646,8 @@ int fft_product_locked(const uint64_t* da, size_t na, const uint64_t* db, size_t
     const uint32_t nchunks = (uint32_t)((uint64_t)bits * nn / 256);
     const size_t y_bytes = align256(nn * sizeof(double2)), co_bytes = align256(nn * 8);
     const size_t ch_bytes = align256((size_t)nchunks * 32), sp_bytes = align256((size_t)nchunks * 8);
-    const size_t fl_bytes = align256((size_t)carry_blocks(nchunks) * 8);
-    int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + co_bytes + ch_bytes + sp_bytes + fl_bytes);
+    if (carry_blocks(nchunks) > kFlagWords) return BGPU_ERR_CAPACITY;
+    int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + co_bytes + ch_bytes + sp_bytes);
     if (rc != BGPU_OK) return rc;
     char* base = static_cast<char*>(g.d_scratch);
     FftScratch fs{};
@@ -645,7 +658,7 @@ int fft_product_locked(const uint64_t* da, size_t na, const uint64_t* db, size_t
     fs.maxerr = g.d_fft_err;
     fs.nchunks = nchunks;
     ProductScratch ps{};
-    ps.flags = reinterpret_cast<uint64_t*>(base + y_bytes + co_bytes + ch_bytes + sp_bytes);
+    ps.flags = g.d_flags;
     ps.ticket = g.d_ticket;
     ps.err = g.d_err;
     cudaError_t e = cudaMemsetAsync(g.d_fft_err, 0, sizeof(unsigned long long), st);
