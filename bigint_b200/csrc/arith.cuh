@@ -43,7 +43,9 @@ constexpr int kNumSets = 8;
 constexpr int kFirstWideSet = 2;
 constexpr int kMaxLogN = 26;    // largest transform overall (set 1)
 constexpr int kLazyMaxLogN = 23;  // largest transform of set 0
-constexpr int kMaxLogRow = 15;  // stage tables cover pair distances h < 2^15
+constexpr int kMaxLogRow = 15;      // longest row of sets 0 and 1: their stage tables cover pair distances h <= 2^14
+constexpr int kMaxLogWideRow = 14;  // of the wide sets
+constexpr int stage_log_of(int set) { return set < kFirstWideSet ? kMaxLogRow : kMaxLogWideRow; }
 
 constexpr int kWideLazyMaxLogN = 22;  // largest transform of set 2
 constexpr int kWideMaxLogN = 25;      // of set 3

@@ -16,6 +16,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "../../include/bigint_b200.h"
@@ -148,15 +149,17 @@ void release_locked() {
 
 int build_tables_locked() {
     for (int ps = 0; ps < kNumSets; ++ps) {
-        std::vector<uint2> host(table_entries(ps, kMaxLogRow));
-        build_tables(ps, kMaxLogRow, host.data());
-        cudaError_t e = cudaMalloc(&g.d_tables[ps], host.size() * sizeof(uint2));
+        const int stage_log = stage_log_of(ps);
+        const std::unique_ptr<uint2[]> host(new (std::nothrow) uint2[table_entries(ps, stage_log)]);
+        if (!host) return BGPU_ERR_OOM;
+        build_tables(ps, stage_log, host.get());
+        const size_t bytes = table_entries(ps, stage_log) * sizeof(uint2);
+        cudaError_t e = cudaMalloc(&g.d_tables[ps], bytes);
         if (e != cudaSuccess) return cuda_status(e);
-        e = cudaMemcpy(g.d_tables[ps], host.data(), host.size() * sizeof(uint2),
-                       cudaMemcpyHostToDevice);
+        e = cudaMemcpy(g.d_tables[ps], host.get(), bytes, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cuda_status(e);
-        g.consts[ps] = make_consts(ps, kMaxLogRow, static_cast<const uint2*>(g.d_tables[ps]));
-        e = ps < 2 ? upload_consts(kSlotEngine + ps, g.consts[ps]) : upload_wide_consts(ps, g.consts[ps]);
+        g.consts[ps] = make_consts(ps, stage_log, static_cast<const uint2*>(g.d_tables[ps]));
+        e = ps < kFirstWideSet ? upload_consts(kSlotEngine + ps, g.consts[ps]) : upload_wide_consts(ps, g.consts[ps]);
         if (e != cudaSuccess) return cuda_status(e);
     }
     std::vector<double2> fh(2 * fft_table_block());

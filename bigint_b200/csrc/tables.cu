@@ -23,15 +23,38 @@ uint32_t inv32(uint32_t p) {  // p^-1 mod 2^32, p odd (Newton iteration)
     return x;
 }
 
-uint2 shoup_pair(uint64_t v, uint32_t p) {
-    const uint32_t w = (uint32_t)(v % p);
-    return make_uint2(w, (uint32_t)(((uint64_t)w << 32) / p));
-}
+// Arithmetic modulo p < 2^31 without divisions: three 64-bit ones an entry, over
+// the 42 primes of all sets, took most of the library's initialisation (42 ms on
+// the host of a B200; six primes took 5 ms).
+struct Mod {
+    uint32_t p, inv;  // p^-1 mod 2^32
+    uint64_t m;       // floor(2^64 / p)
+    explicit Mod(uint32_t prime) : p(prime), inv(inv32(prime)), m(~0ull / prime) {}
+    // floor(w 2^32 / p) for w < p, and the remainder: the estimate from m is at
+    // most one too small.
+    uint32_t quotient(uint32_t w, uint32_t* rem) const {
+        uint32_t q = (uint32_t)(((uint64_t)w * m) >> 32);
+        uint64_t r = ((uint64_t)w << 32) - (uint64_t)q * p;
+        if (r >= p) r -= p, ++q;
+        *rem = (uint32_t)r;
+        return q;
+    }
+    uint2 shoup(uint32_t w) const {  // w < p
+        uint32_t r;
+        return make_uint2(w, quotient(w, &r));
+    }
+    uint2 mont(uint32_t w) const {  // w < p
+        uint32_t r;
+        quotient(w, &r);
+        return make_uint2(r, r * inv);
+    }
+    uint32_t mul(uint32_t v, uint2 s) const {  // v s for a Shoup pair s, v < p
+        const uint32_t r = v * s.x - (uint32_t)(((uint64_t)v * s.y) >> 32) * p;
+        return r >= p ? r - p : r;
+    }
+};
 
-uint2 mont_pair(uint64_t v, uint32_t p) {
-    const uint32_t w = (uint32_t)(((v % p) << 32) % p);
-    return make_uint2(w, w * inv32(p));
-}
+uint2 mont_pair(uint64_t v, uint32_t p) { return Mod(p).mont((uint32_t)(v % p)); }
 
 }  // namespace
 
@@ -42,53 +65,55 @@ void build_tables(int ps, int stage_log, uint2* host) {
     const size_t blk = table_block_entries(ps, stage_log);
     for (int q = 0; q < s.np; ++q) {
         const uint32_t p = s.p[q];
+        const Mod f(p);
         for (int dir = 0; dir < 2; ++dir) {
             uint2* base = host + (size_t)(q * 2 + dir) * blk;
-            base[0] = shoup_pair(1, p);
-            for (size_t h = 1; h < stage_n; h <<= 1) {
-                uint64_t root = pow_mod(s.g[q], (p - 1) / (2 * h), p);
-                if (dir) root = pow_mod(root, p - 2, p);
-                uint64_t v = 1;
-                for (size_t m = 0; m < h; ++m) {
-                    base[h + m] = shoup_pair(v, p);
-                    v = v * root % p;
-                }
-            }
-            uint64_t r = pow_mod(s.g[q], (p - 1) >> s.log_max, p);
-            if (dir) r = pow_mod(r, p - 2, p);
+            auto root_of = [&](int log_order) {  // omega_{2^log_order}^(+-1)
+                const uint64_t r = pow_mod(s.g[q], (p - 1) >> log_order, p);
+                return (uint32_t)(dir ? pow_mod(r, p - 2, p) : r);
+            };
+            // the longest stage; the others are its even entries
+            const size_t top = stage_n / 2;
+            const uint2 root = f.shoup(root_of(stage_log));
+            uint32_t v = 1;
+            for (size_t m = 0; m < top; ++m, v = f.mul(v, root)) base[top + m] = f.shoup(v);
+            for (size_t h = top / 2; h >= 1; h /= 2)
+                for (size_t m = 0; m < h; ++m) base[h + m] = base[2 * (h + m)];
+            base[0] = base[1];
+            const uint32_t r = root_of(s.log_max);
             uint2* th = base + stage_n;
             uint2* tl = th + th_n;
-            const uint64_t step_hi = pow_mod(r, tl_n, p);
-            uint64_t v = 1;
-            for (size_t i = 0; i < th_n; ++i, v = v * step_hi % p) th[i] = mont_pair(v, p);
+            const uint2 step_lo = f.shoup(r), step_hi = f.shoup((uint32_t)pow_mod(r, tl_n, p));
             v = 1;
-            for (size_t i = 0; i < tl_n; ++i, v = v * r % p) tl[i] = mont_pair(v, p);
+            for (size_t i = 0; i < th_n; ++i, v = f.mul(v, step_hi)) th[i] = f.mont(v);
+            v = 1;
+            for (size_t i = 0; i < tl_n; ++i, v = f.mul(v, step_lo)) tl[i] = f.mont(v);
         }
     }
 }
 
-// exp(sign * 2 pi i * num / den) rounded from long double.
-static double2 root_of_unity(uint64_t num, uint64_t den, int sign) {
+// exp(-2 pi i num / den) rounded from long double.
+static double2 root_of_unity(uint64_t num, uint64_t den) {
     const long double pi = 3.141592653589793238462643383279502884L;
     const long double ang = 2.0L * pi * (long double)num / (long double)den;
-    return make_double2((double)cosl(ang), (double)(sign * sinl(ang)));
+    return make_double2((double)cosl(ang), -(double)sinl(ang));
 }
 
 void build_fft_tables(double2* host) {
     const size_t stage_n = (size_t)1 << kFftStageLog;
     const size_t th_n = (size_t)1 << (kFftTwLog - kFftTwSplit), tl_n = (size_t)1 << kFftTwSplit;
-    for (int dir = 0; dir < 2; ++dir) {
-        const int sign = dir ? 1 : -1;  // forward uses exp(-2 pi i / N)
-        double2* base = host + (size_t)dir * fft_table_block();
-        base[0] = make_double2(1.0, 0.0);
-        for (size_t h = 1; h < stage_n; h <<= 1)
-            for (size_t m = 0; m < h; ++m) base[h + m] = root_of_unity(m, 2 * h, sign);
-        double2* th = base + stage_n;
-        double2* tl = th + th_n;
-        const uint64_t full = (uint64_t)1 << kFftTwLog;
-        for (size_t i = 0; i < th_n; ++i) th[i] = root_of_unity((uint64_t)i << kFftTwSplit, full, sign);
-        for (size_t i = 0; i < tl_n; ++i) tl[i] = root_of_unity(i, full, sign);
-    }
+    double2* stage = host;
+    stage[0] = make_double2(1.0, 0.0);
+    for (size_t h = 1; h < stage_n; h <<= 1)
+        for (size_t m = 0; m < h; ++m) stage[h + m] = root_of_unity(m, 2 * h);
+    double2* th = stage + stage_n;
+    double2* tl = th + th_n;
+    const uint64_t full = (uint64_t)1 << kFftTwLog;
+    for (size_t i = 0; i < th_n; ++i) th[i] = root_of_unity((uint64_t)i << kFftTwSplit, full);
+    for (size_t i = 0; i < tl_n; ++i) tl[i] = root_of_unity(i, full);
+    double2* inverse = host + fft_table_block();  // the conjugates
+    inverse[0] = host[0];
+    for (size_t i = 1; i < fft_table_block(); ++i) inverse[i] = make_double2(host[i].x, -host[i].y);
 }
 
 FftConsts make_fft_consts(const double2* dev_tables) {

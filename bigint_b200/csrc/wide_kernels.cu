@@ -877,6 +877,7 @@ cudaError_t dispatch_cols(int l2, bool fwd, const WideFwdArgs& a, uint32_t count
 
 template <bool LAZY, int L1, bool SQR>
 cudaError_t launch_rows_of(const WideArgs& a, uint32_t count, cudaStream_t st) {
+    static_assert(L1 <= kMaxLogWideRow, "stage tables");
     constexpr int RP = wide_rows_per_cta(L1);
     const size_t sm = (size_t)RP * wide_row_words(L1, SQR) * 4;
     auto k = k_wide_rows<LAZY, L1, SQR>;
