@@ -619,7 +619,7 @@ class BatchPlan:
 
 
 def mul_batch_device(products, stream: int = 0, flags: int = 0) -> None:
-    """One-shot batch (create, run, synchronize, destroy)."""
+    """One-shot batch: queued without a graph, and synchronized."""
     _ensure_init()
     arr = (Product * max(1, len(products)))()
     for i, (a, na, b, nb, out) in enumerate(products):

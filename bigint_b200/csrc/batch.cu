@@ -6,10 +6,11 @@
 // fast_pow callers produce many independent products per step
 // (examples/pi.cpp:41-80).  A plan sorts the products of a batch into classes:
 // products small enough for the schoolbook kernel (one CTA each), and NTT
-// classes of equal transform length and squaring flag.  Every class runs as one
-// set of launches with a grid slice per product, on its own branch of a CUDA
-// graph so small classes overlap; the graph is built once per plan and
-// replayed per run.
+// classes of equal transform length, digit width and squaring flag.  Every class
+// runs as one set of launches with a grid slice per product, the classes in turn
+// on the branches of a CUDA graph so that small ones overlap; the graph is built
+// once per plan and replayed per run.  A batch that runs once
+// (batch_plan_launch) goes to the same streams without a graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,11 +44,6 @@ constexpr int kBatchWideLog32 = 14;
 // bits 150 us; a line at 2^13 points 5.46 ms and 154 us, at 2^20 5.49 ms and
 // 166 us); fewer leave the GPU idle while their four launches pass.
 constexpr uint64_t kBatchSplitPoints = 1u << 16;
-// Graph branches of a plan, its classes in turn: each one more is a stream made and
-// dropped while the plan is recorded.  512 products of 2^10..2^20 bits, six branches
-// against one a class: built in 2.0 ms against 3.45, run in 0.31 against 0.29.
-constexpr size_t kBatchBranches = 6;
-
 struct BatchClass {
     int log_n = 0;      // 32-bit digits
     WideForm form;      // wide-digit transform; np == 0: three primes
@@ -142,11 +138,40 @@ void destroy_plan(bgpu_batch_plan_s* p) {
 
 }  // namespace
 
-// Record the plan's work on `st`: reset the carry-scan state, fork one branch
-// per class onto the prepared streams, launch, and join back.
-int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks,
-                 const std::vector<cudaStream_t>& branches, const std::vector<cudaEvent_t>& joins,
-                 cudaEvent_t fork) {
+// The first n branches of the engine's streams and events, made when first needed.
+static int ensure_streams(BatchStreams* s, size_t n) {
+    if (!s->cap && (cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking) != cudaSuccess ||
+                    cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) != cudaSuccess))
+        return BGPU_ERR_CUDA;
+    for (size_t i = 0; i < n; ++i)
+        if (!s->join[i] && (cudaStreamCreateWithFlags(&s->branch[i], cudaStreamNonBlocking) != cudaSuccess ||
+                            cudaEventCreateWithFlags(&s->join[i], cudaEventDisableTiming) != cudaSuccess))
+            return BGPU_ERR_CUDA;
+    return BGPU_OK;
+}
+
+void release_streams(BatchStreams* s) {
+    for (size_t i = 0; i < kBatchBranches; ++i) {
+        if (s->branch[i]) cudaStreamDestroy(s->branch[i]);
+        if (s->join[i]) cudaEventDestroy(s->join[i]);
+    }
+    if (s->cap) cudaStreamDestroy(s->cap);
+    if (s->fork) cudaEventDestroy(s->fork);
+    *s = BatchStreams{};
+}
+
+static size_t plan_branches(const bgpu_batch_plan_s* p) {
+    return std::min(kBatchBranches, p->mixed ? p->first_mixed
+                                             : p->classes.size() + (p->school.empty() ? 0 : 1) + (p->kara.empty() ? 0 : 1));
+}
+
+// Queue (or record, where `st` is capturing) the plan's work on `st`: reset the
+// carry-scan state, fork the classes onto the branch streams, launch, and join back.
+static int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks) {
+    const size_t nbranch = plan_branches(p);
+    const cudaStream_t* branches = hooks.streams->branch;
+    const cudaEvent_t* joins = hooks.streams->join;
+    const cudaEvent_t fork = hooks.streams->fork;
     char* base = static_cast<char*>(p->d_mem);
     const ProductDesc* d_descs = reinterpret_cast<const ProductDesc*>(base);
     size_t n_desc = 0, flag_words = 0;
@@ -163,10 +188,9 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
     const size_t flags_base = tick_off + al256(std::max<size_t>(1, p->classes.size()) * 8);
     // Carry-scan state restarts every run: ticket counters and flag words at 0,
     // epoch 1 baked into the launches.
-    cudaError_t e = cudaMemsetAsync(tickets, 0, std::max<size_t>(1, p->classes.size()) * 8, st);
-    if (e == cudaSuccess && flag_words) e = cudaMemsetAsync(base + flags_base, 0, flag_words * 8, st);
-    if (e == cudaSuccess) e = cudaEventRecord(fork, st);
-    for (size_t i = 0; e == cudaSuccess && i < branches.size(); ++i) e = cudaStreamWaitEvent(branches[i], fork, 0);
+    cudaError_t e = cudaMemsetAsync(tickets, 0, flags_base - tick_off + flag_words * 8, st);
+    if (e == cudaSuccess && nbranch) e = cudaEventRecord(fork, st);
+    for (size_t i = 0; e == cudaSuccess && i < nbranch; ++i) e = cudaStreamWaitEvent(branches[i], fork, 0);
     if (e != cudaSuccess) return BGPU_ERR_CUDA;
     uint32_t launches = 0;
     if (p->mixed) {
@@ -197,26 +221,26 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
         cl.ticket = tickets + ci;
         cl.err = hooks.err;
         e = c.form.np ? launch_wide_batch(c.form, d_descs + c.desc_off, (uint32_t)c.members.size(),
-                                       c.square, kFmtLimb64, c.bpp, cl, branches[ci % branches.size()])
+                                       c.square, kFmtLimb64, c.bpp, cl, branches[ci % nbranch])
                    : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], d_descs + c.desc_off,
-                                      (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci % branches.size()]);
+                                      (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci % nbranch]);
         if (e != cudaSuccess) return BGPU_ERR_CUDA;
         launches += c.form.np ? wide_launches(c.form) : kNttLaunches;
     }
     size_t bi = nbranched;
     if (!p->school.empty() && !p->mixed) {
         const SchoolDesc* d_school = reinterpret_cast<const SchoolDesc*>(base + school_off);
-        if (launch_schoolbook_batch(d_school, (uint32_t)p->school.size(), branches[bi++ % branches.size()]) != cudaSuccess)
+        if (launch_schoolbook_batch(d_school, (uint32_t)p->school.size(), branches[bi++ % nbranch]) != cudaSuccess)
             return BGPU_ERR_CUDA;
         launches += 1;
     }
     if (!p->kara.empty() && !p->mixed) {
         const SchoolDesc* d_kara = reinterpret_cast<const SchoolDesc*>(base + kara_off);
-        if (launch_karatsuba_batch(d_kara, (uint32_t)p->kara.size(), branches[bi++ % branches.size()]) != cudaSuccess)
+        if (launch_karatsuba_batch(d_kara, (uint32_t)p->kara.size(), branches[bi++ % nbranch]) != cudaSuccess)
             return BGPU_ERR_CUDA;
         launches += 1;
     }
-    for (size_t i = 0; i < branches.size(); ++i) {
+    for (size_t i = 0; i < nbranch; ++i) {
         if (cudaEventRecord(joins[i], branches[i]) != cudaSuccess ||
             cudaStreamWaitEvent(st, joins[i], 0) != cudaSuccess)
             return BGPU_ERR_CUDA;
@@ -225,8 +249,9 @@ int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks& hooks
     return BGPU_OK;
 }
 
-int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, int device,
-                      const EngineHooks& hooks, bgpu_batch_plan_s** out) {
+// A plan without its graph: classes, memory and descriptors.
+static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, int device,
+                       const EngineHooks& hooks, bgpu_batch_plan_s** out) {
     auto* p = new (std::nothrow) bgpu_batch_plan_s();
     if (!p) return BGPU_ERR_OOM;
     p->device = device;
@@ -369,45 +394,50 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
         destroy_plan(p);
         return BGPU_ERR_CUDA;
     }
-    // Capture the whole batch into one graph (streams and events made first).
-    const size_t nbranch =
-        std::min(kBatchBranches, p->mixed ? p->first_mixed
-                                          : p->classes.size() + (p->school.empty() ? 0 : 1) + (p->kara.empty() ? 0 : 1));
-    std::vector<cudaStream_t> branches(nbranch, nullptr);
-    std::vector<cudaEvent_t> joins(nbranch, nullptr);
-    cudaStream_t cap = nullptr;
-    cudaEvent_t fork = nullptr;
-    int rc = BGPU_OK;
-    if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess)
+    const int rc = ensure_streams(hooks.streams, plan_branches(p));
+    if (rc != BGPU_OK) {
+        release_streams(hooks.streams);
+        destroy_plan(p);
+        return rc;
+    }
+    *out = p;
+    return BGPU_OK;
+}
+
+int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, int device,
+                      const EngineHooks& hooks, bgpu_batch_plan_s** out) {
+    bgpu_batch_plan_s* p = nullptr;
+    int rc = plan_layout(prods, count, flags, device, hooks, &p);
+    if (rc != BGPU_OK) return rc;
+    // The whole batch as one graph.
+    const cudaStream_t cap = hooks.streams->cap;
+    if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         rc = BGPU_ERR_CUDA;
-    for (size_t i = 0; rc == BGPU_OK && i < nbranch; ++i) {
-        if (cudaStreamCreateWithFlags(&branches[i], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&joins[i], cudaEventDisableTiming) != cudaSuccess)
-            rc = BGPU_ERR_CUDA;
+    } else {
+        rc = batch_record(p, cap, hooks);
+        const cudaError_t ec = cudaStreamEndCapture(cap, &p->graph);
+        if (rc == BGPU_OK && ec != cudaSuccess) rc = BGPU_ERR_CUDA;
     }
-    cudaGraph_t g = nullptr;
-    if (rc == BGPU_OK) {
-        if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-            rc = BGPU_ERR_CUDA;
-        } else {
-            rc = batch_record(p, cap, hooks, branches, joins, fork);
-            const cudaError_t ec = cudaStreamEndCapture(cap, &g);
-            if (rc == BGPU_OK && ec != cudaSuccess) rc = BGPU_ERR_CUDA;
-        }
+    if (rc != BGPU_OK) {
+        cudaGetLastError();
+        release_streams(hooks.streams);  // whatever state the capture left them in
+    } else if (cudaGraphInstantiate(&p->exec, p->graph, 0) != cudaSuccess) {
+        cudaGetLastError();
+        rc = BGPU_ERR_CUDA;
     }
-    for (auto x : branches)
-        if (x) cudaStreamDestroy(x);
-    for (auto x : joins)
-        if (x) cudaEventDestroy(x);
-    if (fork) cudaEventDestroy(fork);
-    if (cap) cudaStreamDestroy(cap);
-    if (rc == BGPU_OK) {
-        p->graph = g;
-        if (cudaGraphInstantiate(&p->exec, g, 0) != cudaSuccess) rc = BGPU_ERR_CUDA;
-    } else if (g) {
-        cudaGraphDestroy(g);
+    if (rc != BGPU_OK) {
+        destroy_plan(p);
+        return rc;
     }
+    *out = p;
+    return BGPU_OK;
+}
+
+int batch_plan_launch(const bgpu_product* prods, size_t count, uint32_t flags, int device, const EngineHooks& hooks,
+                      cudaStream_t st, bgpu_batch_plan_s** out) {
+    bgpu_batch_plan_s* p = nullptr;
+    int rc = plan_layout(prods, count, flags, device, hooks, &p);
+    if (rc == BGPU_OK) rc = batch_record(p, st, hooks);
     if (rc != BGPU_OK) {
         cudaGetLastError();
         destroy_plan(p);

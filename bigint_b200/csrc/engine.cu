@@ -51,6 +51,7 @@ struct Engine {
     void* d_io = nullptr;
     size_t io_bytes = 0;
     TreeArena tree;  // product-tree values, descriptors and scratch
+    BatchStreams batch;
     // digit buffers of the device-resident reciprocal (one per live value)
     uint32_t* rs[23] = {};
     size_t rs_bytes[23] = {};
@@ -131,6 +132,7 @@ void release_locked() {
     cudaFree(g.d_flags);
     cudaFree(g.d_io);
     cudaFree(g.tree.ptr);
+    release_streams(&g.batch);
     for (auto p : g.rs) cudaFree(p);
     if (g.ev0) cudaEventDestroy(g.ev0);
     if (g.ev1) cudaEventDestroy(g.ev1);
@@ -1922,6 +1924,7 @@ static EngineHooks hooks_locked() {
     EngineHooks h{};
     for (int ps = 0; ps < kNumSets; ++ps) h.consts[ps] = g.consts[ps];
     h.err = g.d_err;
+    h.streams = &g.batch;
     return h;
 }
 
@@ -2094,10 +2097,9 @@ static int run_products(const bgpu_product* pr, size_t count, cudaStream_t st, u
         return BGPU_OK;
     }
     bgpu_batch_plan_s* plan = nullptr;
-    int rc = batch_plan_create(pr, count, BGPU_METHOD_AUTO, g.device, hooks_locked(), &plan);
+    int rc = batch_plan_launch(pr, count, BGPU_METHOD_AUTO, g.device, hooks_locked(), st, &plan);
     if (rc != BGPU_OK) return rc;
-    rc = batch_plan_run(plan, st);
-    if (rc == BGPU_OK) rc = cuda_status(cudaStreamSynchronize(st));
+    rc = cuda_status(cudaStreamSynchronize(st));
     *launches += batch_plan_launches(plan);
     batch_plan_destroy(plan);
     return rc;
@@ -2533,11 +2535,18 @@ int bgpu_batch_plan_destroy(bgpu_batch_plan plan) {
 uint32_t bgpu_batch_plan_launches(bgpu_batch_plan plan) { return batch_plan_launches(plan); }
 
 int bgpu_mul_batch_device(const bgpu_product* products, size_t count, uint32_t flags, void* stream) {
+    if (!products && count) return BGPU_ERR_INVALID_ARG;
     bgpu_batch_plan plan = nullptr;
-    int rc = bgpu_batch_plan_create(products, count, flags, &plan);
-    if (rc != BGPU_OK) return rc;
-    rc = bgpu_batch_plan_run(plan, stream);
-    if (rc == BGPU_OK) rc = bgpu_device_status(stream);
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (g.device < 0) return BGPU_ERR_NOT_INIT;
+        cudaSetDevice(g.device);
+        const int rc = batch_plan_launch(products, count, flags, g.device, hooks_locked(),
+                                         static_cast<cudaStream_t>(stream), &plan);
+        if (rc != BGPU_OK) return rc;
+        g.last_launches = batch_plan_launches(plan);
+    }
+    const int rc = bgpu_device_status(stream);
     bgpu_batch_plan_destroy(plan);
     return rc;
 }

@@ -312,9 +312,22 @@ cudaError_t launch_carry(const uint64_t* chunks, const uint64_t* spill, uint32_t
                          cudaStream_t stream);
 
 // ---- batched products (batch.cu) ----
+// Streams and events that plans are recorded with, a branch for their classes
+// in turn.  The engine keeps them: made and dropped with each plan, six branches
+// took 0.9 of the 1.5 ms in which a plan of 64 products of 2^10..2^18 bits was built.
+// A branch costs 50 us where the graph is made and saves where it runs: 2, 4, 6
+// branches 70, 56, 58 us (the plan above), 184, 146, 138 (2^10..2^22 bits), 267, 218,
+// 231 (512 products of 2^10..2^20 bits).
+constexpr size_t kBatchBranches = 4;
+struct BatchStreams {
+    cudaStream_t cap = nullptr, branch[kBatchBranches] = {};
+    cudaEvent_t fork = nullptr, join[kBatchBranches] = {};
+};
+void release_streams(BatchStreams* s);
 struct EngineHooks {
     NttConsts consts[kNumSets];
     uint32_t* err;
+    BatchStreams* streams;
 };
 }  // namespace bgpu
 struct bgpu_batch_plan_s;
@@ -323,6 +336,10 @@ namespace bgpu {
 int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, int device,
                       const EngineHooks& hooks, bgpu_batch_plan_s** out);
 int batch_plan_run(bgpu_batch_plan_s* p, cudaStream_t st);
+// The batch's work queued on `st` once, without a graph; the plan is to be
+// destroyed when it has run.
+int batch_plan_launch(const bgpu_product* prods, size_t count, uint32_t flags, int device, const EngineHooks& hooks,
+                      cudaStream_t st, bgpu_batch_plan_s** out);
 void batch_plan_destroy(bgpu_batch_plan_s* p);
 uint32_t batch_plan_launches(const bgpu_batch_plan_s* p);
 // Device memory the product tree keeps between calls (grow-only).

@@ -285,7 +285,7 @@ int bgpu_batch_plan_run(bgpu_batch_plan plan, void* stream);
 int bgpu_batch_plan_destroy(bgpu_batch_plan plan);
 /* Kernel launches one run of the plan makes (its graph's kernel nodes). */
 uint32_t bgpu_batch_plan_launches(bgpu_batch_plan plan);
-/* One-shot: create, run, synchronize, destroy. */
+/* One-shot: the launches of a plan queued on `stream` without a graph, and synchronized. */
 int bgpu_mul_batch_device(const bgpu_product* products, size_t count, uint32_t flags, void* stream);
 
 /* Pairwise product tree of n u64 values (the binary-splitting pattern of
