@@ -249,9 +249,12 @@ static int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks
     return BGPU_OK;
 }
 
-// A plan without its graph: classes, memory and descriptors.
+// A plan without its graph: classes, memory and descriptors.  The descriptors
+// are copied on `st` (null: the streams' own), which orders them before work
+// queued there; a copy from pageable memory returns before it has arrived, so
+// other streams have to wait for it.
 static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, int device,
-                       const EngineHooks& hooks, bgpu_batch_plan_s** out) {
+                       const EngineHooks& hooks, const cudaStream_t* st, bgpu_batch_plan_s** out) {
     auto* p = new (std::nothrow) bgpu_batch_plan_s();
     if (!p) return BGPU_ERR_OOM;
     p->device = device;
@@ -345,7 +348,9 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
         return BGPU_ERR_OOM;
     }
     char* base = static_cast<char*>(p->d_mem);
-    std::vector<ProductDesc> descs(n_desc);
+    std::vector<uint64_t> host(tick_off / 8);  // all descriptors, one copy
+    auto host_at = [&](size_t off) { return reinterpret_cast<char*>(host.data()) + off; };
+    auto* descs = reinterpret_cast<ProductDesc*>(host_at(0));
     for (auto& c : p->classes) {
         const size_t nn = (size_t)1 << c.log_n;
         const size_t per = ntt_scratch_bytes(c.log_n, c.square, c.form);
@@ -364,41 +369,37 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
             d.out_cap = q.na + q.nb;
         }
     }
-    cudaError_t e = cudaMemcpy(base, descs.data(), n_desc * sizeof(ProductDesc), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && p->mixed) {
+    if (p->mixed) {
         std::vector<MixedClassSpec> spec(nmixed);
         for (size_t i = 0; i < nmixed; ++i) {
             const BatchClass& c = p->classes[p->first_mixed + i];
             spec[i] = MixedClassSpec{reinterpret_cast<const ProductDesc*>(base) + c.desc_off,
                                      (uint32_t)c.members.size(), c.log_n, c.square};
         }
-        std::vector<MixedClass> mc(nmixed);
-        if (mixed_fill(mc.data(), (int)mc.size(), spec.data(), kSlotEngine + 0, hooks.consts[0],
-                       &p->mixed_sizes) != 0) {
+        auto* mc = reinterpret_cast<MixedClass*>(host_at(mixed_off));
+        if (mixed_fill(mc, (int)nmixed, spec.data(), kSlotEngine + 0, hooks.consts[0], &p->mixed_sizes) != 0) {
             destroy_plan(p);
             return BGPU_ERR_INVALID_ARG;
         }
-        for (auto& k : mc) k.inv.err = hooks.err;
-        p->mixed_begin.resize(mc.size());
-        for (size_t i = 0; i < mc.size(); ++i)
+        p->mixed_begin.resize(nmixed);
+        for (size_t i = 0; i < nmixed; ++i) {
+            mc[i].inv.err = hooks.err;
             for (int pass = 0; pass < 4; ++pass) p->mixed_begin[i][pass] = mc[i].begin[pass];
-        e = cudaMemcpy(base + mixed_off, mc.data(), mc.size() * sizeof(MixedClass), cudaMemcpyHostToDevice);
+        }
     }
-    if (e == cudaSuccess && !p->school.empty())
-        e = cudaMemcpy(base + school_off, p->school.data(), p->school.size() * sizeof(SchoolDesc),
-                       cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !p->kara.empty())
-        e = cudaMemcpy(base + kara_off, p->kara.data(), p->kara.size() * sizeof(SchoolDesc),
-                       cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        destroy_plan(p);
-        return BGPU_ERR_CUDA;
-    }
+    if (!p->school.empty()) memcpy(host_at(school_off), p->school.data(), p->school.size() * sizeof(SchoolDesc));
+    if (!p->kara.empty()) memcpy(host_at(kara_off), p->kara.data(), p->kara.size() * sizeof(SchoolDesc));
     const int rc = ensure_streams(hooks.streams, plan_branches(p));
     if (rc != BGPU_OK) {
         release_streams(hooks.streams);
         destroy_plan(p);
         return rc;
+    }
+    if (tick_off && cudaMemcpyAsync(base, host.data(), tick_off, cudaMemcpyHostToDevice,
+                                    st ? *st : hooks.streams->cap) != cudaSuccess) {
+        cudaGetLastError();
+        destroy_plan(p);
+        return BGPU_ERR_CUDA;
     }
     *out = p;
     return BGPU_OK;
@@ -407,10 +408,15 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
 int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, int device,
                       const EngineHooks& hooks, bgpu_batch_plan_s** out) {
     bgpu_batch_plan_s* p = nullptr;
-    int rc = plan_layout(prods, count, flags, device, hooks, &p);
+    int rc = plan_layout(prods, count, flags, device, hooks, nullptr, &p);
     if (rc != BGPU_OK) return rc;
-    // The whole batch as one graph.
     const cudaStream_t cap = hooks.streams->cap;
+    if (cudaStreamSynchronize(cap) != cudaSuccess) {  // the plan may run on any stream
+        cudaGetLastError();
+        destroy_plan(p);
+        return BGPU_ERR_CUDA;
+    }
+    // The whole batch as one graph.
     if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         rc = BGPU_ERR_CUDA;
     } else {
@@ -436,7 +442,7 @@ int batch_plan_create(const bgpu_product* prods, size_t count, uint32_t flags, i
 int batch_plan_launch(const bgpu_product* prods, size_t count, uint32_t flags, int device, const EngineHooks& hooks,
                       cudaStream_t st, bgpu_batch_plan_s** out) {
     bgpu_batch_plan_s* p = nullptr;
-    int rc = plan_layout(prods, count, flags, device, hooks, &p);
+    int rc = plan_layout(prods, count, flags, device, hooks, &st, &p);
     if (rc == BGPU_OK) rc = batch_record(p, st, hooks);
     if (rc != BGPU_OK) {
         cudaGetLastError();

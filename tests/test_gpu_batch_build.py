@@ -52,6 +52,28 @@ def test_one_shot(bb, port, lo, hi):
         check(port, host, dev)
 
 
+def test_one_shot_descriptors_arrive_first(bb, port):
+    """The launches of a one-shot call wait for its descriptors: hundreds of
+    KB from pageable memory, other ones each time, on a stream that does not wait for
+    the legacy default stream."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(SEED + 73)
+    n, count = 3, 16384
+    a = rng.integers(0, 2**64, (count, n), dtype=np.uint64)
+    b = rng.integers(0, 2**64, (count, n), dtype=np.uint64)
+    da, db = (torch.from_numpy(x.view(np.int64)).cuda() for x in (a, b))
+    out = torch.zeros((count, 2 * n), dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    for turn in range(4):  # product i against operand i + turn
+        bb.mul_batch_device([(da.data_ptr() + 8 * n * i, n, db.data_ptr() + 8 * n * ((i + turn) % count), n,
+                              out.data_ptr() + 16 * n * i) for i in range(count)], stream=s.cuda_stream)
+        got = out.cpu().numpy().view(np.uint64)
+        for i in range(0, count, 501):
+            want = port.mul(a[i], b[(i + turn) % count])
+            assert np.array_equal(got[i, : want.size], want) and not got[i, want.size :].any(), (turn, i)
+
+
 def test_one_shot_from_threads_while_plans_are_built(bb, port):
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(SEED + 71)
