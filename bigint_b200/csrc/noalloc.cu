@@ -92,6 +92,8 @@ int setup_device(int dev, DeviceSetup* s) {
     s->consts = make_consts(kNaSet, kNaStageLog, static_cast<const uint2*>(tables));
     if (upload_consts(kSlotNoAlloc + kNaSet, s->consts) != cudaSuccess) return BGPU_ERR_CUDA;
     if (cudaMemset(s->scratch + kOffErr, 0, sizeof(uint32_t)) != cudaSuccess) return BGPU_ERR_CUDA;
+    // the copies and the clearing above, before work on any other stream
+    if (cudaStreamSynchronize(nullptr) != cudaSuccess) return BGPU_ERR_CUDA;
     (void)dev;
     s->ready = true;
     return BGPU_OK;
