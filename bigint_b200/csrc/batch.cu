@@ -281,7 +281,7 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
         }
         int ln = ceil_log2(2 * (uint64_t)(q.na + q.nb) - 1);
         if (ln < 5) ln = 5;
-        if (!shape_supported_batch(ln, square)) {
+        if (ln > kMaxLogN) {
             destroy_plan(p);
             return BGPU_ERR_CAPACITY;
         }
@@ -313,7 +313,7 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
     p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && p->first_mixed == 0 && nshort >= 2 &&
                nshort <= (size_t)kMaxMixedClasses;
     for (size_t i = p->first_mixed; i < p->classes.size(); ++i)
-        p->mixed = p->mixed && mixed_class_ok(p->classes[i].log_n, p->classes[i].square);
+        p->mixed = p->mixed && mixed_class_ok(p->classes[i].log_n);
     split_wide_classes(p, prods);
     // Layout: [ProductDesc...][MixedClass...][SchoolDesc: schoolbook...]
     //         [SchoolDesc: Karatsuba...][tickets][flags][scratch].
@@ -547,7 +547,7 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
         } else {
             L.kind = 3;
             while (((uint64_t)1 << L.log_n) < 4 * (uint64_t)w - 1) ++L.log_n;
-            if (!shape_supported_batch(L.log_n, false)) return BGPU_ERR_CAPACITY;
+            if (L.log_n > kMaxLogN) return BGPU_ERR_CAPACITY;
             if (L.log_n > kWideMinLogN && L.log_n - 1 <= kWideMaxLogN) L.form = {kWidePrimes, L.log_n - 1};
             L.bpp = L.form.np ? wide_carry_blocks(kWidePrimes, 2 * w, kFmtLimb64)
                            : carry_blocks((uint32_t)(((size_t)1 << L.log_n) / 8));

@@ -344,9 +344,9 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     const uint32_t method = flags & BGPU_METHOD_MASK;
     const uint64_t total32 = (uint64_t)a.nd32 + b.nd32;
     const int log_n = ceil_log2(total32 - 1);
-    if (log_n > kMaxLogN || !shape_supported(log_n < 5 ? 5 : log_n, square))
-        return BGPU_ERR_CAPACITY;
-    if (const WideForm f = wide_form(a.nd32, b.nd32, kLongDigitMinLogN); f.np) return multiply_wide(a, b, square, f, out, out_fmt, out_cap, st, stats);
+    if (log_n > kMaxLogN) return BGPU_ERR_CAPACITY;
+    if (const WideForm f = wide_form(a.nd32, b.nd32, kLongDigitMinLogN); f.np)
+        return multiply_wide(a, b, square, f, out, out_fmt, out_cap, st, stats);
     const int ln = log_n < 5 ? 5 : log_n;
     ProductScratch s{};
     int rc = prepare_scratch(ln, square, &s);

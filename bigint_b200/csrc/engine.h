@@ -160,9 +160,11 @@ struct MixedSizes {
     uint32_t blocks[4];  // NTT CTAs of each pass's launch (carry: tickets)
     size_t smem[4];      // dynamic shared memory of each launch's NTT CTAs
 };
+// Split of a class in the mixed launches: the batch split, where they hold it.
+TransformShape mixed_shape(int log_n);
 // A class the mixed launches can run (lazy prime set, column tiles of at most
-// 2^9 rows, rows of at most 2^9 points, at the batch split).
-bool mixed_class_ok(int log_n, bool square);
+// 2^9 rows, rows of at most 2^9 points).
+bool mixed_class_ok(int log_n);
 // Fill the host copy of `nclasses` classes (descs already on the device) and
 // the launch sizes; -1 when a class does not qualify.
 int mixed_fill(MixedClass* classes, int nclasses, const MixedClassSpec* spec, int slot, const NttConsts& c,
@@ -170,14 +172,14 @@ int mixed_fill(MixedClass* classes, int nclasses, const MixedClassSpec* spec, in
 // The four launches of a mixed-length batch on `stream`.
 cudaError_t launch_ntt_mixed(const MixedArgs& m, const MixedSizes& sizes, cudaStream_t stream);
 
-TransformShape choose_shape(int log_n);        // the tuned split (bgpu_set_split), else the built-in one
-TransformShape choose_shape_batch(int log_n);  // batch classes (bgpu_set_batch_split), else built-in
-TransformShape builtin_shape(int log_n);       // the built-in split only
-int tuned_split(int log_n, bool batch);        // the split set by bgpu_set_split or bgpu_set_batch_split, or 0
+// The tuned split (bgpu_set_split; of batch classes bgpu_set_batch_split) where
+// its kernels are built, else the built-in one.
+TransformShape choose_shape(int log_n);
+TransformShape choose_shape_batch(int log_n);
+TransformShape builtin_shape(int log_n);  // the built-in split only
+int tuned_split(int log_n, bool batch);   // the split set by bgpu_set_split or bgpu_set_batch_split, or 0
 int set_split(int log_n, int log_n2);  // 0 on success; log_n2 == 0 restores the default
 int set_batch_split(int log_n, int log_n2);
-bool shape_supported(int log_n, bool square);
-bool shape_supported_batch(int log_n, bool square);
 size_t smem_fwd_cols(int log_n2, int cols);
 size_t smem_mid_rows(int log_n1, bool square);
 size_t smem_inv_cols(int log_n2);

@@ -1041,31 +1041,27 @@ TransformShape builtin_shape(int log_n) {
     return s;
 }
 
-static TransformShape shape_from(const int* table, int log_n) {
-    TransformShape s = builtin_shape(log_n);
-    if (log_n >= 0 && log_n <= kMaxLogN && table[log_n]) {
-        s.log_n2 = table[log_n];
-        s.log_n1 = log_n - s.log_n2;
-    }
-    return s;
-}
-
-TransformShape choose_shape(int log_n) { return shape_from(g_split, log_n); }
-TransformShape choose_shape_batch(int log_n) { return shape_from(g_batch_split, log_n); }
-
-static bool shape_ok(const TransformShape& s, bool square) {
+static bool shape_ok(const TransformShape& s) {
     if (s.log_n < 5 || s.log_n > kMaxLogN) return false;
     if (s.log_n2 < 2 || s.log_n2 > 11) return false;
     if (s.log_n1 < 3 || s.log_n1 > 15) return false;
     // Rows of 2^15 points are built for the strict prime set only (transforms
     // above 2^23 points: spectral sums).
-    if (s.log_n1 == 15 && prime_set_for(s.log_n) == 0) return false;
-    (void)square;
-    return true;
+    return s.log_n1 != 15 || prime_set_for(s.log_n) == 1;
 }
 
-bool shape_supported(int log_n, bool square) { return shape_ok(choose_shape(log_n), square); }
-bool shape_supported_batch(int log_n, bool square) { return shape_ok(choose_shape_batch(log_n), square); }
+// A split may be set for the wide-digit transforms alone: where these kernels
+// are not built for it, the built-in one serves.
+static TransformShape shape_from(const int* table, int log_n) {
+    if (log_n >= 0 && log_n <= kMaxLogN && table[log_n]) {
+        const TransformShape s{log_n, log_n - table[log_n], table[log_n]};
+        if (shape_ok(s)) return s;
+    }
+    return builtin_shape(log_n);
+}
+
+TransformShape choose_shape(int log_n) { return shape_from(g_split, log_n); }
+TransformShape choose_shape_batch(int log_n) { return shape_from(g_batch_split, log_n); }
 
 size_t smem_fwd_cols(int l2, int cols) { return ((size_t)cols * 4 << l2) + cols * 17 * sizeof(uint2); }
 size_t smem_mid_rows(int l1, bool square) {
@@ -1254,7 +1250,7 @@ static cudaError_t launch_ntt_core(int slot, const NttConsts& c, const ProductDe
                                    const TransformShape& sh, int out_fmt, const CarryLaunch& cl,
                                    cudaStream_t st, cudaEvent_t* ev) {
     const int log_n = sh.log_n;
-    if (!shape_ok(sh, square) || log_n > c.log_max || c.log_max != kPrimeSets[0].log_max || count < 1)
+    if (!shape_ok(sh) || log_n > c.log_max || c.log_max != kPrimeSets[0].log_max || count < 1)
         return cudaErrorInvalidValue;
     const uint32_t tiles = (1u << sh.log_n1) / kCols;
     if (ev) cudaEventRecord(ev[0], st);
@@ -1376,7 +1372,7 @@ cudaError_t launch_ntt_batch(int slot, const NttConsts& c, const ProductDesc* de
 
 bool spectral_supported(int log_n) {
     const TransformShape sh = choose_shape(log_n);
-    return shape_ok(sh, false) && spec_rows_built(prime_set_for(log_n), sh.log_n1);
+    return shape_ok(sh) && spec_rows_built(prime_set_for(log_n), sh.log_n1);
 }
 
 cudaError_t launch_ntt_spectrum(int slot, const NttConsts& c, const OperandDesc& a, int log_n, uint32_t* spec,
@@ -1599,10 +1595,15 @@ __global__ void __launch_bounds__(kCarryThreads) k_mixed_carry(const MixedArgs m
                                           m.err);
 }
 
-bool mixed_class_ok(int log_n, bool square) {
-    const TransformShape sh = choose_shape_batch(log_n);
-    return shape_ok(sh, square) && prime_set_for(log_n) == 0 && sh.log_n2 <= 9 && sh.log_n1 <= 9;
+static bool mixed_built(const TransformShape& sh) {
+    return shape_ok(sh) && prime_set_for(sh.log_n) == 0 && sh.log_n2 <= 9 && sh.log_n1 <= 9;
 }
+// The tuned split where the mixed launches hold it, else the built-in one.
+TransformShape mixed_shape(int log_n) {
+    const TransformShape sh = choose_shape_batch(log_n);
+    return mixed_built(sh) ? sh : builtin_shape(log_n);
+}
+bool mixed_class_ok(int log_n) { return mixed_built(mixed_shape(log_n)); }
 
 int mixed_fill(MixedClass* classes, int nclasses, const MixedClassSpec* spec, int slot, const NttConsts& c,
                MixedSizes* sizes) {
@@ -1611,8 +1612,8 @@ int mixed_fill(MixedClass* classes, int nclasses, const MixedClassSpec* spec, in
     size_t sm_fwd = 0, sm_mid = 0, sm_inv = 0;
     for (int i = 0; i < nclasses; ++i) {
         const MixedClassSpec& sp = spec[i];
-        if (!mixed_class_ok(sp.log_n, sp.square)) return -1;
-        const TransformShape sh = choose_shape_batch(sp.log_n);
+        if (!mixed_class_ok(sp.log_n)) return -1;
+        const TransformShape sh = mixed_shape(sp.log_n);
         MixedClass& k = classes[i];
         k = MixedClass{};
         const int nops = sp.square ? 1 : 2;
