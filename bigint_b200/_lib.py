@@ -543,7 +543,7 @@ def set_block_limbs(limbs: int) -> None:
 
 
 def set_split(log2_points: int, log2_column: int) -> None:
-    """Column-pass length 2^log2_column for 2^log2_points-point transforms (0 = default)."""
+    """Column-pass length 2^log2_column for products of 2^log2_points 32-bit digits (0 = default)."""
     _check(lib.bgpu_set_split(int(log2_points), int(log2_column)), "bgpu_set_split")
 
 
@@ -553,6 +553,7 @@ def set_batch_split(log2_points: int, log2_column: int) -> None:
 
 
 def get_batch_split(log2_points: int) -> int:
+    """The column length exponent in use there."""
     r = lib.bgpu_get_batch_split(int(log2_points))
     if r < 0:
         _check(r, "bgpu_get_batch_split")
@@ -560,6 +561,7 @@ def get_batch_split(log2_points: int) -> int:
 
 
 def get_split(log2_points: int) -> int:
+    """The column length exponent a product of that length runs with (0: no split)."""
     r = lib.bgpu_get_split(int(log2_points))
     if r < 0:
         _check(r, "bgpu_get_split")

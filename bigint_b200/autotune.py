@@ -6,10 +6,13 @@ brute up to 16384 total bits, FFT up to ``fft::MAX_TOTAL_BITS``, NTT above)
 and has one radix-2 transform schedule (src/mul/ntt_multithread.cpp:333-379).
 Here each choice is timed on the device:
 
-* transform split: for every transform length 2^L (L = 12..25) the column
-  length 2^c (row length 2^(L-c)) with the shortest device time per product,
-  and separately (L = 10..22) the one with the highest throughput for the
-  NTT classes of batch plans and product-tree levels;
+* transform split: for products of 2^L 32-bit digits (L = 14..25, wide-digit
+  transforms of 2^(L-1) points) the column length 2^c (row length 2^(L-1-c))
+  with the shortest device time per product, and separately (L = 14..22) the one
+  with the highest throughput for the NTT classes of batch plans and
+  product-tree levels; shorter products have no split, but several short
+  lengths of a batch share three-prime launches, whose split (row length
+  2^(L-c)) is timed there (L = 10..13);
 * schoolbook vs Karatsuba vs NTT for single products, and for products
   inside a batch plan (one CTA per schoolbook or Karatsuba product vs a
   batched NTT class);
@@ -57,15 +60,15 @@ def _rand_dev(torch, dev, rng, shape):
     return torch.from_numpy(rng.integers(0, 2**63, shape, dtype=np.int64)).to(dev)
 
 
+FIRST_SPLIT = 14  # products of 2^14 32-bit digits and more have a split
+
+
 def valid_splits(log_n: int) -> list[int]:
-    """Column-length exponents the engine accepts for 2^log_n points (rows of
-    2^15 points exist for transforms above 2^23 points only)."""
-    out = []
-    for l2 in range(2, 12):
-        l1 = log_n - l2
-        if 3 <= l1 <= (15 if log_n > 23 else 14):
-            out.append(l2)
-    return out
+    """Column-length exponents that products of 2^log_n 32-bit digits can run with
+    (below FIRST_SPLIT those of the launches that a batch's short lengths share)."""
+    if log_n < FIRST_SPLIT:
+        return [l2 for l2 in range(2, 10) if 3 <= log_n - l2 <= 9]
+    return [l2 for l2 in range(5, 12) if 5 <= log_n - 1 - l2 <= 14]
 
 
 def tune_splits(bb, torch, dev, stream, log_ns, reps_small=40, reps_large=10):
@@ -107,7 +110,8 @@ def tune_splits(bb, torch, dev, stream, log_ns, reps_small=40, reps_large=10):
 
 def tune_batch_splits(bb, torch, dev, stream, log_ns):
     """Best column-length exponent per transform length for the NTT classes of
-    batch plans: throughput of a batch large enough to fill the GPU."""
+    batch plans: throughput of a batch large enough to fill the GPU.  A short
+    length has one product of another length with it, so that the two share launches."""
     sp = stream.cuda_stream
     res = {}
     for ln in log_ns:
@@ -121,6 +125,11 @@ def tune_batch_splits(bb, torch, dev, stream, log_ns):
         B = _rand_dev(torch, dev, rng, (count, n))
         O = torch.empty((count, 2 * n), dtype=torch.int64, device=dev)
         prods = [(A[i].data_ptr(), n, B[i].data_ptr(), n, O[i].data_ptr()) for i in range(count)]
+        if ln < FIRST_SPLIT:
+            m = 1 << ((ln + 1 if ln + 1 < FIRST_SPLIT else ln - 1) - 2)
+            C, D = _rand_dev(torch, dev, rng, (m,)), _rand_dev(torch, dev, rng, (m,))
+            E = torch.empty(2 * m, dtype=torch.int64, device=dev)
+            prods.append((C.data_ptr(), m, D.data_ptr(), m, E.data_ptr()))
         times = {}
         for l2 in cands:
             bb.set_batch_split(ln, l2)
@@ -260,12 +269,12 @@ def write_table(path: str, device: str, splits, bsplits, small, bsmall, fft, fft
     bsb, bka, bsb_rows = bsmall
     lines = [f"# bigint_b200 tuning table for {device}",
              f"# written by bigint_b200/autotune.py at {datetime.datetime.now(datetime.timezone.utc).isoformat(timespec='seconds')}",
-             "# split <log2 points> <log2 column length>   (device us per product: best / built-in)"]
+             "# split <log2 32-bit digits> <log2 column length>   (device us per product: best / built-in)"]
     for ln in sorted(splits):
         r = splits[ln]
         lines.append(f"split {ln} {r['best']}    # {r['ms'][r['best']] * 1e3:.1f} / "
                      f"{r['ms'].get(r['default'], float('nan')) * 1e3:.1f}")
-    lines.append("# batch_split <log2 points> <log2 column length>   (us per batch of `count` products:"
+    lines.append("# batch_split <log2 32-bit digits> <log2 column length>   (us per batch of `count` products:"
                  " best / built-in)")
     for ln in sorted(bsplits):
         r = bsplits[ln]
@@ -303,7 +312,7 @@ def main(argv=None) -> int:
     dev = torch.device("cuda", args.device)
     torch.cuda.set_device(dev)
     stream = torch.cuda.Stream(dev)
-    log_ns = range(12, 26, 3 if args.quick else 1)
+    log_ns = range(FIRST_SPLIT, 26, 3 if args.quick else 1)
     splits = tune_splits(bb, torch, dev, stream, log_ns)
     for ln, r in splits.items():  # later stages measure with the tuned splits
         bb.set_split(ln, r["best"])

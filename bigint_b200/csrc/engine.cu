@@ -2616,9 +2616,15 @@ int bgpu_set_split(uint32_t log2_points, uint32_t log2_column) {
     return set_split((int)log2_points, (int)log2_column) == 0 ? BGPU_OK : BGPU_ERR_INVALID_ARG;
 }
 
+// Lengths that the wide-digit transforms serve, in half as many points: whole
+// in one block (no split), or by wide_shape.
+static bool wide_whole(int log_n) { return log_n > kWideMinLogN && log_n - 1 <= kWideShortMaxLogN; }
+static bool wide_split(int log_n) { return log_n - 1 > kWideShortMaxLogN && log_n - 1 <= kWideMaxLogN; }
 int bgpu_get_split(uint32_t log2_points) {
     if (log2_points < 5 || log2_points > kMaxLogN) return BGPU_ERR_INVALID_ARG;
-    return choose_shape((int)log2_points).log_n2;
+    std::lock_guard<std::mutex> lk(g_mu);
+    const int ln = (int)log2_points;
+    return wide_whole(ln) ? 0 : wide_split(ln) ? wide_shape(ln - 1, false).log_n2 : choose_shape(ln).log_n2;
 }
 
 int bgpu_set_batch_split(uint32_t log2_points, uint32_t log2_column) {
@@ -2628,7 +2634,10 @@ int bgpu_set_batch_split(uint32_t log2_points, uint32_t log2_column) {
 
 int bgpu_get_batch_split(uint32_t log2_points) {
     if (log2_points < 5 || log2_points > kMaxLogN) return BGPU_ERR_INVALID_ARG;
-    return choose_shape_batch((int)log2_points).log_n2;
+    std::lock_guard<std::mutex> lk(g_mu);
+    const int ln = (int)log2_points;
+    return wide_whole(ln) ? mixed_shape(ln).log_n2
+                          : wide_split(ln) ? wide_shape(ln - 1, true).log_n2 : choose_shape_batch(ln).log_n2;
 }
 
 int bgpu_set_tuning(uint32_t key, uint64_t value) {

@@ -309,18 +309,23 @@ int bgpu_product_tree_u64(const uint64_t* leaves, size_t n, uint64_t* out, size_
  * oracle at small sizes; 0 restores the default. */
 int bgpu_set_block_limbs(uint64_t limbs);
 
-/* Transform split used for products of 2^log2_points 32-bit digits (a wide-digit
- * transform of 2^(log2_points - 1) points takes it where its kernels are built; up
- * to 2^12 points it has no split): the column pass
- * length 2^log2_column (the row pass gets the rest).  Set by the autotuner
- * (bigint_b200/autotune.py); log2_column = 0 restores the built-in choice.
+/* Transform split used for products of 2^log2_points 32-bit digits: the column
+ * pass length 2^log2_column (the row pass gets the rest).  From 2^14 digits on
+ * these are wide-digit transforms of half as many points, whose columns have 2^5 to
+ * 2^11 points and rows 2^5 to 2^14; from 2^9 to 2^13 digits a product has no
+ * split.  The three-prime transforms of the same length (mixed batches, products
+ * beyond the largest transform) take a split that they are built for too.  Set by the autotuner
+ * (bigint_b200/autotune.py); log2_column = 0 restores the built-in choice, and
+ * a transform not built for the split keeps it.
  * No reference counterpart (the reference has one radix-2 schedule,
  * src/mul/ntt_multithread.cpp:333-379). */
 int bgpu_set_split(uint32_t log2_points, uint32_t log2_column);
-/* The column length exponent currently used for 2^log2_points points. */
+/* The column length exponent that a product of 2^log2_points 32-bit digits runs
+ * with now; 0 where it has no split. */
 int bgpu_get_split(uint32_t log2_points);
 /* The same for the NTT classes of batch plans and product-tree levels, which
- * the autotuner sets for throughput rather than single-product latency. */
+ * the autotuner sets for throughput rather than single-product latency.  From
+ * 2^9 to 2^13 digits it is the split of the launches that several lengths share. */
 int bgpu_set_batch_split(uint32_t log2_points, uint32_t log2_column);
 int bgpu_get_batch_split(uint32_t log2_points);
 
