@@ -1,6 +1,6 @@
 """Benchmark: bit-exact big-integer products per second on one B200.
 
-Workload (one step = one product): the plain three-prime NTT multiply of two
+Workload (one step = one product): the plain NTT multiply of two
 2^24-bit operands (262144 x 262144 u64 limbs), seeded uniform random limbs
 with the top bit set -- the size the project's roofline target is stated at.
 Inputs are generated on the host with a fixed seed and are synthetic.
@@ -123,7 +123,7 @@ def cpu_thread_counts() -> list[int]:
 
 
 def workload_name(bits: int) -> str:
-    return (f"plain three-prime NTT multiply, 2^{bits.bit_length() - 1} x 2^{bits.bit_length() - 1}"
+    return (f"plain NTT multiply, 2^{bits.bit_length() - 1} x 2^{bits.bit_length() - 1}"
             f"-bit operands ({bits // 64} x {bits // 64} u64 limbs), seeded uniform random limbs")
 
 
@@ -265,12 +265,31 @@ def measured_peaks() -> tuple[float, str]:
         return 6650.0, "fallback"
 
 
+def digit_bits(np_: int) -> int:
+    """Bits of a digit over np_ primes."""
+    return 16 * (np_ - 1)
+
+
+def wide_form(na: int, nb: int) -> tuple[int, int]:
+    """Primes and log2 points of a single product's transform: the shortest that
+    holds it, over the fewest primes that reach it; more than five primes
+    (digits of 80 and 96 bits) from 2^16 points."""
+    best = (5, 99)
+    for np_, lo, hi in ((5, 8, 25), (6, 16, 24), (7, 16, 23)):
+        bits = digit_bits(np_)
+        ln = (-(-64 * na // bits) + -(-64 * nb // bits) - 2).bit_length()
+        if lo <= ln <= hi and ln < best[1]:
+            best = (np_, ln)
+    return best
+
+
 def kernel_bytes(name: str, na: int, nb: int, log_n: int, square: bool) -> int:
     """Algorithmic global-memory bytes of one launch (minimal reads + writes).
-    `log_n` counts 32-bit digits; the five-prime kernels (k_wide_*) take half
-    as many points of 64-bit digits."""
+    `log_n` counts 32-bit digits; the wide-digit kernels (k_wide_*) have the
+    points and primes of the product's form."""
     n = 1 << log_n
-    s64 = 10 * n  # five primes x u32 on n / 2 points
+    np_, ln = wide_form(na, nb)
+    sw = 4 * np_ << ln  # one operand's residues there
     s32 = 12 * n  # one operand's residues: 3 primes x u32 per point
     ops = 1 if square else 2
     inp = (na + (0 if square else nb)) * 8
@@ -280,10 +299,11 @@ def kernel_bytes(name: str, na: int, nb: int, log_n: int, square: bool) -> int:
         "k_mid_rows": ops * s32 + s32,
         "k_inv_cols": s32 + chunk_bytes,
         "k_carry": chunk_bytes + (na + nb) * 8,
-        "k_wide_fwd": inp + ops * s64,
-        "k_wide_rows": ops * s64 + s64,
-        "k_wide_inv": 2 * s64,
-        "k_wide_carry": s64 + (na + nb) * 8,
+        "k_wide_fwd": inp + ops * sw,
+        "k_wide_rows": ops * sw + sw,
+        "k_wide_inv": 2 * sw,
+        "k_wide_short": inp + sw,
+        "k_wide_carry": sw + (na + nb) * 8,
     }[name]
 
 
@@ -310,51 +330,52 @@ def _bfly_muls(l: int) -> float:
     return (1 << (l - 1)) * stages * 3
 
 
-def source_mul_counts(na: int, nb: int, log_n: int, log_n1: int, log_n2: int, square: bool) -> dict:
-    """32-bit multiply operations per launch of each NTT kernel, counted from
-    the kernels' source (butterflies x 3, Montgomery products x 3, the digit
-    reduction x 2, Garner CRT x 14 per point); the compiler's own instruction
-    choice (address arithmetic, moves on the multiply pipe) is not in it."""
-    n, n1, n2 = 1 << log_n, 1 << log_n1, 1 << log_n2
+def source_mul_counts(na: int, nb: int, log_col: int, square: bool) -> dict:
+    """32-bit multiply operations per launch of each kernel of a product of na
+    and nb limbs with columns of 2^log_col points (0: none), counted from the kernels'
+    source per point and prime: butterflies x 3, Shoup twiddles x 6 in the
+    forward and the row pass, pointwise Montgomery products x 3, two operations for each
+    word or Montgomery reduction of a digit, and one per prime and word of the
+    CRT; the compiler's own instruction choice (address arithmetic, moves on the
+    multiply pipe) is not in it."""
+    np_, log_n = wide_form(na, nb)
+    n = 1 << log_n
     ops = 1 if square else 2
-    half = 2 * 2 * max(na, nb) <= n  # every operand in the lower half: half the digits loaded
-    loads = n // 2 if half else n
-    fwd = ops * 3 * (n1 * _bfly_muls(log_n2) + 2 * loads + 6 * n + 4 * n // 8)
-    r0 = _plan_rounds(log_n1)[0]
-    mid = 3 * (n2 * (ops + 1) * _bfly_muls(log_n1) + 4 * n + 6 * n + 7 * n / (1 << r0))
-    inv = 3 * n1 * _bfly_muls(log_n2) + 14 * n
-    # the five-prime kernels, on n / 2 points with the same column length: digit
-    # reduction 4, Shoup twiddles 6 a point, pointwise Montgomery product 3, CRT 20
-    m, m1 = n // 2, n1 // 2
-    wfwd = ops * 5 * (m1 * _bfly_muls(log_n2) + 4 * (m // 2 if half else m) + 6 * m)
-    wmid = 5 * (n2 * (ops + 1) * _bfly_muls(log_n1 - 1) + 9 * m)
-    winv = 5 * m1 * _bfly_muls(log_n2)
-    return {"k_fwd_cols": fwd, "k_mid_rows": mid, "k_inv_cols": inv, "k_carry": 0.0,
-            "k_wide_fwd": wfwd, "k_wide_rows": wmid, "k_wide_inv": winv, "k_wide_carry": 20.0 * m}
+    half = 2 * -(-64 * max(na, nb) // digit_bits(np_)) <= n  # every operand in the lower half: half the digits loaded
+    digits = {5: 4, 6: 6, 7: 8}[np_] * (n // 2 if half else n)
+    carry = {"k_wide_carry": float(np_ * (np_ - 1) * n)}
+    if not log_col:
+        return {"k_wide_short": np_ * ((ops + 1) * _bfly_muls(log_n) + ops * digits + 6 * n), **carry}
+    rows, cols = 1 << log_col, n >> log_col
+    return {"k_wide_fwd": ops * np_ * (cols * _bfly_muls(log_col) + digits + 6 * n),
+            "k_wide_rows": np_ * (rows * (ops + 1) * _bfly_muls(log_n - log_col) + 9 * n),
+            "k_wide_inv": np_ * cols * _bfly_muls(log_col), **carry}
 
 
-def profiled_pipes() -> dict | None:
+def profiled_pipes(bits: int) -> dict | None:
     """Per-launch pipe counters of the four NTT kernels at 2^24 x 2^24 bits
-    from the committed ncu summary, if any."""
+    from the committed ncu summary, if any (None for other sizes)."""
+    if bits != 1 << 24:
+        return None
     try:
         return json.load(open(os.path.join(ROOT, "profiles", "ntt_2p24_pipes.json")))
     except (OSError, ValueError):
         return None
 
 
-def compute_roofline(kernels_ms: dict, dom: str, prod_ms: float, sm_mhz: float | None, counts: dict) -> dict:
+def compute_roofline(kernels_ms: dict, dom: str, prod_ms: float, sm_mhz: float | None, counts: dict,
+                     prof: dict | None) -> dict:
     """The ceiling that binds the transform passes: the 32-bit multiply pipe
     (fmaheavy: IMAD, IMAD.HI, IMAD.WIDE at 2 warp instructions per SM per
     cycle, the wide and high forms taking two of those slots) and instruction
     issue (4 warp instructions per SM per cycle).  Busy cycles per SM come
     from the committed ncu counters (a clock-independent count); the fraction
     divides them by the cycles of the live time at the sampled SM clock."""
-    prof = profiled_pipes()
     res = {"bound": "int32 multiply pipe (fmaheavy)", "kernel": dom,
            "source_mul_ops_per_launch": counts.get(dom),
            "source_mul_ops_per_product": sum(v for k, v in counts.items() if k in kernels_ms),
            "source_note": "counted from the kernel source: 3 per Shoup butterfly or Montgomery product, "
-                          "2 to 4 per digit reduction, 14 per Garner CRT point, 20 per five-prime CRT point"}
+                          "4 to 8 per digit reduction, 20 (five primes) to 42 (seven) per CRT point"}
     if not prof or dom not in prof or not sm_mhz:
         res["profile"] = None
         return res
@@ -384,8 +405,11 @@ def compute_roofline(kernels_ms: dict, dom: str, prod_ms: float, sm_mhz: float |
     return res
 
 
-def profiled_traffic(kernel: str) -> float | None:
-    """Per-launch DRAM bytes of `kernel` from the committed ncu summary, if any."""
+def profiled_traffic(kernel: str, bits: int) -> float | None:
+    """Per-launch DRAM bytes of `kernel` at 2^24 x 2^24 bits from the committed
+    ncu summary, if any (None for other sizes)."""
+    if bits != 1 << 24:
+        return None
     path = os.path.join(ROOT, "profiles", "ntt_2p24_traffic.json")
     try:
         return float(json.load(open(path))[kernel]["dram_bytes_per_launch"])
@@ -1075,12 +1099,15 @@ def batched_form(bb, torch, device, port, nprod: int = 4096, runs: int = 5, ref_
         if port.mod_m61(a) * port.mod_m61(b) % M != port.mod_m61(c):
             raise SystemExit(f"bench batched: product {i} failed the residue check")
 
-    def one_by_one(_):
+    def one_by_one(_, launched=None):
         for i in range(nprod):
             a_ptr, n_a, b_ptr, n_b, o_ptr = prods[i]
             bb.mul_device(a_ptr, n_a, b_ptr, n_b, o_ptr, stream=sp, method=bb.BGPU_METHOD_NTT)
+            if launched is not None:
+                launched.append(bb.last_launch_count())
     dout.zero_()
-    one_by_one(0)
+    launches_single = []
+    one_by_one(0, launches_single)
     bb.device_status(sp)
     if not np.array_equal(dout.cpu().numpy().view(np.uint64), host):
         raise SystemExit("bench batched: the batch differs from one plain NTT call per product")
@@ -1120,11 +1147,12 @@ def batched_form(bb, torch, device, port, nprod: int = 4096, runs: int = 5, ref_
                         "plan_build_s": t_plan},
             "per_class_launch_sets": {"ms_per_batch": ms_pc, "products_per_s": nprod / (ms_pc * 1e-3),
                                       "launches_per_batch": launches_pc, "speedup": ms_single / ms_pc,
-                                      "note": "BGPU_BATCH_PER_CLASS: every NTT class its own four "
-                                              "launches on parallel graph branches; same outputs"},
+                                      "note": "BGPU_BATCH_PER_CLASS: short lengths too get launches of their "
+                                              "own; the same plan as the default where there is a class "
+                                              "of 2^14 digits or more, as here"},
             "one_plain_ntt_launch_per_product": {"ms": ms_single,
                                                  "products_per_s": nprod / (ms_single * 1e-3),
-                                                 "launches": 4 * nprod},
+                                                 "launches": sum(launches_single)},
             "speedup": ms_single / ms_batch, "verified": verified}
 
 
@@ -1427,7 +1455,9 @@ def run_gpu_arm(args) -> None:
 
     # roofline of the dominant kernel
     log_n = (2 * na + 2 * nb - 2).bit_length()
-    mean_k = dict(ktimes)
+    np_, log_pts = wide_form(na, nb)
+    log_col = bb.get_split(log_pts + 1)  # splits are kept by 32-bit digits
+    mean_k = {k: v for k, v in dict(ktimes).items() if k != "none"}
     dom = max(mean_k, key=mean_k.get)
     dom_bytes = kernel_bytes(dom, na, nb, log_n, square=False)
     peak, peak_kind = measured_peaks()
@@ -1478,27 +1508,26 @@ def run_gpu_arm(args) -> None:
         "warmup": args.warmup, "ms_per_step": prod_ms, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "u32", "data": "synthetic",
         "config": {"workload": workload_name(args.bits), "method": "ntt",
-                   "transform_points": 1 << log_n, "digit_bits": 32,
+                   "transform_points": 1 << log_pts, "digit_bits": digit_bits(np_), "primes": np_,
                    "l2": f"inputs larger than L2: {npairs} distinct operand pairs "
                          f"({npairs * 2 * na * 8 >> 20} MiB) cycled, steps back to back",
                    "parallelism": f"replicas x{world}", "verified": verified,
-                   "pipelining": "independent products (BGPU_INDEPENDENT); launches chained with "
+                   "pipelining": "products back to back on one stream, launches chained with "
                                  "programmatic dependent launch",
-                   "transform": "64-bit digits over five primes, half as many points as 32-bit digits",
                    "timing": f"median of {nwin} windows of exactly K={args.steps} products, each window "
                              "bracketed by barrier + synchronize, CUDA events on the launching stream; "
                              "max over ranks",
                    "windows_ms": {"median": statistics.median(win_ms), "min": min(win_ms),
                                   "max": max(win_ms), "count": nwin},
                    "host_issue_us_per_product": statistics.median(issue) / args.steps * 1e6,
-                   "host_issue_note": "host time to enqueue one product (4 launches through the C-ABI); "
+                   "host_issue_note": f"host time to enqueue one product ({launches_per_step} launches through the C-ABI); "
                                       "below the device time per product, the launches are hidden",
                    "prequeued_us_per_product": None if preq_ms is None else preq_ms / args.steps * 1e3,
                    "prequeued_note": "the same K products with every launch queued before the first one "
                                      "starts (behind a GPU sleep), median of 5 windows: equal to ms_per_step "
                                      "when the timed windows' host launches are hidden"},
         "sequential": {"ms_per_step": seq_ms / args.steps, "value": world * args.steps / (seq_ms * 1e-3),
-                       "note": "the same products without BGPU_INDEPENDENT, each after the previous "
+                       "note": "the same products without BGPU_INDEPENDENT, which their transforms make no use of "
                                f"(median of {len(seq_win)} windows)"},
         "e2e": {"value": world * e2e_steps / e2e_s, "unit": "products/s",
                 "h2d_bytes_per_step": (na + nb) * 8, "d2h_bytes_per_step": (na + nb) * 8,
@@ -1508,15 +1537,15 @@ def run_gpu_arm(args) -> None:
                                 "api": "bgpu_mul_u64, one synchronous call per product"}},
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": profiled_traffic(dom), "algorithmic_bytes": dom_bytes,
+                     "traffic": profiled_traffic(dom, args.bits), "algorithmic_bytes": dom_bytes,
                      "kernel_ms": mean_k[dom], "kernels_ms": mean_k, "kernel_samples": kcount,
                      "kernel_timing": "events between the kernels, second pass of the same K products",
                      "reference_model": {"bytes_per_product": model_b,
                                          "achieved": model_b / (prod_ms * 1e-3) / 1e9,
                                          "frac": model_b / (prod_ms * 1e-3) / 1e9 / peak},
                      "compute": compute_roofline(mean_k, dom, prod_ms, clocks.get("sm_mhz"),
-                                                 source_mul_counts(na, nb, log_n, log_n - bb.get_split(log_n),
-                                                                   bb.get_split(log_n), False))},
+                                                 source_mul_counts(na, nb, log_col, False),
+                                                 profiled_pipes(args.bits))},
         "cpu_baseline": cpu,
         "clocks": clocks,
         "gpu_launches": launches_per_step * args.steps,

@@ -29,6 +29,35 @@ def test_kernel_bytes_sum_for_headline():
     assert tot == 6 * s32 + 2 * (5 << 20) + 2 * (2 * n * 8)
 
 
+@pytest.mark.parametrize("na,nb,form", [(1 << 18, 1 << 18, (5, 19)), (65, 65, (5, 8)), (2048, 2048, (5, 12)),
+                                        (140626, 488041, (6, 19)), (1 << 24, 1 << 24, (5, 25)),
+                                        (49152, 49152, (7, 16)), (49153, 49153, (5, 17)), (3000, 3000, (5, 13))])
+def test_figures_of_the_form_that_runs(na, nb, form):
+    """Bytes and multiplies exist for every kernel a product of the form has, and
+    follow its primes, points and columns."""
+    np_, log_n = form
+    assert bench.wide_form(na, nb) == form
+    plane = 4 * np_ << log_n
+    log32 = (2 * na + 2 * nb - 2).bit_length()
+    if log_n <= 12:
+        assert bench.kernel_bytes("k_wide_short", na, nb, log32, False) == (na + nb) * 8 + plane
+        counts = bench.source_mul_counts(na, nb, 0, False)
+        assert set(counts) == {"k_wide_short", "k_wide_carry"}
+    else:
+        assert bench.kernel_bytes("k_wide_fwd", na, nb, log32, False) == (na + nb) * 8 + 2 * plane
+        assert bench.kernel_bytes("k_wide_rows", na, nb, log32, False) == 3 * plane
+        assert bench.kernel_bytes("k_wide_inv", na, nb, log32, False) == 2 * plane
+        counts = bench.source_mul_counts(na, nb, 6, False)
+        assert set(counts) == {"k_wide_fwd", "k_wide_rows", "k_wide_inv", "k_wide_carry"}
+        assert counts["k_wide_inv"] == np_ * (1 << (log_n - 6)) * bench._bfly_muls(6)
+    assert bench.kernel_bytes("k_wide_carry", na, nb, log32, False) == (na + nb) * 8 + plane
+    assert counts["k_wide_carry"] == np_ * (np_ - 1) << log_n
+
+
+def test_profiled_figures_are_of_their_size():
+    assert bench.profiled_pipes(1 << 20) is None and bench.profiled_traffic("k_wide_rows", 1 << 20) is None
+
+
 def test_pairs_exceed_l2():
     l2 = bench.l2_bytes()
     assert l2 >= 1 << 20
