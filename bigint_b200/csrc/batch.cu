@@ -87,6 +87,11 @@ int ceil_log2(uint64_t x) {
     return l;
 }
 
+// Kernels of `count` products of one class or tree level.
+uint32_t batch_launches(WideForm f, uint32_t count) {
+    return (f.np ? wide_launches(f) : kNttLaunches) * ((count + kBatchPiece - 1) / kBatchPiece);
+}
+
 size_t ntt_scratch_bytes(int log_n, bool square, WideForm f) {
     if (f.np) return al256((square ? 1 : 2) * (size_t)f.np * ((size_t)4 << f.log_n));
     const size_t nn = (size_t)1 << log_n;
@@ -225,7 +230,7 @@ static int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks
                    : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], d_descs + c.desc_off,
                                       (int)c.members.size(), c.square, c.log_n, kFmtLimb64, cl, branches[ci % nbranch]);
         if (e != cudaSuccess) return BGPU_ERR_CUDA;
-        launches += c.form.np ? wide_launches(c.form) : kNttLaunches;
+        launches += batch_launches(c.form, (uint32_t)c.members.size());
     }
     size_t bi = nbranched;
     if (!p->school.empty() && !p->mixed) {
@@ -659,7 +664,7 @@ int product_tree_device(const uint64_t* d_leaves, size_t n, uint64_t* d_out, siz
                            : launch_ntt_batch(kSlotEngine + ps, hooks.consts[ps], pd, (int)L.m2, false, L.log_n,
                                               kFmtLimb64, cl, st);
             }
-            nl += kNttLaunches;
+            nl += batch_launches(L.form, L.m2);
         }
         if (e == cudaSuccess && (L.m & 1)) {
             k_tree_tail<<<1, 256, 0, st>>>(in + (size_t)(L.m - 1) * w, out + (size_t)L.m2 * 2 * w, (uint32_t)w);

@@ -85,7 +85,7 @@ struct Engine {
     // optional per-kernel timing of NTT products: a ring of event sets, one
     // set per product, read back (and averaged) without per-product syncs
     bool kernel_timing = false;
-    int timed_wide = 0;  // the last product timed: 0 three primes, 1 wide digits, 2 a short transform of them
+    int timed_kind = 0;  // of the products in the ring: 0 three primes, 1 wide digits, 2 a short transform of them
     std::vector<cudaEvent_t> kev;  // kTimingRing * (kNttLaunches + 1)
     uint64_t kev_count = 0;
     // operand block of products beyond the largest transform (a power of
@@ -252,6 +252,15 @@ int prepare_scratch(int log_n, bool square, ProductScratch* s) {
     return BGPU_OK;
 }
 
+// Events of the next timed product (null: timing is off).  The ring holds
+// products with the same kernels.
+cudaEvent_t* timing_events(int kind) {
+    if (!g.kernel_timing) return nullptr;
+    if (kind != g.timed_kind) g.kev_count = 0;
+    g.timed_kind = kind;
+    return g.kev.data() + (g.kev_count++ % kTimingRing) * (kNttLaunches + 1);
+}
+
 // Product of two device operands on the wide-digit transform.
 int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, WideForm f, void* out, int out_fmt,
                   size_t out_cap, cudaStream_t st, bgpu_stats* stats) {
@@ -274,12 +283,7 @@ int multiply_wide(const OperandDesc& a, const OperandDesc& b, bool square, WideF
     cl.err = g.d_err;
     g.ticket_base += bpp;
     g.ntt_log_n = -1;  // no forward pass overlaps this product's carry scan
-    cudaEvent_t* ev = nullptr;
-    if (g.kernel_timing) {
-        ev = g.kev.data() + (g.kev_count % kTimingRing) * (kNttLaunches + 1);
-        ++g.kev_count;
-        g.timed_wide = f.log_n <= kWideShortMaxLogN ? 2 : 1;
-    }
+    cudaEvent_t* ev = timing_events(f.log_n <= kWideShortMaxLogN ? 2 : 1);
     const cudaError_t e = launch_wide_product(f, nullptr, one, WideStep{}, 1, square, out_fmt, bpp, cl, st, ev);
     g.last_launches = wide_launches(f);
     if (stats) {
@@ -302,7 +306,7 @@ int multiply_wide_many(WideForm f, const bgpu_product* pr, size_t count, cudaStr
     const size_t y_bytes = 2 * (size_t)f.np * ((size_t)4 << f.log_n);
     if (bpp > kFlagWords) return BGPU_ERR_CAPACITY;
     const size_t group = std::min<size_t>(
-        {count, kWidePiece, std::max<uint64_t>(1, kWideGroupPoints >> f.log_n), kFlagWords / bpp});
+        {count, kBatchPiece, std::max<uint64_t>(1, kWideGroupPoints >> f.log_n), kFlagWords / bpp});
     int rc = ensure(&g.d_scratch, &g.scratch_bytes, group * y_bytes);
     if (rc != BGPU_OK) return rc;
     auto apart = [&](const void* x, const void* y) { return static_cast<const char*>(x) - static_cast<const char*>(y); };
@@ -365,12 +369,7 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     g.ntt_square = square;
     const uint32_t nch = (uint32_t)(((size_t)1 << ln) / 8);
     g.ticket_base += cl.narrow ? carry_blocks_narrow(nch) : carry_blocks(nch);
-    cudaEvent_t* ev = nullptr;
-    if (g.kernel_timing) {
-        ev = g.kev.data() + (g.kev_count % kTimingRing) * (kNttLaunches + 1);
-        ++g.kev_count;
-        g.timed_wide = 0;
-    }
+    cudaEvent_t* ev = timing_events(0);
     const int ps = prime_set_for(ln);
     cudaError_t e = launch_ntt_product(kSlotEngine + ps, g.consts[ps], a, b, square, ln, s, out,
                                        out_fmt, out_cap, cl, st, ev);
@@ -437,6 +436,7 @@ int huge_spectral(const uint64_t* da, size_t na, const uint64_t* db, size_t nb, 
     ProductScratch s{};
     rc = prepare_scratch(ln, true, &s);  // 3 residue planes: the sums' row pass output
     if (rc != BGPU_OK) return rc;
+    uint32_t nl = 0;
     const int slot = kSlotEngine + ps;
     cudaError_t e = cudaMemsetAsync(dout, 0, L * 8, st);
     for (uint64_t i = 0; e == cudaSuccess && i < nspec; ++i) {
@@ -445,6 +445,7 @@ int huge_spectral(const uint64_t* da, size_t na, const uint64_t* db, size_t nb, 
         const uint64_t len = std::min<uint64_t>(S, (from_a ? na : nb) - off);
         const OperandDesc od{(from_a ? da : db) + off, (uint32_t)len, (uint32_t)(2 * len), kFmtLimb64};
         e = launch_ntt_spectrum(slot, g.consts[ps], od, ln, spec(i), st);
+        nl += kSpectrumLaunches;
     }
     if (e != cudaSuccess) return cuda_status(e);
     // (i, j) pairs of output block k in sums of at most tmax; `first`: the
@@ -469,6 +470,7 @@ int huge_spectral(const uint64_t* da, size_t na, const uint64_t* db, size_t nb, 
             const cudaError_t e2 = launch_ntt_spectral_sum(slot, g.consts[ps], sa, sb, n, twice, ln, s, dout + off,
                                                            win, nadd ? dout + off : nullptr, nadd, cl, st);
             if (e2 != cudaSuccess) return e2;
+            nl += kSpectralSumLaunches + (nadd || twice ? 1 : 0);  // and the merge
         }
         return cudaSuccess;
     };
@@ -490,6 +492,7 @@ int huge_spectral(const uint64_t* da, size_t na, const uint64_t* db, size_t nb, 
         if (e == cudaSuccess) e = run_sums(twice, k, true, first);
     }
     g.ntt_log_n = -1;  // no forward pass overlaps the carry scans that end this product
+    g.last_launches = nl;
     return cuda_status(e);
 }
 
@@ -517,6 +520,7 @@ int huge_product(const uint64_t* da, size_t na, const uint64_t* db, size_t nb, u
     uint32_t* cin = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(agg) + acc);
     cudaError_t e = cudaMemsetAsync(dout, 0, L * 8, st);
     if (e != cudaSuccess) return cuda_status(e);
+    uint32_t nl = 0;
     for (uint64_t ia = 0; ia < na; ia += S) {
         for (uint64_t ib = square ? ia : 0; ib < nb; ib += S) {
             const uint64_t la = std::min<uint64_t>(S, na - ia), lb = std::min<uint64_t>(S, nb - ib);
@@ -526,12 +530,15 @@ int huge_product(const uint64_t* da, size_t na, const uint64_t* db, size_t nb, u
             rc = multiply_device(oa, diag ? oa : ob, diag, tmp, kFmtLimb64, la + lb, BGPU_METHOD_AUTO, st,
                                  nullptr);
             if (rc != BGPU_OK) return rc;
+            nl += g.last_launches;
             for (int twice = 0; twice < (square && !diag ? 2 : 1); ++twice) {
                 e = launch_accumulate(dout + ia + ib, L - (ia + ib), tmp, la + lb, agg, cin, st);
                 if (e != cudaSuccess) return cuda_status(e);
+                nl += kAccumulateLaunches;
             }
         }
     }
+    g.last_launches = nl;
     return BGPU_OK;
 }
 
@@ -724,7 +731,9 @@ int mul_u64_locked(const uint64_t* a, size_t na, const uint64_t* b, size_t nb, u
         if (!(err <= kFftMaxErr)) {  // also catches NaN
             OperandDesc oa{da, (uint32_t)na, (uint32_t)(2 * na), kFmtLimb64};
             OperandDesc ob{db, (uint32_t)nb, (uint32_t)(2 * nb), kFmtLimb64};
+            const uint32_t fft_launches = g.last_launches;
             rc = multiply_device(oa, ob, square, dout, kFmtLimb64, nout, flags, st, nullptr);
+            g.last_launches += fft_launches;
             if (stats) stats->fell_back = 1;
         }
     } else if (const uint32_t sm = small_method(flags, na, nb)) {
@@ -770,11 +779,13 @@ int device_product(const uint64_t* da, size_t na, const uint64_t* db, size_t nb,
         *launches += 1;
         return launch_small(sm, da, na, db, nb, dout, st);
     }
-    if (beyond_transform(na, nb)) return huge_product(da, na, db, nb, dout, square, st);
     OperandDesc oa{da, (uint32_t)na, (uint32_t)(2 * na), kFmtLimb64};
     OperandDesc ob{db, (uint32_t)nb, (uint32_t)(2 * nb), kFmtLimb64};
-    *launches += kNttLaunches;
-    return multiply_device(oa, ob, square, dout, kFmtLimb64, na + nb, BGPU_METHOD_AUTO, st, nullptr);
+    const int rc = beyond_transform(na, nb)
+                       ? huge_product(da, na, db, nb, dout, square, st)
+                       : multiply_device(oa, ob, square, dout, kFmtLimb64, na + nb, BGPU_METHOD_AUTO, st, nullptr);
+    if (rc == BGPU_OK) *launches += g.last_launches;
+    return rc;
 }
 
 uint64_t bit_length(const uint64_t* x, size_t n) {  // n > 0, x[n-1] != 0
@@ -947,11 +958,12 @@ int mul_u64_many_locked(const bgpu_host_product* p, size_t count, uint32_t flags
                 nl += 1;
             } else if (beyond_transform(m.na, m.nb)) {
                 rc = huge_product(da, m.na, db, m.nb, dout, m.square, st);
+                nl += g.last_launches;
             } else {
                 OperandDesc oa{da, (uint32_t)m.na, (uint32_t)(2 * m.na), kFmtLimb64};
                 OperandDesc ob{db, (uint32_t)m.nb, (uint32_t)(2 * m.nb), kFmtLimb64};
                 rc = multiply_device(oa, ob, m.square, dout, kFmtLimb64, m.na + m.nb, flags, st, nullptr);
-                nl += kNttLaunches;
+                nl += g.last_launches;
             }
             if (rc != BGPU_OK) return rc;
             if (m.na + m.nb < nout) e = cudaMemsetAsync(dout + m.na + m.nb, 0, (nout - m.na - m.nb) * 8, st);
@@ -1046,7 +1058,7 @@ int mul_digits_locked(const uint32_t* a, size_t na, const uint32_t* b, size_t nb
                     : huge_product(la_d, la64, lb_d, lb64, lo_d, square, st);
         if (rc == BGPU_OK)
             rc = cuda_status(launch_limbs_to_digits28(lo_d, (uint32_t)(la64 + lb64), dres, (uint32_t)nres, st));
-        g.last_launches = square ? 3 : 4;
+        g.last_launches = (sm ? 1 : g.last_launches) + (square ? 2 : 3);  // and the conversions
         if (stats) stats->method = sm ? (int32_t)sm : BGPU_METHOD_NTT;
     } else {
         // 32-bit digit counts from the true bit lengths: a number of exactly
@@ -2779,7 +2791,7 @@ int bgpu_kernel_times(const char** names, float* mean_ms, int cap, uint32_t* npr
             if (cudaEventElapsedTime(&t, ev[k], ev[k + 1]) != cudaSuccess) return BGPU_ERR_CUDA;
             sum += t;
         }
-        if (names) names[k] = g.timed_wide ? kWideKernelNames[g.timed_wide - 1][k] : kNttKernelNames[k];
+        if (names) names[k] = g.timed_kind ? kWideKernelNames[g.timed_kind - 1][k] : kNttKernelNames[k];
         if (mean_ms) mean_ms[k] = (float)(sum / (double)n);
     }
     if (nproducts) *nproducts = (uint32_t)n;

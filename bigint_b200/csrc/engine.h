@@ -221,6 +221,9 @@ cudaError_t launch_ntt_product(int slot, const NttConsts& host, const OperandDes
                                const CarryLaunch& cl, cudaStream_t stream,
                                cudaEvent_t* ev = nullptr, const TransformShape* shape = nullptr);
 constexpr int kNttLaunches = 4;
+constexpr int kSpectrumLaunches = 2, kSpectralSumLaunches = 3, kAccumulateLaunches = 3;
+// Products of one launch of a batch: grid y and z end at 65535, two operands a product.
+constexpr uint32_t kBatchPiece = 16384;
 extern const char* const kNttKernelNames[kNttLaunches];
 
 // Carry-scan blocks: kCarryThreads threads, each resolving kCarryPer

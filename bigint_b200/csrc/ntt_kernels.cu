@@ -1355,12 +1355,10 @@ cudaError_t launch_ntt_product(int slot, const NttConsts& c, const OperandDesc& 
 cudaError_t launch_ntt_batch(int slot, const NttConsts& c, const ProductDesc* descs, int count,
                              bool square, int log_n, int out_fmt, const CarryLaunch& cl,
                              cudaStream_t st) {
-    // Grid y/z limits (65535) cap the products of one launch; larger batches
-    // go in pieces, each piece's carry scan continuing the ticket sequence.
-    constexpr int kPiece = 16384;
+    // Batches go in pieces that fit a launch grid, each piece's carry scan continuing the ticket sequence.
     const uint32_t bpp = carry_blocks((uint32_t)(((size_t)1 << log_n) / kCols));
-    for (int done = 0; done < count; done += kPiece) {
-        const int n = count - done < kPiece ? count - done : kPiece;
+    for (int done = 0; done < count; done += kBatchPiece) {
+        const int n = std::min(count - done, (int)kBatchPiece);
         CarryLaunch piece = cl;
         piece.ticket_base = cl.ticket_base + (uint64_t)done * bpp;
         const cudaError_t e = launch_ntt_core(slot, c, descs + done, ProductDesc{}, n, square,

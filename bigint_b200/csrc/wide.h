@@ -108,8 +108,7 @@ extern const char* const kWideKernelNames[2][kNttLaunches];
 
 // The four launches of `count` products of one form (digits of both operands
 // together at most 2^log_n + 1); each product's carry scan has `bpp` blocks
-// (tickets).  At most kWidePiece products.
-constexpr uint32_t kWidePiece = 16384;  // grid z limit 65535, two operands a product
+// (tickets).  At most kBatchPiece products.
 cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const ProductDesc& one, const WideStep& step,
                                 uint32_t count, bool square, int out_fmt, uint32_t bpp,
                                 const CarryLaunch& cl, cudaStream_t st, cudaEvent_t* ev);

@@ -1054,7 +1054,7 @@ cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const Prod
                                 uint32_t count, bool square, int out_fmt, uint32_t bpp, const CarryLaunch& cl, cudaStream_t st,
                                 cudaEvent_t* ev) {
     const int log_n = f.log_n;
-    if (f.np < kWidePrimes || f.np > kWideMaxPrimes || log_n > wide_max_log(f.np) || count < 1 || count > kWidePiece)
+    if (f.np < kWidePrimes || f.np > kWideMaxPrimes || log_n > wide_max_log(f.np) || count < 1 || count > kBatchPiece)
         return cudaErrorInvalidValue;
     const bool whole = log_n <= kWideShortMaxLogN;
     const int l2 = whole ? 0 : wide_shape(log_n, descs != nullptr || count > 1).log_n2;
@@ -1117,10 +1117,10 @@ cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const Prod
 
 cudaError_t launch_wide_batch(WideForm f, const ProductDesc* descs, uint32_t count, bool square, int out_fmt,
                               uint32_t bpp, const CarryLaunch& cl, cudaStream_t st) {
-    for (uint32_t done = 0; done < count; done += kWidePiece) {
+    for (uint32_t done = 0; done < count; done += kBatchPiece) {
         CarryLaunch piece = cl;
         piece.ticket_base = cl.ticket_base + (uint64_t)done * bpp;
-        const uint32_t n = count - done < kWidePiece ? count - done : kWidePiece;
+        const uint32_t n = count - done < kBatchPiece ? count - done : kBatchPiece;
         const cudaError_t e = launch_wide_product(f, descs + done, ProductDesc{}, WideStep{}, n, square, out_fmt,
                                                   bpp, piece, st, nullptr);
         if (e != cudaSuccess) return e;

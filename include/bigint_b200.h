@@ -247,9 +247,10 @@ uint32_t bgpu_last_launch_count(void);
 int bgpu_set_kernel_timing(int on);
 
 /* Mean device time of each kernel over the NTT products launched since
- * timing was switched on (the last 1024 of them): names[i], mean_ms[i] in
- * launch order, *nproducts = products averaged (products of short transforms
- * have two kernels and name the two entries between them "none").  Returns the kernel count
+ * timing was switched on (the last 1024 of them, and none from before a product
+ * with other kernels): names[i], mean_ms[i] in launch order, *nproducts =
+ * products averaged (products of short transforms have two kernels and name
+ * the two entries between them "none").  Returns the kernel count
  * (0 if none recorded).  Synchronizes on the last recorded event. */
 int bgpu_kernel_times(const char** names, float* mean_ms, int cap, uint32_t* nproducts);
 
