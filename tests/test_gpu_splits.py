@@ -83,3 +83,53 @@ def test_batch_split_beyond_the_mixed_launches(bb, port):
     for (a, b), c in zip(pairs, got):
         want = port.mul(a, b)
         assert np.array_equal(c[: want.size], want) and not c[want.size :].any()
+
+
+# every column and row length of the wide-digit kernels, the lazy primes
+# (2^13 points and more): columns of all lengths over rows of 2^8 points and
+# less, rows of all lengths over the shortest columns, the longest of each
+@pytest.mark.parametrize("col,row", [(5, 8), (6, 7), (7, 6), (8, 5), (9, 5), (10, 5), (11, 5), (5, 9), (5, 10), (5, 11),
+                                     (5, 12), (5, 13), (5, 14), (8, 14), (11, 11), (9, 13)])
+@pytest.mark.parametrize("batch", [False, True])
+def test_wide_splits(bb, port, col, row, batch):
+    rng = np.random.default_rng([SEED, col, row])
+    n = 1 << (col + row)  # limbs of the product: the longest of this many points
+    a, b = rand_limbs(rng, n - n // 3), rand_limbs(rng, n // 3)  # more and less than half the points
+    c = np.full(n // 2, 0xFFFFFFFFFFFFFFFF, dtype=np.uint64)
+    with split(bb, col + row + 1, col, batch):
+        assert (bb.get_batch_split if batch else bb.get_split)(col + row + 1) == col
+        got = run_plan(bb, [(a, b), (c, c)])[0] if batch else [bb.ntt_mul(a, b), bb.ntt_mul(c)]
+    for (x, y), z in zip([(a, b), (c, c)], got):
+        assert port.mod_m61(z) == port.mod_m61(x) * port.mod_m61(y) % M61
+
+
+# six and seven primes on columns of every length: the lazy sets at 2^16 points,
+# the strict ones at 2^21 and 2^19, and 2^24 and 2^23, the longest
+@pytest.mark.parametrize("quarters,col,log_n", [(q, col, ln) for q, ls in ((5, (16, 21)), (6, (16, 19))) for ln in ls
+                                                for col in range(max(5, ln - 14), min(12, ln - 4))]
+                         + [(5, 10, 24), (6, 10, 23)])
+def test_long_digit_splits(bb, port, quarters, col, log_n):
+    rng = np.random.default_rng([SEED, quarters, col, log_n])
+    n = quarters << (log_n - 2)  # limbs of the product: the longest in 80 or 96 bits
+    a, b = rand_limbs(rng, n - n // 2 + 7), rand_limbs(rng, n // 2 - 7)
+    with split(bb, log_n + 1, col):
+        got = bb.ntt_mul(a, b), bb.ntt_mul(a[: n // 2])
+    assert port.mod_m61(got[0]) == port.mod_m61(a) * port.mod_m61(b) % M61
+    assert port.mod_m61(got[1]) == port.mod_m61(a[: n // 2]) ** 2 % M61
+
+
+# classes of 80- and 96-bit digits (2^16 points of a class together), squares among
+# them, on short transforms and on longer ones
+@pytest.mark.parametrize("quarters,log_n,count", [(5, 12, 20), (6, 12, 20), (6, 13, 10), (5, 16, 2), (6, 16, 2)])
+def test_long_digit_classes(bb, port, quarters, log_n, count):
+    rng = np.random.default_rng([SEED, quarters, log_n])
+    n = quarters << (log_n - 2)
+    pairs = []
+    for k in range(count):
+        a = rand_limbs(rng, n // 2 - k)
+        pairs += [(a, a), (a, rand_limbs(rng, n // 2 - 2 * k))]
+    got, launches = run_plan(bb, pairs)
+    assert launches == 2 * (2 if log_n <= 12 else 4)  # one class of squares, one of products
+    for (a, b), c in zip(pairs, got):
+        want = port.mul(a, b)
+        assert np.array_equal(c[: want.size], want) and not c[want.size :].any()
