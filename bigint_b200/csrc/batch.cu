@@ -61,10 +61,9 @@ struct bgpu_batch_plan_s {
     int device = -1;
     size_t count = 0;
     std::vector<bgpu::BatchClass> classes;
-    // the three-prime classes (classes[first_mixed ..)) and the small products
-    // run in the four mixed-length launches, one per pass
+    // three-prime classes, which share four launches, one per pass, with the
+    // small products
     bool mixed = false;
-    size_t first_mixed = 0;
     bgpu::MixedSizes mixed_sizes{};
     std::vector<std::array<uint32_t, 4>> mixed_begin;  // per class, per pass
     std::vector<bgpu::SchoolDesc> school;  // schoolbook products
@@ -98,14 +97,11 @@ size_t ntt_scratch_bytes(int log_n, bool square, WideForm f) {
     return al256((square ? 1 : 2) * (size_t)kNumPrimes * nn * 4) + al256(nn / 2 * 8) + al256(nn / 8 * 8);
 }
 
-// The wide-digit transforms of the classes outside the mixed-length launches.
+// The wide-digit transforms of a plan's classes.
 void split_wide_classes(bgpu_batch_plan_s* p, const bgpu_product* prods) {
     std::vector<BatchClass> all;
-    size_t first_mixed = 0;
-    for (size_t i = 0; i < p->classes.size(); ++i) {
-        BatchClass& c = p->classes[i];
-        if (i == p->first_mixed) first_mixed = all.size();
-        if ((i < p->first_mixed || !p->mixed) && c.log_n > kWideMinLogN && c.log_n - 1 <= kWideMaxLogN) {
+    for (BatchClass& c : p->classes) {
+        if (c.log_n > kWideMinLogN && c.log_n - 1 <= kWideMaxLogN) {
             BatchClass part[kWideMaxPrimes + 1];
             for (uint32_t m : c.members) {
                 const WideForm f = wide_form((uint32_t)(2 * prods[m].na), (uint32_t)(2 * prods[m].nb), kWideMinLogN);
@@ -127,9 +123,7 @@ void split_wide_classes(bgpu_batch_plan_s* p, const bgpu_product* prods) {
             all.push_back(std::move(c));
         }
     }
-    if (p->first_mixed >= p->classes.size()) first_mixed = all.size();
     p->classes = std::move(all);
-    p->first_mixed = first_mixed;
 }
 
 void destroy_plan(bgpu_batch_plan_s* p) {
@@ -166,8 +160,8 @@ void release_streams(BatchStreams* s) {
 }
 
 static size_t plan_branches(const bgpu_batch_plan_s* p) {
-    return std::min(kBatchBranches, p->mixed ? p->first_mixed
-                                             : p->classes.size() + (p->school.empty() ? 0 : 1) + (p->kara.empty() ? 0 : 1));
+    if (p->mixed) return 0;
+    return std::min(kBatchBranches, p->classes.size() + (p->school.empty() ? 0 : 1) + (p->kara.empty() ? 0 : 1));
 }
 
 // Queue (or record, where `st` is capturing) the plan's work on `st`: reset the
@@ -185,7 +179,7 @@ static int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks
         flag_words += c.flags_words;
     }
     const size_t mixed_off = al256(n_desc * sizeof(ProductDesc));
-    const size_t nmixed = p->mixed ? p->classes.size() - p->first_mixed : 0;
+    const size_t nmixed = p->mixed ? p->classes.size() : 0;
     const size_t school_off = mixed_off + al256(nmixed * sizeof(MixedClass));
     const size_t kara_off = school_off + al256(p->school.size() * sizeof(SchoolDesc));
     const size_t tick_off = kara_off + al256(p->kara.size() * sizeof(SchoolDesc));
@@ -205,7 +199,7 @@ static int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks
         m.nclasses = (int)nmixed;
         for (size_t i = 0; i < nmixed; ++i)
             for (int pass = 0; pass < 4; ++pass) m.begin[pass][i] = p->mixed_begin[i][pass];
-        m.ticket = tickets + p->first_mixed;
+        m.ticket = tickets;
         m.ticket_base = 0;
         m.epoch = 1;
         m.err = hooks.err;
@@ -216,7 +210,7 @@ static int batch_record(bgpu_batch_plan_s* p, cudaStream_t st, const EngineHooks
         if (launch_ntt_mixed(m, p->mixed_sizes, st) != cudaSuccess) return BGPU_ERR_CUDA;
         launches += kNttLaunches;
     }
-    const size_t nbranched = p->mixed ? p->first_mixed : p->classes.size();
+    const size_t nbranched = p->mixed ? 0 : p->classes.size();
     for (size_t ci = 0; ci < nbranched; ++ci) {
         const BatchClass& c = p->classes[ci];
         const int ps = prime_set_for(c.log_n);
@@ -304,8 +298,8 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
     // of each pass, start in the first wave and the short ones fill the tail.
     std::stable_sort(p->classes.begin(), p->classes.end(),
                      [](const BatchClass& x, const BatchClass& y) { return x.log_n > y.log_n; });
-    // The mixed-length launches take the short classes when each qualifies and
-    // there are several lengths, unless the caller asks for per-class launch
+    // The mixed-length launches take a plan of several short classes, when each
+    // qualifies, unless the caller asks for per-class launch
     // sets (BGPU_BATCH_PER_CLASS); a single length runs its own per-length
     // kernels (tuned for it, without the mixed launches' register budget):
     // a uniform batch of the decimal conversions' levels ran 5.6 -> 9.0 ms
@@ -313,13 +307,10 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
 #ifndef BGPU_MIXED_BATCH
 #define BGPU_MIXED_BATCH 1
 #endif
-    while (p->first_mixed < p->classes.size() && p->classes[p->first_mixed].log_n >= kBatchWideLog32) ++p->first_mixed;
-    const size_t nshort = p->classes.size() - p->first_mixed;
-    p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && p->first_mixed == 0 && nshort >= 2 &&
-               nshort <= (size_t)kMaxMixedClasses;
-    for (size_t i = p->first_mixed; i < p->classes.size(); ++i)
-        p->mixed = p->mixed && mixed_class_ok(p->classes[i].log_n);
-    split_wide_classes(p, prods);
+    p->mixed = BGPU_MIXED_BATCH && !(flags & BGPU_BATCH_PER_CLASS) && p->classes.size() >= 2 &&
+               p->classes.size() <= (size_t)kMaxMixedClasses && p->classes[0].log_n < kBatchWideLog32;
+    for (const BatchClass& c : p->classes) p->mixed = p->mixed && mixed_class_ok(c.log_n);
+    if (!p->mixed) split_wide_classes(p, prods);
     // Layout: [ProductDesc...][MixedClass...][SchoolDesc: schoolbook...]
     //         [SchoolDesc: Karatsuba...][tickets][flags][scratch].
     size_t n_desc = 0, flag_words = 0, scratch = 0;
@@ -339,7 +330,7 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
         c.scratch_off = scratch;
         scratch += c.members.size() * ntt_scratch_bytes(c.log_n, c.square, c.form);
     }
-    const size_t nmixed = p->mixed ? nshort : 0;
+    const size_t nmixed = p->mixed ? p->classes.size() : 0;
     const size_t mixed_off = al256(n_desc * sizeof(ProductDesc));
     const size_t school_off = mixed_off + al256(nmixed * sizeof(MixedClass));
     const size_t kara_off = school_off + al256(p->school.size() * sizeof(SchoolDesc));
@@ -377,7 +368,7 @@ static int plan_layout(const bgpu_product* prods, size_t count, uint32_t flags, 
     if (p->mixed) {
         std::vector<MixedClassSpec> spec(nmixed);
         for (size_t i = 0; i < nmixed; ++i) {
-            const BatchClass& c = p->classes[p->first_mixed + i];
+            const BatchClass& c = p->classes[i];
             spec[i] = MixedClassSpec{reinterpret_cast<const ProductDesc*>(base) + c.desc_off,
                                      (uint32_t)c.members.size(), c.log_n, c.square};
         }
