@@ -239,7 +239,7 @@ int prepare_scratch(int log_n, bool square, ProductScratch* s) {
     const size_t y_bytes = align256((square ? 1 : 2) * (size_t)kNumPrimes * nn * 4);
     const size_t ch_bytes = align256(nn / 2 * 8);
     const size_t sp_bytes = align256(nn / 8 * 8);
-    if (carry_blocks_narrow((uint32_t)(nn / 8)) > kFlagWords) return BGPU_ERR_CAPACITY;  // either shape
+    if (carry_blocks((uint32_t)(nn / 8)) > kFlagWords) return BGPU_ERR_CAPACITY;
     int rc = ensure(&g.d_scratch, &g.scratch_bytes, y_bytes + ch_bytes + sp_bytes);
     if (rc != BGPU_OK) return rc;
     char* b = static_cast<char*>(g.d_scratch);
@@ -363,12 +363,10 @@ int multiply_device(const OperandDesc& a, const OperandDesc& b, bool square, voi
     // only an identical layout keeps this forward pass's planes clear of the
     // previous product's carry data while that scan still runs.
     cl.overlap_prev = overlap_prev && st == g.ntt_stream && ln == g.ntt_log_n && square == g.ntt_square;
-    cl.narrow = !cl.overlap_prev;
     g.ntt_stream = st;
     g.ntt_log_n = ln;
     g.ntt_square = square;
-    const uint32_t nch = (uint32_t)(((size_t)1 << ln) / 8);
-    g.ticket_base += cl.narrow ? carry_blocks_narrow(nch) : carry_blocks(nch);
+    g.ticket_base += carry_blocks((uint32_t)(((size_t)1 << ln) / 8));
     cudaEvent_t* ev = timing_events(0);
     const int ps = prime_set_for(ln);
     cudaError_t e = launch_ntt_product(kSlotEngine + ps, g.consts[ps], a, b, square, ln, s, out,

@@ -203,10 +203,6 @@ struct CarryLaunch {
     // on the stream (the previous product's carry scan), waiting for it only
     // before it exits; only for operands that nothing in flight writes.
     bool overlap_prev = false;
-    // Single products: the carry scan in the narrow shape (ticket count
-    // carry_blocks_narrow), for a product whose forward pass waited for its
-    // predecessor (a chain of dependent products, whose scans overlap nothing).
-    bool narrow = false;
 };
 
 // Launch the full NTT product pipeline (4 kernels) on `stream`.
@@ -238,15 +234,6 @@ constexpr int kCarryThreads = BGPU_CARRY_THREADS;
 constexpr int kCarryPer = BGPU_CARRY_PER;
 constexpr uint32_t kCarryChunksPerBlock = (uint32_t)(kCarryThreads * kCarryPer);
 uint32_t carry_blocks(uint32_t nchunks);
-// The narrow shape, for a single product that waits for its predecessor
-// (CarryLaunch::narrow): more, smaller blocks shorten the scan on the
-// product's critical path (2^20 points: 66.70 -> 66.15 us per product back to
-// back), while a scan that runs under the next product's forward pass keeps
-// the default (63.60 against 63.81 us there).  Scratch sized for a product's
-// flag words takes the narrow count, the larger of the two.
-constexpr int kCarryNarrowThreads = 128;
-constexpr int kCarryNarrowPer = 2;
-uint32_t carry_blocks_narrow(uint32_t nchunks);
 
 // Diagnostic launch of the carry scan's bounded wait on one flag word.
 cudaError_t launch_wait_selftest(const uint64_t* flag, uint64_t epoch, uint32_t limit, uint32_t* err,

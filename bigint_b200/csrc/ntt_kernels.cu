@@ -32,26 +32,6 @@
 
 namespace bgpu {
 
-// Row-pass CTAs are held to a register budget below what the compiler takes
-// on its own, so that more of them share an SM: rows of 2^10 to 2^12 points at
-// 1024 threads' worth per SM (64 registers a thread: sixteen, eight or four
-// CTAs), rows of 2^13 points at three 256-thread CTAs (80 registers; their two
-// shared row buffers leave room for no more).  Measured per product back to
-// back, each against the compiler's own choice or the earlier cap:
-//   2^20 points (2^24 x 2^24 bits, rows of 2^11): 61.98 us against 62.16 at
-//     1152 threads' worth (56 registers), 63.42 at 1280 (48), 62.87 at 896;
-//   2^19 points (rows of 2^10): 38.97 against 39.6 at 1280;
-//   2^21 points (rows of 2^12): 119.2 against 126.4 (95 registers, two CTAs),
-//     122.3 at three CTAs, 121.4 at five;
-//   2^22 points (rows of 2^13): 239.7 against 254.8 (88 registers, two CTAs).
-// Longer rows keep the compiler's choice.
-#ifndef BGPU_MID_THREADS_PER_SM
-#define BGPU_MID_THREADS_PER_SM 1024
-#endif
-__host__ __device__ constexpr int mid_min_blocks(int l1, int threads) {
-    return threads < 64 ? 1 : (l1 <= 12 ? BGPU_MID_THREADS_PER_SM / threads : (l1 == 13 ? 768 / threads : 1));
-}
-
 constexpr int kCols = 8;  // columns per outer tile == 32-bit digits per carry chunk
 // The forward pass's tiles and threads (measured against 4-column tiles of
 // 128 or 64 threads and 8-column tiles of 128 threads: all slower).
@@ -444,7 +424,7 @@ __device__ __forceinline__ void mid_rows_body(const MidRowsArgs& a, uint32_t slo
 }
 
 template <int PS, int L1, int T, bool SQR>
-__global__ void __launch_bounds__(T, mid_min_blocks(L1, T)) k_mid_rows(const MidRowsArgs a) {
+__global__ void __launch_bounds__(T) k_mid_rows(const MidRowsArgs a) {
     extern __shared__ __align__(16) uint32_t sm[];
     mid_rows_body<PS, L1, T, SQR>(a, blockIdx.x, blockIdx.y, sm);
 }
@@ -1065,10 +1045,11 @@ TransformShape choose_shape_batch(int log_n) { return shape_from(g_batch_split, 
 
 size_t smem_fwd_cols(int l2, int cols) { return ((size_t)cols * 4 << l2) + cols * 17 * sizeof(uint2); }
 size_t smem_mid_rows(int l1, bool square) {
-    return (square || l1 >= 15 ? 1 : 2) * ((size_t)4 << l1) + 16 * sizeof(uint2);
+    return (square ? 1 : 2) * ((size_t)4 << l1) + 16 * sizeof(uint2);
 }
 size_t smem_inv_cols(int l2) { return (size_t)kNumPrimes * kCols * 4 << l2; }
 
+// Threads of a row (rows of 2^10 points and more: spectral sums only).
 static constexpr int mid_threads(int l1) { return l1 >= 12 ? 256 : (l1 >= 9 ? (1 << (l1 - 4)) : 32); }
 
 
@@ -1127,8 +1108,9 @@ static cudaError_t launch_mid(const MidRowsArgs& m, bool square, uint32_t rows, 
     return launch_k(k, grid, dim3(T), sm, st, m);
 }
 
-// Lazy set only: transforms of the strict one are products of spectral sums,
-// every other product as long is a wide-digit one.
+// Lazy set only, rows of at most 2^9 points: the products are the shortest ones
+// and those of the no-allocation entry point (2^17 points); longer ones are
+// wide-digit products and spectral sums.
 static cudaError_t dispatch_mid(int l1, const MidRowsArgs& m, bool square, uint32_t rows, int count,
                                 cudaStream_t st) {
     switch (l1) {
@@ -1139,11 +1121,6 @@ static cudaError_t dispatch_mid(int l1, const MidRowsArgs& m, bool square, uint3
         case 7: return launch_mid<0, 7>(m, square, rows, count, st);
         case 8: return launch_mid<0, 8>(m, square, rows, count, st);
         case 9: return launch_mid<0, 9>(m, square, rows, count, st);
-        case 10: return launch_mid<0, 10>(m, square, rows, count, st);
-        case 11: return launch_mid<0, 11>(m, square, rows, count, st);
-        case 12: return launch_mid<0, 12>(m, square, rows, count, st);
-        case 13: return launch_mid<0, 13>(m, square, rows, count, st);
-        case 14: return launch_mid<0, 14>(m, square, rows, count, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -1215,11 +1192,6 @@ static cudaError_t dispatch_spec_rows(int l1, const SpecArgs& s, bool mac, uint3
 
 uint32_t carry_blocks(uint32_t nchunks) {
     return (nchunks + 1 + kCarryChunksPerBlock - 1) / kCarryChunksPerBlock;
-}
-
-uint32_t carry_blocks_narrow(uint32_t nchunks) {
-    constexpr uint32_t cpb = (uint32_t)(kCarryNarrowThreads * kCarryNarrowPer);
-    return (nchunks + 1 + cpb - 1) / cpb;
 }
 
 static uint32_t mont_of(uint64_t v, uint32_t p) { return (uint32_t)((v % p << 32) % p); }
@@ -1319,14 +1291,8 @@ static cudaError_t launch_inverse_carry(int slot, int ps, const ProductDesc* des
     ca.ticket_base = cl.ticket_base;
     ca.epoch = cl.epoch;
     ca.err = cl.err;
-    if (cl.narrow && count == 1) {
-        ca.bpp = carry_blocks_narrow(ca.nchunks);
-        e = launch_k(k_carry<kCarryNarrowThreads, kCarryNarrowPer>, dim3(ca.bpp), dim3(kCarryNarrowThreads), 0, st,
-                     ca);
-    } else {
-        ca.bpp = carry_blocks(ca.nchunks);
-        e = launch_k(k_carry<kCarryThreads, kCarryPer>, dim3(ca.bpp * count), dim3(kCarryThreads), 0, st, ca);
-    }
+    ca.bpp = carry_blocks(ca.nchunks);
+    e = launch_k(k_carry<kCarryThreads, kCarryPer>, dim3(ca.bpp * count), dim3(kCarryThreads), 0, st, ca);
     if (ev) cudaEventRecord(ev[4], st);
     return e;
 }
