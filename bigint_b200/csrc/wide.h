@@ -98,7 +98,7 @@ __host__ __device__ inline uint32_t wide_carry_blocks(int np, size_t out_cap, in
 
 // Split of 2^log_n points: the tuned one of 2^(log_n + 1) 32-bit digits
 // (bgpu_set_split, bgpu_set_batch_split) where its kernels are built, else the
-// built-in one.  log_n2 == 0: no transform of this length.
+// built-in one.  log_n2 == 0: one block does it whole, or no transform of this length.
 TransformShape wide_shape(int log_n, bool batch);
 cudaError_t upload_wide_consts(int set, const NttConsts& c);
 // Kernels of a form: four, or two where one block does a transform whole (the

@@ -1005,20 +1005,19 @@ cudaError_t upload_wide_consts(int set, const NttConsts& c) {
 
 // Built-in column lengths, the fastest measured on B200 for one product and
 // for a batch that fills the GPU (two operands of half the points).  us per
-// product back to back, the choice against the nearest other length: 2^12
-// points 9.8 (2^6) / 11.3 (2^7), 2^17 21.0 (2^6) / 22.2 (2^7), 2^18 28.9 (2^8) /
+// product back to back, the choice against the nearest other length: 2^17 points 21.0 (2^6) / 22.2 (2^7), 2^18 28.9 (2^8) /
 // 29.8 (2^7), 2^19 47.7 (2^8) / 49.5 (2^9), 2^20 88.7 (2^8) / 90.4 (2^9), 2^21 175.7
 // (2^10) / 180.5 (2^9), 2^23 753 (2^10) / 780 (2^11), 2^24 1543 (2^10) / 1572 (2^11).
 // Batches, us per 2^19 points: 2^13 33.7 (2^7) / 35.7 (2^6), 2^15 34.5 (2^8) /
 // 35.4 (2^7), 2^17 37.8 (2^9) / 38.8 (2^8), 2^19 38.7 (2^8) / 40.4 (2^9).
-static constexpr int8_t kWideColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  5,  6,  6,
+static constexpr int8_t kWideColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  0,  0,  0,
                                                          7, 8, 8, 8, 6, 8, 8, 8, 10, 10, 10, 10, 11};
-static constexpr int8_t kWideBatchColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  5,  6,  6,
+static constexpr int8_t kWideBatchColumn[kWideMaxLogN + 1] = {0, 0, 0, 0, 0, 0, 0, 0, 0,  0,  0,  0,  0,
                                                               7, 8, 8, 8, 9, 8, 8, 9, 10, 10, 10, 10, 11};
 
 TransformShape wide_shape(int log_n, bool batch) {
     TransformShape s{log_n, 0, 0};
-    if (log_n < kWideMinLogN || log_n > kWideMaxLogN) return s;
+    if (log_n <= kWideShortMaxLogN || log_n > kWideMaxLogN) return s;
     auto built = [&](int l2) { return l2 >= 5 && l2 <= 11 && log_n - l2 >= 5 && log_n - l2 <= 14; };
     const int tuned = tuned_split(log_n + 1, batch);
     s.log_n2 = built(tuned) ? tuned : (batch ? kWideBatchColumn : kWideColumn)[log_n];
@@ -1057,7 +1056,7 @@ cudaError_t launch_wide_product(WideForm f, const ProductDesc* descs, const Prod
     if (f.np < kWidePrimes || f.np > kWideMaxPrimes || log_n > wide_max_log(f.np) || count < 1 || count > kBatchPiece)
         return cudaErrorInvalidValue;
     const bool whole = log_n <= kWideShortMaxLogN;
-    const int l2 = whole ? 0 : wide_shape(log_n, descs != nullptr || count > 1).log_n2;
+    const int l2 = wide_shape(log_n, descs != nullptr || count > 1).log_n2;
     if (log_n < kWideMinLogN || (!whole && !l2)) return cudaErrorInvalidValue;
     const int w = wide_set_for(f.np, log_n) - kFirstWideSet;
     const bool lazy = w % 2 == 0;
