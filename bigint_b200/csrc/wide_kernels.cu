@@ -222,10 +222,13 @@ __device__ __forceinline__ OperandDesc wide_operand(const WideFwdArgs& fa, uint3
 
 // CTAs per SM (register caps): 1024 threads' worth of 64 registers, except
 // columns of 2^9 rows at 1280 (2^19 points of a batch: 15.0 + 5.7 us; at 1024
-// 15.5 + 6.2, at 2048 15.1 + 5.9), of 2^8 rows nine CTAs, which hold the 1280 CTAs
-// of a 2^19-point inverse pass in one wave (with the same for rows of 2^11 points
-// a product of 2^19 points 47.6 -> 46.2 us, at ten 47.2; 2^20 points 88.0 -> 87.8),
-// and the inverse pass's tiles of 2^11 rows.
+// 15.5 + 6.2, at 2048 15.1 + 5.9), of 2^8 rows nine CTAs, and the inverse pass's
+// tiles of 2^11 rows.  Nine CTAs (here, and for rows of 2^11 points) hold the 1280
+// CTAs of a 2^19-point inverse pass over five primes in one wave; us per product,
+// eight -> nine: 2^14 to 2^16 points 11.9 -> 12.0, 15.1 -> 15.1, 16.6 -> 16.6, 2^18
+// 29.1 -> 28.7, 2^19 47.7 -> 46.4 (ten 47.2), 2^20 89.4 -> 89.2, 2^21 174.8 ->
+// 175.1; 2^18 over six primes 36.8 -> 37.4, over seven 39.1 -> 39.4, 2^19 61.7 -> 61.8;
+// per 2^19 points of a batch, 2^14 to 2^20 points, 0.1 to 0.2 less.
 __host__ __device__ constexpr int wide_col_blocks(int l2, bool fwd) {
     return l2 == 8 ? 9 : l2 == 9 ? 5 : l2 == 11 && !fwd ? 3 : 1024 / wide_col_threads(l2, fwd);
 }
