@@ -306,11 +306,14 @@ cudaError_t launch_carry(const uint64_t* chunks, const uint64_t* spill, uint32_t
 // ---- batched products (batch.cu) ----
 // Streams and events that plans are recorded with, a branch for their classes
 // in turn.  The engine keeps them: made and dropped with each plan, six branches
-// took 0.9 of the 1.5 ms in which a plan of 64 products of 2^10..2^18 bits was built.
-// A branch costs 50 us where the graph is made and saves where it runs: 2, 4, 6
-// branches 70, 56, 58 us (the plan above), 184, 146, 138 (2^10..2^22 bits), 267, 218,
-// 231 (512 products of 2^10..2^20 bits).
-constexpr size_t kBatchBranches = 4;
+// took 0.7 of the 1.4 ms in which a plan of 64 products of 2^10..2^18 bits was built.
+// A branch costs 50 us where the graph is made (4, 6, 8 branches 0.60, 0.76, 0.70 ms
+// for that plan), and where it runs the number decides which classes follow one
+// another: us at 4, 6, 8 branches 41.5, 46.5, 34.8 (that plan), 116, 106, 96 and 124,
+// 111, 116 (two of 64 products of 2^10..2^22 bits), 199, 207, 188 (512 of 2^10..2^20),
+// 130, 116, 130 (1024 of 2^10..2^18), 2174, 2155, 2154 (1748 of 2^10..2^22), 4837,
+// 4831, 4841 (4096).
+constexpr size_t kBatchBranches = 6;
 struct BatchStreams {
     cudaStream_t cap = nullptr, branch[kBatchBranches] = {};
     cudaEvent_t fork = nullptr, join[kBatchBranches] = {};
