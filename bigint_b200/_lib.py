@@ -518,8 +518,9 @@ def mul_device(a_ptr: int, na: int, b_ptr: int, nb: int, out_ptr: int, stream: i
     ``out_ptr`` receives na+nb limbs.  Equal pointers and lengths square.
     ``stream`` is a cudaStream_t handle (0 = legacy default stream), e.g.
     ``torch.cuda.current_stream().cuda_stream``.  ``method`` may include
-    ``BGPU_INDEPENDENT`` for a stream of independent products (the next
-    product's transform starts under the previous one's carry scan)."""
+    ``BGPU_INDEPENDENT`` for a stream of independent products (of those on the
+    three-prime transform the next one's transform starts under the previous
+    one's carry scan)."""
     _ensure_init()
     rc = lib.bgpu_mul_u64_device(C.c_void_p(a_ptr), na, C.c_void_p(b_ptr), nb,
                                  C.c_void_p(out_ptr), method, C.c_void_p(stream or None))

@@ -21,7 +21,7 @@ LIB = os.path.join(HERE, "libbigint_b200.so")
 BUILD_DIR = os.path.join(HERE, "_build")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # Device code stays uncompressed: unpacking it took 37 of the 118 ms of a
-# process's first bgpu_init (the library is 70 MB instead of 26 MB).
+# process's first bgpu_init (the library is 67 MB instead of 25 MB).
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a", "-no-compress"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
          "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include"), "-I", CSRC]

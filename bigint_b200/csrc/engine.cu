@@ -2119,8 +2119,8 @@ static int run_products(const bgpu_product* pr, size_t count, cudaStream_t st, u
 // (src/bigint.cpp:25-90) and convert_from_dec_string (:92-124).  The sign and
 // the digit characters are picked out on the host exactly as the reference
 // reads them; the value is built on the device (decimal.cu): leaves of 19
-// digits, then levels of hi * 10^(19 * 2^j) + lo, each level one batch plan
-// of equal products and one segmented carry add.
+// digits, then levels of hi * 10^(19 * 2^j) + lo, each level one set of
+// launches of equal products (run_products) and one segmented carry add.
 static int from_decimal_locked(const char* s, size_t len, uint32_t* out, size_t out_cap, size_t* out_len,
                                int* out_neg) {
     size_t i = 0;

@@ -51,9 +51,9 @@ struct OperandDesc {
 // whether they are squares.
 struct ProductDesc {
     OperandDesc op[2];  // op[1] == op[0] when squaring
-    uint32_t* y;        // (square ? 1 : 2) * 3 * N residues
-    uint64_t* chunks;   // N/2 limbs (8-coefficient chunk sums)
-    uint64_t* spill;    // N/8 spills
+    uint32_t* y;        // (square ? 1 : 2) * 3 * N residues (wide digits: the form's primes and N)
+    uint64_t* chunks;   // three primes: N/2 limbs (8-coefficient chunk sums)
+    uint64_t* spill;    // three primes: N/8 spills
     uint64_t* flags;    // carry-scan block status words
     void* out;          // output in the launch's format
     size_t out_cap;     // elements of out

@@ -5,8 +5,8 @@
 // code that runs under a caller-owned memory budget or pool that must not
 // grow, host threads that may not call cudaMalloc (it can synchronize the
 // device), or a process that pre-plans every byte it uses on the GPU.
-// bgpu_mul_u64_device_noalloc serves them: it runs the same four NTT kernels
-// as bgpu_mul_u64_device, but every scratch buffer (residue planes, chunk
+// bgpu_mul_u64_device_noalloc serves them: it runs the four three-prime NTT
+// kernels (bgpu_mul_u64_device runs products as long on wide digits), and every scratch buffer (residue planes, chunk
 // sums, spills, carry-scan flags, ticket, error word) lives in the file-scope
 // array g_noalloc_scratch below and the twiddle tables in file-scope arrays
 // too.  Nothing is allocated: no cudaMalloc / cudaFree / allocating library
